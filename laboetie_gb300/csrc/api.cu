@@ -80,6 +80,7 @@ LbConst64 make_const64(double tau)
     K.c1 = 1.0 - 1.0 / t;
     K.c2 = 1.0 / t;
     K.c3 = 1.0 - 1.0 / (2.0 * t);
+    K.c3h = 0.5 * K.c3;
     for (int w = 0; w < 3; ++w) {
         K.c2a0[w] = K.c2 * K.a0[w];
         K.c2a1[w] = K.c2 * K.a1[w];

@@ -70,7 +70,7 @@ struct FlowArgs32 {
 // FP64 strict ---------------------------------------------------------------------------
 // fused step: pull-stream (halfway bounce-back) + moments + [l2err, j store] + collision
 cudaError_t launch_flow_step_f64(const FlowArgs64 &a, int fmask, bool field, bool check,
-                                 bool ref, unsigned grid, cudaStream_t s);
+                                 bool ref, cudaStream_t s);
 // collision only, reading pre-collision n from src buffer (parity) and density/j arrays,
 // writing post-collision populations to the other buffer
 cudaError_t launch_collide_f64(const FlowArgs64 &a, int fmask, bool field, cudaStream_t s);

@@ -500,7 +500,7 @@ int lbgpu_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int h
     cudaGraphExec_t exec;
     LBG_CK(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int g = 0; g < G; ++g) {
-        cudaError_t e = launch_flow_step_f64(a, fmask, field, true, true, 0, s);
+        cudaError_t e = launch_flow_step_f64(a, fmask, field, true, true, s);
         if (e != cudaSuccess) {
             cudaStreamEndCapture(s, &graph);
             return ctx_cuda(ctx, e, "capture flow step");
@@ -559,7 +559,7 @@ int lbgpu_flow_steps(lbgpu_ctx *ctx, int nsteps, int force_on)
         a.parity = ctx->cur;
         a.force_moment = ctx->force_last_collide;
         a.force_collide = force_on ? 1 : 0;
-        LBG_CK(ctx, launch_flow_step_f64(a, fmask, false, false, false, 0, ctx->stream));
+        LBG_CK(ctx, launch_flow_step_f64(a, fmask, false, false, false, ctx->stream));
         ctx->prev_force_moment = ctx->force_last_collide;
         ctx->force_last_collide = a.force_collide;
         ctx->cur ^= 1;
@@ -593,7 +593,7 @@ int lbgpu_time_flow_steps(lbgpu_ctx *ctx, int nsteps, int force_on, float *ms)
             a.parity = ctx->cur ^ k;
             a.force_moment = force_on;
             a.force_collide = force_on;
-            cudaError_t e = launch_flow_step_f64(a, fmask, false, false, false, 0, s);
+            cudaError_t e = launch_flow_step_f64(a, fmask, false, false, false, s);
             if (e != cudaSuccess) {
                 cudaStreamEndCapture(s, &g);
                 return ctx_cuda(ctx, e, "capture");

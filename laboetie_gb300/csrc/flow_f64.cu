@@ -14,7 +14,7 @@
 // (equilibration.f90:204-243).  Each population takes part in at most one swap, so the pair is
 // exactly the pull rule  n_new(x,l) = n*(x - c_l, l)  if nature(x - c_l) == nature(x),
 // else n*(x, inv l).  The kernels pull; bit l of the node flag word says which source to use.
-#include <cfloat>
+#include <type_traits>
 
 #include "common.cuh"
 #include "flow.h"
@@ -51,7 +51,21 @@ __device__ __forceinline__ double addsgn(double s, double t)
 // module_collision.f90:77-108 for one fluid node, all 19 velocities.
 // FMASK: which components of the force are non-zero (bit 0 x, 1 y, 2 z); 0 = no force.
 // UCF: the force is the launch-uniform f_ext and c_l.F is taken from a.cf.
-template <int FMASK, bool UCF>
+// TAU1: the relaxation time is 1 (c1 = 0, c2 = 1, c3 = 1/2), the reference's default.
+//
+// The step is bound by the FP64 pipe (one warp instruction per 19 cycles of an SM), so what counts
+// is the number of FP64 instructions.  Every rounding of the reference is kept, but a product that
+// is exact needs no rounding of its own: scaling by a power of two is exact, and a fused
+// multiply-add of an exact product rounds where the reference's separate addition does.  With the
+// reference's weights a2 = 1/4, 1/8 and 2 a2 = 1/2, 1/4 (axis, diagonal), so
+//   x + a2 S              = fma(a2, S, x)
+//   (2 a2 cu) cF + x      = fma(2 a2, cu cF, x)      cu cF formed once per pair (both change sign)
+// and a1 and 2 a2 of a diagonal link are half of an axis link's, so T of a diagonal link is half
+// of the same expression with the axis constants (c3 T = (c3/2) (2 T)).  With TAU1 also
+//   c1 n + c2 neq         = fma(c1, n, neq),         x + c3 T = fma(c3, T, x).
+// (Exact unless a value falls below the smallest normal double.)  The step of the 192^3 porous
+// medium issues 334 FP64 instructions per node in the term-by-term form.
+template <int FMASK, bool UCF, bool TAU1>
 __device__ __forceinline__ void collide_node(double (&n)[Q], const double rho, const double jx,
                                              const double jy, const double jz, const double fx,
                                              const double fy, const double fz,
@@ -71,31 +85,27 @@ __device__ __forceinline__ void collide_node(double (&n)[Q], const double rho, c
     if constexpr (FMASK & 1) { gx0 = (-ux) * fx; gxp = (1.0 - ux) * fx; gxm = (-1.0 - ux) * fx; }
     if constexpr (FMASK & 2) { gy0 = (-uy) * fy; gyp = (1.0 - uy) * fy; gym = (-1.0 - uy) * fy; }
     if constexpr (FMASK & 4) { gz0 = (-uz) * fz; gzp = (1.0 - uz) * fz; gzm = (-1.0 - uz) * fz; }
-
-    static_for<0, Q>([&](auto L) {
+    // a2 term: jx*ux*(cx^2-cs^2) + jx*uy*cx*cy + ... + jz*uz*(cz^2-cs^2), even in c
+    auto a2_sum = [&](auto CX, auto CY, auto CZ) {
+        constexpr int cx = decltype(CX)::value, cy = decltype(CY)::value, cz = decltype(CZ)::value;
+        double S = cx != 0 ? Dx1 : Dx0;
+        S = addsgn<cx * cy>(S, Pxy);
+        S = addsgn<cx * cz>(S, Pxz);
+        S = addsgn<cy * cx>(S, Pyx);
+        S = S + (cy != 0 ? Dy1 : Dy0);
+        S = addsgn<cy * cz>(S, Pyz);
+        S = addsgn<cz * cx>(S, Pzx);
+        S = addsgn<cz * cy>(S, Pzy);
+        return S + (cz != 0 ? Dz1 : Dz0);
+    };
+    // c1 n + c2 neq + c3 T of direction l, T = a1*((cx-ux)*fx + (cy-uy)*fy + (cz-uz)*fz)
+    // + 2*a2*(c.u)*(c.f), cucf = (c.u)*(c.f)
+    auto relax = [&](auto L, double neq, double cucf) {
         constexpr int l = decltype(L)::value;
         constexpr Vel c = vel(l);
         constexpr int w = wclass(l);
-        // a2 term: jx*ux*(cx^2-cs^2) + jx*uy*cx*cy + ... + jz*uz*(cz^2-cs^2)
-        double S = c.x != 0 ? Dx1 : Dx0;
-        S = addsgn<c.x * c.y>(S, Pxy);
-        S = addsgn<c.x * c.z>(S, Pxz);
-        S = addsgn<c.y * c.x>(S, Pyx);
-        S = S + (c.y != 0 ? Dy1 : Dy0);
-        S = addsgn<c.y * c.z>(S, Pyz);
-        S = addsgn<c.z * c.x>(S, Pzx);
-        S = addsgn<c.z * c.y>(S, Pzy);
-        S = S + (c.z != 0 ? Dz1 : Dz0);
-        double neq;
-        if constexpr (l == 0) {
-            neq = ar[0] + K.a2[0] * S;
-        } else {
-            const double cj = dotc<c.x, c.y, c.z>(jx, jy, jz);
-            neq = (ar[w] + K.a1[w] * cj) + K.a2[w] * S;
-        }
-        double r = K.c1 * n[l] + K.c2 * neq;
+        double r = TAU1 ? __fma_rn(K.c1, n[l], neq) : K.c1 * n[l] + K.c2 * neq;
         if constexpr (FMASK != 0) {
-            // a1*((cx-ux)*fx + (cy-uy)*fy + (cz-uz)*fz) + 2*a2*(c.u)*(c.f)
             double t1 = 0.0;
             if constexpr (FMASK & 1) t1 = c.x > 0 ? gxp : (c.x < 0 ? gxm : gx0);
             if constexpr (FMASK & 2) {
@@ -108,20 +118,54 @@ __device__ __forceinline__ void collide_node(double (&n)[Q], const double rho, c
                 if constexpr (FMASK & 3) t1 = t1 + g;
                 else t1 = g;
             }
-            double T = K.a1[w] * t1;
+            // T (rest, axis), 2 T (diagonal); a1 of the rest velocity is 1
+            double T = l == 0 ? t1 : K.a1[1] * t1;
             constexpr bool hasT2 = ((FMASK & 1) && c.x != 0) || ((FMASK & 2) && c.y != 0) ||
                                    ((FMASK & 4) && c.z != 0);
-            if constexpr (hasT2) {
-                const double cu = dotc<c.x, c.y, c.z>(ux, uy, uz);
-                double cfl;
-                if constexpr (UCF) cfl = a.cf[l];
-                else cfl = dotc<(FMASK & 1) ? c.x : 0, (FMASK & 2) ? c.y : 0, (FMASK & 4) ? c.z : 0>(fx, fy, fz);
-                T = T + K.two_a2[w] * cu * cfl;
-            }
-            r = r + K.c3 * T;
+            if constexpr (hasT2) T = __fma_rn(K.two_a2[1], cucf, T);
+            const double k3 = w == 2 ? K.c3h : K.c3;
+            r = TAU1 ? __fma_rn(k3, T, r) : r + k3 * T;
         }
         n[l] = r;
+    };
+    relax(std::integral_constant<int, 0>{},
+          ar[0] + K.a2[0] * a2_sum(std::integral_constant<int, 0>{}, std::integral_constant<int, 0>{},
+                                   std::integral_constant<int, 0>{}),
+          0.0);
+    static_for<0, 9>([&](auto P) {
+        constexpr int l = pair_l(decltype(P)::value);
+        constexpr int li = inv(l);
+        constexpr Vel c = vel(l);
+        constexpr int w = wclass(l);
+        const double S = a2_sum(std::integral_constant<int, c.x>{}, std::integral_constant<int, c.y>{},
+                                std::integral_constant<int, c.z>{});
+        const double a1cj = K.a1[w] * dotc<c.x, c.y, c.z>(jx, jy, jz);
+        double cucf = 0.0;
+        if constexpr (FMASK != 0) {
+            double cfl;
+            if constexpr (UCF) cfl = a.cf[l];
+            else cfl = dotc<(FMASK & 1) ? c.x : 0, (FMASK & 2) ? c.y : 0, (FMASK & 4) ? c.z : 0>(fx, fy, fz);
+            cucf = dotc<c.x, c.y, c.z>(ux, uy, uz) * cfl;
+        }
+        relax(std::integral_constant<int, l>{}, __fma_rn(K.a2[w], S, ar[w] + a1cj), cucf);
+        relax(std::integral_constant<int, li>{}, __fma_rn(K.a2[w], S, ar[w] - a1cj), cucf);
     });
+}
+
+// The same for a force switched on or off at run time, in the form of the box's relaxation time.
+template <int FMASK, bool UCF>
+__device__ __forceinline__ void collide_strict(double (&n)[Q], const double rho, const double jx,
+                                               const double jy, const double jz, const double fx,
+                                               const double fy, const double fz, const FlowArgs64 &a,
+                                               const bool force)
+{
+    if (a.K.c2 == 1.0 && a.K.c3 == 0.5) {
+        if (force) collide_node<FMASK, UCF, true>(n, rho, jx, jy, jz, fx, fy, fz, a);
+        else collide_node<0, true, true>(n, rho, jx, jy, jz, 0.0, 0.0, 0.0, a);
+    } else {
+        if (force) collide_node<FMASK, UCF, false>(n, rho, jx, jy, jz, fx, fy, fz, a);
+        else collide_node<0, true, false>(n, rho, jx, jy, jz, 0.0, 0.0, 0.0, a);
+    }
 }
 
 // LBGPU_FP64_FUSED: density and flux from the pair sums and differences of opposite velocities
@@ -259,15 +303,20 @@ __device__ __forceinline__ void moments19(const double (&n)[Q], double fhx, doub
     jz = Z;
 }
 
+// n < 0 and NaN / Inf tests on the bits, off the FP64 pipe (a comparison of doubles occupies it like
+// an addition): with the sign bit dropped, a non-finite value has a high word of 0x7ff00000 or
+// more; n < 0 is a set sign bit on anything but -0 and a NaN.
 __device__ __forceinline__ unsigned check19(const double (&n)[Q])
 {
-    unsigned bad = 0;
+    bool neg = false, nonfinite = false;
 #pragma unroll
     for (int l = 0; l < Q; ++l) {
-        if (n[l] < 0.0) bad |= LBGPU_ERR_NEGATIVE_POPULATION;
-        if (!(fabs(n[l]) <= DBL_MAX)) bad |= LBGPU_ERR_NONFINITE;
+        const unsigned hi = (unsigned)__double2hiint(n[l]), lo = (unsigned)__double2loint(n[l]);
+        const unsigned mag = hi & 0x7fffffffu;
+        nonfinite |= mag >= 0x7ff00000u;
+        neg |= (int)hi < 0 && (mag | lo) != 0u && (mag < 0x7ff00000u || (mag == 0x7ff00000u && lo == 0u));
     }
-    return bad;
+    return (neg ? (unsigned)LBGPU_ERR_NEGATIVE_POPULATION : 0u) | (nonfinite ? (unsigned)LBGPU_ERR_NONFINITE : 0u);
 }
 
 __device__ __forceinline__ double warp_max(double v)
@@ -283,19 +332,20 @@ __device__ __forceinline__ unsigned warp_or(unsigned v)
     return v;
 }
 
-// Block-wide max/or; result valid in thread 0.
+// Block-wide max/or (any number of full warps up to BLOCK / 32); result valid in thread 0.
 __device__ __forceinline__ void block_max_or(double &err, unsigned &bad)
 {
     __shared__ double se[BLOCK / 32];
     __shared__ unsigned sb[BLOCK / 32];
     err = warp_max(err);
     bad = warp_or(bad);
+    if (blockDim.x == 32) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0) { se[wid] = err; sb[wid] = bad; }
     __syncthreads();
     if (wid == 0) {
-        err = lane < BLOCK / 32 ? se[lane] : 0.0;
-        bad = lane < BLOCK / 32 ? sb[lane] : 0u;
+        err = lane < (blockDim.x >> 5) ? se[lane] : 0.0;
+        bad = lane < (blockDim.x >> 5) ? sb[lane] : 0u;
         err = warp_max(err);
         bad = warp_or(bad);
     }
@@ -363,7 +413,7 @@ __global__ void __launch_bounds__(BLOCK) k_flow_step(const FlowArgs64 a)
     const long long N = a.N;
     // one thread per fluid node through the list (every lane of a warp does work), else one per
     // lattice node
-    const long long i = (long long)blockIdx.x * BLOCK + threadIdx.x;
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long node = a.fidx ? (i < a.Nf ? (long long)a.fidx[i] : N) : i;
     double err = 0.0;
     unsigned bad = 0;
@@ -403,8 +453,7 @@ __global__ void __launch_bounds__(BLOCK) k_flow_step(const FlowArgs64 a)
                 if (fc) collide_node_fused<FMASK, !FIELD>(n, rho, jx, jy, jz, fx, fy, fz, a);
                 else collide_node_fused<0, true>(n, rho, jx, jy, jz, 0.0, 0.0, 0.0, a);
             } else {
-                if (fc) collide_node<FMASK, !FIELD>(n, rho, jx, jy, jz, fx, fy, fz, a);
-                else collide_node<0, true>(n, rho, jx, jy, jz, 0.0, 0.0, 0.0, a);
+                collide_strict<FMASK, !FIELD>(n, rho, jx, jy, jz, fx, fy, fz, a, fc != 0);
             }
 #pragma unroll
             for (int l = 0; l < Q; ++l) dst[(long long)l * N + node] = n[l];
@@ -454,10 +503,8 @@ __global__ void __launch_bounds__(BLOCK) k_collide(const FlowArgs64 a)
             fy = a.F[1];
             fz = a.F[2];
         }
-        if (a.force_collide)
-            collide_node<FMASK, !FIELD>(n, a.rho[node], a.jx[node], a.jy[node], a.jz[node], fx, fy, fz, a);
-        else
-            collide_node<0, true>(n, a.rho[node], a.jx[node], a.jy[node], a.jz[node], 0.0, 0.0, 0.0, a);
+        collide_strict<FMASK, !FIELD>(n, a.rho[node], a.jx[node], a.jy[node], a.jz[node], fx, fy, fz, a,
+                                      a.force_collide != 0);
     }
 #pragma unroll
     for (int l = 0; l < Q; ++l) dst[(long long)l * N + node] = n[l];
@@ -549,43 +596,55 @@ __global__ void __launch_bounds__(BLOCK) k_init(const FlowArgs64 a, const double
 
 unsigned grid_of(long long N) { return (unsigned)((N + BLOCK - 1) / BLOCK); }
 
+// Threads per block of a step over n nodes.  A warp instruction of doubles occupies its quarter of
+// an SM for 64 cycles whatever its lanes, so a small box is spread over the SMs warp by warp: up to
+// 608 warps (152 SMs x 4 quarters) as one-warp blocks, then two-warp blocks until a block of eight
+// warps leaves no SM without its share (152 SMs x 8 blocks), where the fewer atomics of large
+// blocks win.
+unsigned step_block(long long n)
+{
+    const long long warps = (n + 31) / 32;
+    return warps <= 608 ? 32u : (warps <= 152 * 8 * (BLOCK / 32) ? 64u : (unsigned)BLOCK);
+}
+
 template <bool FIELD, bool CHECK, bool REF, bool FUSED>
-cudaError_t step_dispatch(const FlowArgs64 &a, int fmask, unsigned grid, cudaStream_t s)
+cudaError_t step_dispatch(const FlowArgs64 &a, int fmask, unsigned grid, unsigned block, cudaStream_t s)
 {
     switch (fmask) {
-    case 0: k_flow_step<0, FIELD, CHECK, REF, FUSED><<<grid, BLOCK, 0, s>>>(a); break;
-    case 1: k_flow_step<1, FIELD, CHECK, REF, FUSED><<<grid, BLOCK, 0, s>>>(a); break;
-    case 2: k_flow_step<2, FIELD, CHECK, REF, FUSED><<<grid, BLOCK, 0, s>>>(a); break;
-    case 4: k_flow_step<4, FIELD, CHECK, REF, FUSED><<<grid, BLOCK, 0, s>>>(a); break;
-    default: k_flow_step<7, FIELD, CHECK, REF, FUSED><<<grid, BLOCK, 0, s>>>(a); break;
+    case 0: k_flow_step<0, FIELD, CHECK, REF, FUSED><<<grid, block, 0, s>>>(a); break;
+    case 1: k_flow_step<1, FIELD, CHECK, REF, FUSED><<<grid, block, 0, s>>>(a); break;
+    case 2: k_flow_step<2, FIELD, CHECK, REF, FUSED><<<grid, block, 0, s>>>(a); break;
+    case 4: k_flow_step<4, FIELD, CHECK, REF, FUSED><<<grid, block, 0, s>>>(a); break;
+    default: k_flow_step<7, FIELD, CHECK, REF, FUSED><<<grid, block, 0, s>>>(a); break;
     }
     return cudaGetLastError();
 }
 
 template <bool FUSED>
 cudaError_t launch_step(const FlowArgs64 &a, int fmask, bool field, bool check, bool ref,
-                        unsigned grid, cudaStream_t s)
+                        unsigned grid, unsigned block, cudaStream_t s)
 {
     if (field) {
         // a per-node force field: every component may be non-zero
-        if (ref) k_flow_step<7, true, true, true, FUSED><<<grid, BLOCK, 0, s>>>(a);
-        else if (check) k_flow_step<7, true, true, false, FUSED><<<grid, BLOCK, 0, s>>>(a);
-        else k_flow_step<7, true, false, false, FUSED><<<grid, BLOCK, 0, s>>>(a);
+        if (ref) k_flow_step<7, true, true, true, FUSED><<<grid, block, 0, s>>>(a);
+        else if (check) k_flow_step<7, true, true, false, FUSED><<<grid, block, 0, s>>>(a);
+        else k_flow_step<7, true, false, false, FUSED><<<grid, block, 0, s>>>(a);
         return cudaGetLastError();
     }
-    if (ref) return step_dispatch<false, true, true, FUSED>(a, fmask, grid, s);
-    return check ? step_dispatch<false, true, false, FUSED>(a, fmask, grid, s)
-                 : step_dispatch<false, false, false, FUSED>(a, fmask, grid, s);
+    if (ref) return step_dispatch<false, true, true, FUSED>(a, fmask, grid, block, s);
+    return check ? step_dispatch<false, true, false, FUSED>(a, fmask, grid, block, s)
+                 : step_dispatch<false, false, false, FUSED>(a, fmask, grid, block, s);
 }
 
 }  // namespace
 
 cudaError_t launch_flow_step_f64(const FlowArgs64 &a, int fmask, bool field, bool check,
-                                 bool ref, unsigned grid, cudaStream_t s)
+                                 bool ref, cudaStream_t s)
 {
-    if (!grid) grid = grid_of(a.fidx ? a.Nf : a.N);
-    return a.fused ? launch_step<true>(a, fmask, field, check, ref, grid, s)
-                   : launch_step<false>(a, fmask, field, check, ref, grid, s);
+    const long long n = a.fidx ? a.Nf : a.N;
+    const unsigned block = step_block(n), grid = (unsigned)((n + block - 1) / block);
+    return a.fused ? launch_step<true>(a, fmask, field, check, ref, grid, block, s)
+                   : launch_step<false>(a, fmask, field, check, ref, grid, block, s);
 }
 
 cudaError_t launch_collide_f64(const FlowArgs64 &a, int fmask, bool field, cudaStream_t s)
