@@ -65,6 +65,11 @@ struct FlowArgs32 {
     // reference loop (lbgpu_equilibration): control block read by the AA launches, l2err history
     FlowCtl *ctl;
     double *hist;
+    // its population check: per weight class the smallest float not below -w rho0 (d < neg_below is
+    // n < 0), and the status bits of every node when rho0 itself is not finite
+    float neg_below[3];
+    unsigned bad_rho0;
+    double half_force[3];        // F/2 of the FP32 force
 };
 
 // FP64 strict ---------------------------------------------------------------------------

@@ -231,10 +231,53 @@ __device__ void control_step32(FlowCtl *c, double *hist, int phase)
     if (finish) c->done = 1;
 }
 
-// Check launch of the FP32 reference loop: FP64 moments of the AA state (natural order after
-// an odd launch, SWAPPED after an even one) with the state's moment force, max |j - j_old| over
-// the fluid nodes, n = d + w rho0 < 0 and non-finite tests, j stored for the next check; the
-// last block runs the control step.  A no-op once the loop has exited.
+// j of 19 FP32 deviations as doubles, each sum formed exactly in 64-bit integers and rounded once: a
+// deviation is its 24-bit significand shifted to a grid 33 bits below the largest one's (57 bits,
+// and the ten terms of a sum stay below 2^61); what lies below the grid is finer than the last bit
+// of a double of the largest deviation's size, so the sum is at least as accurate as FP64 additions
+// one by one.  Those would occupy the FP64 pipe, 19 SM cycles per warp instruction (16 per
+// conversion): 18 conversions and 30 additions, about 860 cycles per 32 nodes, against about 100 of
+// integer work here.
+__device__ __forceinline__ void exact_flux(const float (&f)[Q], double &jx, double &jy, double &jz)
+{
+    int emax = 1;
+#pragma unroll
+    for (int l = 1; l < Q; ++l) emax = max(emax, (int)((__float_as_uint(f[l]) >> 23) & 255u));
+    long long X = 0, Y = 0, Z = 0;
+    static_for<1, Q>([&](auto L) {
+        constexpr int l = decltype(L)::value;
+        constexpr Vel c = vel(l);
+        const unsigned b = __float_as_uint(f[l]);
+        const int e = (int)((b >> 23) & 255u);
+        const unsigned m = (b & 0x7fffffu) | (e ? 0x800000u : 0u);   // a denormal has no leading 1
+        const int up = 33 - (emax - max(e, 1));                      // <= 33
+        const long long v = up >= 0 ? (long long)((unsigned long long)m << up) : (long long)(m >> min(-up, 31));
+        const long long d = (int)b < 0 ? -v : v;
+        if constexpr (c.x > 0) X += d;
+        if constexpr (c.x < 0) X -= d;
+        if constexpr (c.y > 0) Y += d;
+        if constexpr (c.y < 0) Y -= d;
+        if constexpr (c.z > 0) Z += d;
+        if constexpr (c.z < 0) Z -= d;
+    });
+    // one unit of the sums is 2^(emax - 33 - 150) (emax = 255: a non-finite deviation, reported
+    // by the caller); the scaling adds to the exponent of the (normal) double
+    auto scaled = [&](long long v) {
+        const double r = (double)v;
+        return v == 0 ? 0.0 : __hiloint2double(__double2hiint(r) + (emax - 183) * (1 << 20), __double2loint(r));
+    };
+    jx = scaled(X);
+    jy = scaled(Y);
+    jz = scaled(Z);
+}
+
+// Check launch of the FP32 reference loop: j of the AA state (natural order after an odd launch,
+// SWAPPED after an even one) with the state's moment force, max |j - j_old| over the fluid nodes,
+// n = d + w rho0 < 0 and non-finite tests, j stored for the next check; the last block runs the
+// control step.  A no-op once the loop has exited.  n < 0 is d < -w rho0, and for a float d that is
+// d < neg_below, the smallest float not below -w rho0 (formed exactly on the host).
+// 61^3 touching spheres (74 k fluid nodes), AA launch and check: 36.4 us per step with FP64
+// moments (bound by the FP64 pipe), 16.5 with these.
 template <bool SWAPPED, typename Off = unsigned>
 __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
 {
@@ -247,6 +290,7 @@ __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
     if (i < a.Nf) {
         const unsigned c = a.cpos[i];
         const unsigned p = lattice_of(a, c);
+        const double ox = a.jx[p], oy = a.jy[p], oz = a.jz[p];
         const float *g = a.g0;
         float f[Q];
         if constexpr (SWAPPED) {
@@ -255,29 +299,27 @@ __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
 #pragma unroll
             for (int l = 0; l < Q; ++l) f[l] = g[(size_t)l * a.Nf + i];
         }
-        double drho = 0.0, jx = 0.0, jy = 0.0, jz = 0.0;
+        bool neg = false, nonfinite = false;
         static_for<0, Q>([&](auto L) {
             constexpr int l = decltype(L)::value;
-            constexpr Vel v = vel(l);
-            const double d = (double)f[l];
-            drho += d;
-            jx += v.x * d;
-            jy += v.y * d;
-            jz += v.z * d;
-            const double n = d + a.w64[wclass(l)] * a.rho0d;
-            if (n < 0.0) bad |= LBGPU_ERR_NEGATIVE_POPULATION;
-            if (!(fabs(n) <= DBL_MAX)) bad |= LBGPU_ERR_NONFINITE;
+            neg |= f[l] < a.neg_below[wclass(l)];
+            nonfinite |= !(fabsf(f[l]) <= FLT_MAX);
         });
+        bad = (neg ? (unsigned)LBGPU_ERR_NEGATIVE_POPULATION : 0u) | (nonfinite ? (unsigned)LBGPU_ERR_NONFINITE : 0u) |
+              a.bad_rho0;
+        double jx, jy, jz;
+        exact_flux(f, jx, jy, jz);
         if (fm) {
-            jx += 0.5 * (double)a.F[0];
-            jy += 0.5 * (double)a.F[1];
-            jz += 0.5 * (double)a.F[2];
+            jx += a.half_force[0];
+            jy += a.half_force[1];
+            jz += a.half_force[2];
         }
-        err = fmax(fmax(fabs(jx - a.jx[p]), fabs(jy - a.jy[p])), fabs(jz - a.jz[p]));
+        // a NaN difference (of a non-finite first state) is kept: the order of non-negative doubles
+        // and NaN is that of their bits
+        err = max_nonneg(max_nonneg(fabs(jx - ox), fabs(jy - oy)), fabs(jz - oz));
         a.jx[p] = jx;
         a.jy[p] = jy;
         a.jz[p] = jz;
-        a.rho[p] = a.rho0d + drho;
     }
     // block max of err (IEEE order of non-negative doubles = order of their bits) and OR of bad
     __shared__ unsigned long long smax;
@@ -287,7 +329,11 @@ __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
         sbad = 0u;
     }
     __syncthreads();
-    if (err > 0.0 || !(err == err)) atomicMax(&smax, (unsigned long long)__double_as_longlong(err == err ? err : INFINITY));
+    unsigned long long eb = (unsigned long long)__double_as_longlong(err);
+    if (eb > 0x7ff0000000000000ull) eb = 0x7ff0000000000000ull;   // a NaN difference counts as infinite
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, o));
+    if ((threadIdx.x & 31) == 0 && eb) atomicMax(&smax, eb);
     if (bad) atomicOr(&sbad, bad);
     __syncthreads();
     if (threadIdx.x == 0) {

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -64,6 +65,18 @@ static void fill_args32(lbgpu_ctx *ctx, FlowArgs32 &a)
         a.kF[p] = (float)(c3 * K.a1[wclass(l)] * cF);
         a.kT[p] = (float)(c3 * K.two_a2[wclass(l)] * cF);
     }
+}
+
+// The smallest float not below -w rho0, with the product taken exactly (its rounding error by a
+// fused multiply-add).
+static float smallest_float_from(double w, double rho0)
+{
+    const double p = -(w * rho0), rest = std::fma(-w, rho0, -p);   // -w rho0 = p + rest
+    auto below = [&](float f) { return (double)f < p || ((double)f == p && rest > 0.0); };
+    float f = (float)p;
+    while (below(f) && f < INFINITY) f = std::nextafterf(f, INFINITY);
+    while (f > -INFINITY && !below(std::nextafterf(f, -INFINITY))) f = std::nextafterf(f, -INFINITY);
+    return f;
 }
 
 int f32_flow_init(lbgpu_ctx *ctx)
@@ -292,6 +305,12 @@ int f32_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int his
     fill_args32(ctx, a);
     a.ctl = ctx->d_ctl;
     a.hist = d_hist;
+    for (int d = 0; d < 3; ++d) a.half_force[d] = 0.5 * (double)a.F[d];
+    const double rho0 = ctx->p.rho0;
+    if (std::isfinite(rho0))
+        for (int w = 0; w < 3; ++w) a.neg_below[w] = smallest_float_from(a.w64[w], rho0);
+    else
+        a.bad_rho0 = LBGPU_ERR_NONFINITE | (rho0 < 0.0 ? LBGPU_ERR_NEGATIVE_POPULATION : 0);
     // an even number of (AA, check) pairs per graph, so every replay starts at the same phase
     const int G = 2 * (int)std::min<long long>(128, std::max<long long>(4, (1LL << 23) / std::max<unsigned>(ctx->Nf, 1u)));
     cudaGraph_t graph;
