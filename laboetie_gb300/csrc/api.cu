@@ -336,7 +336,8 @@ int lbgpu_host_unregister(void *ptr)
 int lbgpu_sync(lbgpu_ctx *ctx)
 {
     if (!ctx) return LBGPU_ERR_INVALID;
-    return ctx_cuda(ctx, cudaStreamSynchronize(ctx->stream), "lbgpu_sync");
+    if (int rc = ctx_cuda(ctx, cudaStreamSynchronize(ctx->stream), "lbgpu_sync")) return rc;
+    return resident_status(ctx);
 }
 
 }  // extern "C"

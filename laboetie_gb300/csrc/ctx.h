@@ -7,6 +7,7 @@
 #include <string>
 
 #include "common.cuh"
+#include "flow.h"
 #include "lbgpu.h"
 
 namespace lbg {
@@ -79,6 +80,10 @@ struct lbgpu_ctx {
     unsigned Nf = 0;
     bool aa_wide = false;        // Q*Nf >= 2^32 (or LBGPU_AA_WIDE=1): 64-bit gather offsets
     int nw = 0, xbits = 0, ybits = 0;
+    // many steps per launch (flow_f32_resident.cu) where the box is small enough (blocks > 0)
+    lbg::ResidentPlan resident{}, resident_loop{};   // fixed steps, reference loop
+    void *d_gsync = nullptr;
+    bool resident_unchecked = false;   // a grid launch whose waits' outcome has not been read
     uint32_t *d_cpos = nullptr, *d_cmask = nullptr;
     uint2 *d_rowtab = nullptr;
 
@@ -110,6 +115,8 @@ void mp_release(lbgpu_ctx *ctx);
 void pnp_release(lbgpu_ctx *ctx);
 // device potential phi of the Poisson-Nernst-Planck state (N doubles), or null without one
 const double *pnp_potential(const lbgpu_ctx *ctx);
+// LBGPU_ERR_TIMEOUT if a wait of a resident launch since the last call ran out (waits for the stream)
+int resident_status(lbgpu_ctx *ctx);
 // The device address of the host range [p, p + bytes) if it lies inside one range page-locked by
 // lbgpu_host_register (kernels may then read it in place), else null.
 const void *pinned_device_view(const void *p, size_t bytes);

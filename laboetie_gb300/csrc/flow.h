@@ -89,6 +89,21 @@ cudaError_t launch_finalize_f64(const FlowArgs64 &a, bool field, cudaStream_t s)
 cudaError_t launch_init_f64(const FlowArgs64 &a, double rho0, cudaStream_t s);
 
 // FP32 deviation ------------------------------------------------------------------------
+// many steps of one box in one launch (flow_f32_resident.cu): blocks 0 when the box is not run so
+struct ResidentPlan {
+    unsigned blocks, threads;
+    bool cluster;
+};
+ResidentPlan plan_resident32(unsigned Nf, bool wide, bool loop);   // fixed steps, or the reference loop
+size_t grid_sync_bytes();   // device bytes of `sync` below
+// nsteps fixed steps from AA phase `phase`: moment / collision forces fm0 / fc0 in the first, then
+// fc0 / fon, then fon / fon.  A wait that ran out sets LBGPU_ERR_TIMEOUT in a.ctl->status.
+cudaError_t launch_resident_steps32(const ResidentPlan &plan, const FlowArgs32 &a, void *sync, int nsteps, int phase,
+                                    int fm0, int fc0, int fon, cudaStream_t s);
+// at most nsteps steps of the reference loop on the control block a.ctl (as pairs of AA and check
+// launches would leave it), j_old in a.jx..jz
+cudaError_t launch_resident_loop32(const ResidentPlan &plan, const FlowArgs32 &a, void *sync, int nsteps, int phase,
+                                   cudaStream_t s);
 cudaError_t launch_flow_step_f32(const FlowArgs32 &a, unsigned grid, cudaStream_t s);
 cudaError_t launch_init_f32(const FlowArgs32 &a, cudaStream_t s);
 // AA layout: flag word of every compact node

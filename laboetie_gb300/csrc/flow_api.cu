@@ -171,6 +171,9 @@ int ctx_init_device(lbgpu_ctx *ctx, const int8_t *nature)
             int rc = build_compact_layout(ctx, nature);
             if (rc) return rc;
             LBG_CK(ctx, dalloc(&ctx->d_g[0], (size_t)Q * ctx->Nf));
+            ctx->resident = plan_resident32(ctx->Nf, ctx->aa_wide, false);
+            ctx->resident_loop = plan_resident32(ctx->Nf, ctx->aa_wide, true);
+            if (ctx->resident.blocks || ctx->resident_loop.blocks) LBG_CK(ctx, cudaMalloc(&ctx->d_gsync, grid_sync_bytes()));
         } else {
             for (int b = 0; b < 2; ++b) LBG_CK(ctx, dalloc(&ctx->d_g[b], (size_t)Q * N));
         }
@@ -198,6 +201,7 @@ void ctx_release_device(lbgpu_ctx *ctx)
     cudaFree(ctx->d_cpos);
     cudaFree(ctx->d_cmask);
     cudaFree(ctx->d_rowtab);
+    cudaFree(ctx->d_gsync);
     for (int b = 0; b < 2; ++b) {
         cudaFree(ctx->d_f[b]);
         cudaFree(ctx->d_g[b]);

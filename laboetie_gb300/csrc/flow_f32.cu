@@ -14,6 +14,7 @@
 #include <cfloat>
 #include <type_traits>
 
+#include "aa32.cuh"
 #include "collide32.cuh"
 #include "common.cuh"
 #include "compact.cuh"
@@ -134,24 +135,7 @@ __device__ __forceinline__ void aa_update(const FlowArgs32 &a, unsigned i, uint3
 #pragma unroll
         for (int l = 0; l < Q; ++l, q += Nf) f[l] = __ldg(q);
     }
-    float drho = 0.0f, jx = 0.0f, jy = 0.0f, jz = 0.0f;
-    static_for<0, Q>([&](auto L) {
-        constexpr int l = decltype(L)::value;
-        constexpr Vel c = vel(l);
-        drho += f[l];
-        if constexpr (c.x > 0) jx += f[l];
-        if constexpr (c.x < 0) jx -= f[l];
-        if constexpr (c.y > 0) jy += f[l];
-        if constexpr (c.y < 0) jy -= f[l];
-        if constexpr (c.z > 0) jz += f[l];
-        if constexpr (c.z < 0) jz -= f[l];
-    });
-    if (FMASK && fm) {
-        jx = __fadd_rn(jx, __fmul_rn(0.5f, a.F[0]));
-        jy = __fadd_rn(jy, __fmul_rn(0.5f, a.F[1]));
-        jz = __fadd_rn(jz, __fmul_rn(0.5f, a.F[2]));
-    }
-    collide_dev<FMASK>(f, drho, jx, jy, jz, a, fc != 0);
+    aa_relax<FMASK>(f, a, fm, fc);
     if constexpr (ODD) {
         // the population leaving along l goes to the slot the opposite direction was read from
 #pragma unroll
@@ -177,98 +161,15 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_aa32(const FlowArgs32 a)
     __shared__ Off soff[ODD ? Q : 1][BLOCK];
     int fm = a.force_moment, fc = a.force_collide;
     if constexpr (LOOP) {   // reference loop: forces decided on the device; no-op after the exit
-        const volatile FlowCtl *c = a.ctl;
-        if (c->done) return;
-        fm = c->aa_fm;
-        fc = c->aa_fc;
+        if (a.ctl->done) return;
+        fm = a.ctl->aa_fm;
+        fc = a.ctl->aa_fc;
     }
     const unsigned blk = ODD ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
     const unsigned i = blk * BLOCK + threadIdx.x;   // compact (fluid) node
     if (i >= a.Nf) return;
     if constexpr (!ODD) aa_update<false, FMASK>(a, i, 0u, 0u, soff, fm, fc);
     else aa_update<true, FMASK>(a, i, __ldg(a.cmask + i), __ldg(a.cpos + i), soff, fm, fc);
-}
-
-// Control step of the FP32 reference loop, run by the last block of a check launch: the
-// equilibration.f90:339-489 decisions (l2err history, convergence at l2err <= target_error and
-// t > 2, f_ext from the next collision on at the first convergence, exit at the second) for the
-// state S_t of step t.  Unlike the FP64 fused step no step is repeated: the decision is taken
-// before the AA launch of step t+1 collides S_t.
-__device__ void control_step32(FlowCtl *c, double *hist, int phase)
-{
-    const unsigned long long eb = atomicExch(&c->err_bits, 0ull);
-    const double l2 = __longlong_as_double((long long)eb);
-    c->blocks_done = 0;
-    const unsigned st = atomicOr(&c->status, 0u);
-    const int t = c->t;
-    const int fm = c->check_fm;   // moment force of S_t
-    bool finish = false;
-    if (st & (LBGPU_ERR_NEGATIVE_POPULATION | LBGPU_ERR_NONFINITE)) {
-        finish = true;
-    } else {
-        if (hist && t - 1 < c->hist_cap) hist[t - 1] = l2;
-        c->last_l2err = l2;
-        if (l2 <= c->target_error && t > 2) {
-            if (!c->conv_without) {
-                c->conv_without = 1;
-                c->aa_fc = 1;          // f_ext acts from the collision of step t+1 on
-            } else {
-                c->conv_with = 1;
-                finish = true;
-            }
-        }
-    }
-    c->exit_force_moment = fm;
-    c->exit_step = t;
-    c->exit_phase = phase;
-    c->aa_fm = fm;
-    c->check_fm = c->aa_fc;        // S_{t+1} = collide(S_t) with aa_fc: its moments carry it
-    c->t = t + 1;
-    if (!finish && c->max_steps > 0 && t >= c->max_steps) {
-        finish = true;
-        atomicOr(&c->status, (unsigned)LBGPU_ERR_STEP_CAP);
-    }
-    if (finish) c->done = 1;
-}
-
-// j of 19 FP32 deviations as doubles, each sum formed exactly in 64-bit integers and rounded once: a
-// deviation is its 24-bit significand shifted to a grid 33 bits below the largest one's (57 bits,
-// and the ten terms of a sum stay below 2^61); what lies below the grid is finer than the last bit
-// of a double of the largest deviation's size, so the sum is at least as accurate as FP64 additions
-// one by one.  Those would occupy the FP64 pipe, 19 SM cycles per warp instruction (16 per
-// conversion): 18 conversions and 30 additions, about 860 cycles per 32 nodes, against about 100 of
-// integer work here.
-__device__ __forceinline__ void exact_flux(const float (&f)[Q], double &jx, double &jy, double &jz)
-{
-    int emax = 1;
-#pragma unroll
-    for (int l = 1; l < Q; ++l) emax = max(emax, (int)((__float_as_uint(f[l]) >> 23) & 255u));
-    long long X = 0, Y = 0, Z = 0;
-    static_for<1, Q>([&](auto L) {
-        constexpr int l = decltype(L)::value;
-        constexpr Vel c = vel(l);
-        const unsigned b = __float_as_uint(f[l]);
-        const int e = (int)((b >> 23) & 255u);
-        const unsigned m = (b & 0x7fffffu) | (e ? 0x800000u : 0u);   // a denormal has no leading 1
-        const int up = 33 - (emax - max(e, 1));                      // <= 33
-        const long long v = up >= 0 ? (long long)((unsigned long long)m << up) : (long long)(m >> min(-up, 31));
-        const long long d = (int)b < 0 ? -v : v;
-        if constexpr (c.x > 0) X += d;
-        if constexpr (c.x < 0) X -= d;
-        if constexpr (c.y > 0) Y += d;
-        if constexpr (c.y < 0) Y -= d;
-        if constexpr (c.z > 0) Z += d;
-        if constexpr (c.z < 0) Z -= d;
-    });
-    // one unit of the sums is 2^(emax - 33 - 150) (emax = 255: a non-finite deviation, reported
-    // by the caller); the scaling adds to the exponent of the (normal) double
-    auto scaled = [&](long long v) {
-        const double r = (double)v;
-        return v == 0 ? 0.0 : __hiloint2double(__double2hiint(r) + (emax - 183) * (1 << 20), __double2loint(r));
-    };
-    jx = scaled(X);
-    jy = scaled(Y);
-    jz = scaled(Z);
 }
 
 // Check launch of the FP32 reference loop: j of the AA state (natural order after an odd launch,
@@ -281,11 +182,12 @@ __device__ __forceinline__ void exact_flux(const float (&f)[Q], double &jx, doub
 template <bool SWAPPED, typename Off = unsigned>
 __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
 {
-    const volatile FlowCtl *vc = a.ctl;
-    if (vc->done) return;
-    const int fm = vc->check_fm;
+    // the control block is written by the last block only, after every block has read it: plain
+    // loads, which one request per SM serves
+    if (a.ctl->done) return;
+    const int fm = a.ctl->check_fm;
     const unsigned i = blockIdx.x * BLOCK + threadIdx.x;
-    double err = 0.0;
+    unsigned long long err = 0;
     unsigned bad = 0;
     if (i < a.Nf) {
         const unsigned c = a.cpos[i];
@@ -299,14 +201,7 @@ __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
 #pragma unroll
             for (int l = 0; l < Q; ++l) f[l] = g[(size_t)l * a.Nf + i];
         }
-        bool neg = false, nonfinite = false;
-        static_for<0, Q>([&](auto L) {
-            constexpr int l = decltype(L)::value;
-            neg |= f[l] < a.neg_below[wclass(l)];
-            nonfinite |= !(fabsf(f[l]) <= FLT_MAX);
-        });
-        bad = (neg ? (unsigned)LBGPU_ERR_NEGATIVE_POPULATION : 0u) | (nonfinite ? (unsigned)LBGPU_ERR_NONFINITE : 0u) |
-              a.bad_rho0;
+        bad = check_dev19(f, a);
         double jx, jy, jz;
         exact_flux(f, jx, jy, jz);
         if (fm) {
@@ -314,14 +209,12 @@ __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
             jy += a.half_force[1];
             jz += a.half_force[2];
         }
-        // a NaN difference (of a non-finite first state) is kept: the order of non-negative doubles
-        // and NaN is that of their bits
-        err = max_nonneg(max_nonneg(fabs(jx - ox), fabs(jy - oy)), fabs(jz - oz));
+        err = flux_change_bits(jx - ox, jy - oy, jz - oz);
         a.jx[p] = jx;
         a.jy[p] = jy;
         a.jz[p] = jz;
     }
-    // block max of err (IEEE order of non-negative doubles = order of their bits) and OR of bad
+    // block max of err and OR of bad
     __shared__ unsigned long long smax;
     __shared__ unsigned sbad;
     if (threadIdx.x == 0) {
@@ -329,11 +222,12 @@ __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
         sbad = 0u;
     }
     __syncthreads();
-    unsigned long long eb = (unsigned long long)__double_as_longlong(err);
-    if (eb > 0x7ff0000000000000ull) eb = 0x7ff0000000000000ull;   // a NaN difference counts as infinite
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, o));
-    if ((threadIdx.x & 31) == 0 && eb) atomicMax(&smax, eb);
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(0xffffffffu, err, o);
+        err = v > err ? v : err;
+    }
+    if ((threadIdx.x & 31) == 0 && err) atomicMax(&smax, err);
     if (bad) atomicOr(&sbad, bad);
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -343,7 +237,13 @@ __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
         __threadfence();
         if (atomicAdd(&c->blocks_done, 1u) == gridDim.x - 1) {
             __threadfence();
-            control_step32(c, a.hist, SWAPPED ? 1 : 0);
+            const unsigned long long eb = atomicExch(&c->err_bits, 0ull);
+            const unsigned st = atomicOr(&c->status, 0u);
+            FlowCtl d = *c;
+            d.err_bits = 0ull;
+            d.blocks_done = 0u;
+            decide32(d, eb, st, SWAPPED ? 1 : 0, a.hist);
+            *c = d;
         }
     }
 }

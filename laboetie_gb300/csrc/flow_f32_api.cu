@@ -135,8 +135,21 @@ int f32_flow_set(lbgpu_ctx *ctx, const double *n, const double *density, const d
     return LBGPU_OK;
 }
 
+int resident_status(lbgpu_ctx *ctx)
+{
+    if (!ctx->resident_unchecked) return LBGPU_OK;
+    ctx->resident_unchecked = false;
+    unsigned st = 0;
+    LBG_CK(ctx, cudaMemcpyAsync(&st, &ctx->d_ctl->status, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
+    LBG_CK(ctx, cudaStreamSynchronize(ctx->stream));
+    if (!(st & LBGPU_ERR_TIMEOUT)) return LBGPU_OK;
+    LBG_CK(ctx, cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(st), ctx->stream));   // reported once
+    return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, "flow steps: a block did not reach the grid's barrier within its wait limit");
+}
+
 int f32_flow_get(lbgpu_ctx *ctx, double *n, double *density, double *jx, double *jy, double *jz)
 {
+    if (int rc = resident_status(ctx)) return rc;
     if (ctx->prev_kind == PREV_NONE)
         return ctx_fail(ctx, LBGPU_ERR_INVALID, "lbgpu_flow_get: no flow state (call lbgpu_flow_init)");
     const long long N = ctx->N;
@@ -233,7 +246,30 @@ static int aa_steps(lbgpu_ctx *ctx, int nsteps, int force_on, float *ms)
         return LBGPU_OK;
     };
     int rc;
+    // resident boxes: RES_CHUNK steps per launch (a launch of them stays within some 10 ms); a few
+    // steps are not worth a resident launch's set-up, about three steps' time
+    constexpr int RES_CHUNK = 4096, RES_MIN = 8;
+    const bool resident = ctx->resident.blocks > 0 && nsteps >= RES_MIN;
+    auto resident_steps = [&]() -> int {
+        for (int left = nsteps; left > 0;) {
+            const int n = std::min(left, RES_CHUNK);
+            left -= n;
+            LBG_CK(ctx, launch_resident_steps32(ctx->resident, a, ctx->d_gsync, n, ctx->aa_phase, ctx->prev_force_moment,
+                                                ctx->force_last_collide, force_on, s));
+            ctx->aa_phase ^= n & 1;
+            ctx->prev_force_moment = n >= 2 ? force_on : ctx->force_last_collide;
+            ctx->force_last_collide = force_on;
+        }
+        ctx->prev_kind = PREV_POST;
+        ctx->resident_unchecked = !ctx->resident.cluster;
+        return LBGPU_OK;
+    };
+    a.ctl = nullptr;
     if (!ms) {
+        if (resident) {
+            a.ctl = ctx->d_ctl;
+            return resident_steps();
+        }
         for (int t = 0; t < nsteps; ++t)
             if ((rc = one())) return rc;
         return LBGPU_OK;
@@ -243,6 +279,15 @@ static int aa_steps(lbgpu_ctx *ctx, int nsteps, int force_on, float *ms)
     while ((ctx->prev_force_moment != force_on || ctx->force_last_collide != force_on ||
             ctx->aa_phase != 0) && guard++ < 4)
         if ((rc = one())) return rc;
+    if (resident) {
+        a.ctl = ctx->d_ctl;
+        LBG_CK(ctx, cudaEventRecord(ctx->ev0, s));
+        if ((rc = resident_steps())) return rc;
+        LBG_CK(ctx, cudaEventRecord(ctx->ev1, s));
+        LBG_CK(ctx, cudaEventSynchronize(ctx->ev1));
+        LBG_CK(ctx, cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1));
+        return resident_status(ctx);
+    }
     if (!ctx->graph_fixed[force_on] || ctx->graph_fixed_parity[force_on] != 0) {
         if (ctx->graph_fixed[force_on]) cudaGraphExecDestroy(ctx->graph_fixed[force_on]);
         cudaGraph_t g;
@@ -311,37 +356,49 @@ int f32_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int his
         for (int w = 0; w < 3; ++w) a.neg_below[w] = smallest_float_from(a.w64[w], rho0);
     else
         a.bad_rho0 = LBGPU_ERR_NONFINITE | (rho0 < 0.0 ? LBGPU_ERR_NEGATIVE_POPULATION : 0);
-    // an even number of (AA, check) pairs per graph, so every replay starts at the same phase
-    const int G = 2 * (int)std::min<long long>(128, std::max<long long>(4, (1LL << 23) / std::max<unsigned>(ctx->Nf, 1u)));
-    cudaGraph_t graph;
-    cudaGraphExec_t exec;
-    LBG_CK(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < G; ++k) {
-        const bool odd = ((ctx->aa_phase + k) & 1) != 0;   // an even launch leaves the state swapped
-        cudaError_t e = launch_aa_step_f32(a, odd, s);
-        if (e == cudaSuccess) e = launch_aa_check_f32(a, !odd, s);
-        if (e != cudaSuccess) {
-            cudaStreamEndCapture(s, &graph);
-            return ctx_cuda(ctx, e, "capture FP32 reference loop");
+    const bool resident = ctx->resident_loop.blocks > 0;
+    cudaGraphExec_t exec = nullptr;
+    if (!resident) {
+        // an even number of (AA, check) pairs per graph, so every replay starts at the same phase
+        const int G = 2 * (int)std::min<long long>(128, std::max<long long>(4, (1LL << 23) / std::max<unsigned>(ctx->Nf, 1u)));
+        cudaGraph_t graph;
+        LBG_CK(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        for (int k = 0; k < G; ++k) {
+            const bool odd = ((ctx->aa_phase + k) & 1) != 0;   // an even launch leaves the state swapped
+            cudaError_t e = launch_aa_step_f32(a, odd, s);
+            if (e == cudaSuccess) e = launch_aa_check_f32(a, !odd, s);
+            if (e != cudaSuccess) {
+                cudaStreamEndCapture(s, &graph);
+                return ctx_cuda(ctx, e, "capture FP32 reference loop");
+            }
         }
+        LBG_CK(ctx, cudaStreamEndCapture(s, &graph));
+        LBG_CK(ctx, cudaGraphInstantiate(&exec, graph, 0));
+        cudaGraphDestroy(graph);
     }
-    LBG_CK(ctx, cudaStreamEndCapture(s, &graph));
-    LBG_CK(ctx, cudaGraphInstantiate(&exec, graph, 0));
-    cudaGraphDestroy(graph);
     FlowCtl h;
+    int phase = ctx->aa_phase;
     rc = LBGPU_OK;
     for (;;) {
-        cudaError_t e = cudaGraphLaunch(exec, s);
+        constexpr int RES_CHUNK = 2048;   // steps of a resident launch: some milliseconds
+        cudaError_t e = resident ? launch_resident_loop32(ctx->resident_loop, a, ctx->d_gsync, RES_CHUNK, phase, s)
+                                 : cudaGraphLaunch(exec, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h, ctx->d_ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             rc = ctx_cuda(ctx, e, "lbgpu_equilibration (FP32)");
             break;
         }
+        phase = h.exit_phase;
         if (h.done) break;
     }
-    cudaGraphExecDestroy(exec);
+    if (exec) cudaGraphExecDestroy(exec);
     if (rc) return rc;
+    if (h.status & LBGPU_ERR_TIMEOUT) {
+        LBG_CK(ctx, cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(h.status), s));
+        if (d_hist) cudaFreeAsync(d_hist, s);
+        return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, "equilibration: a block did not reach the grid's barrier within its wait limit");
+    }
     ctx->aa_phase = h.exit_phase;
     ctx->prev_force_moment = h.exit_force_moment;
     ctx->force_last_collide = h.aa_fc;

@@ -1,0 +1,109 @@
+// gridsync.cuh -- a barrier over the blocks of one cooperative launch that also forms the maximum of
+// a 64-bit value and the OR of status bits over the grid.
+//
+// Thread 0 of a block adds the block's values to the round's slot, arrives on a counter (release)
+// and polls it (acquire) until every block has arrived.  The three slots rotate: after a round has
+// passed, the slot of the round before it is read by nobody any more and is cleared for the round
+// after next.  The poll is bounded; a block whose wait runs out reports it and the kernel ends.
+// 152 blocks: 1.2 us without values, 1.6 us with them (a launch in a CUDA graph costs 1.04 us, and
+// a step that decides on a reduction needs its tail besides).
+#pragma once
+
+#include <cstdint>
+
+#include "tma.cuh"
+
+namespace lbg {
+
+struct alignas(128) GridSync {
+    struct alignas(128) Slot {
+        unsigned long long value;
+        unsigned bits;
+    } slot[3];
+    alignas(128) unsigned arrived;
+};
+
+// How a launch waits: the limit of each wait, and arrivals to wait for beyond the grid's own (0; a
+// test sets 1, so that the wait runs out without any fault).
+struct GridWait {
+    unsigned long long limit_ns;
+    unsigned extra;
+};
+
+__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p)
+{
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// The grid's rendezvous number `round` (0, 1, ...; all blocks count alike, and the structure is zero
+// before the launch).  VALUES: value / bits become the maximum / OR over every thread of the grid.
+// False, in every thread of the block, when the wait ran out.  Data that other blocks wrote before it
+// must be read from L2 (__ldcg).
+template <bool VALUES>
+__device__ __forceinline__ bool grid_barrier(GridSync *g, unsigned round, const GridWait &wait,
+                                             unsigned long long &value, unsigned &bits)
+{
+    __shared__ unsigned long long sval[32], rval;
+    __shared__ unsigned sbit[32], rbit;
+    __shared__ int ok;
+    if constexpr (VALUES) {
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, value, o);
+            value = v > value ? v : value;
+        }
+        bits = __reduce_or_sync(0xffffffffu, bits);
+        if (lane == 0) {
+            sval[wid] = value;
+            sbit[wid] = bits;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        GridSync::Slot *s = &g->slot[round % 3u];
+        if constexpr (VALUES) {
+            for (unsigned w = 1; w < (blockDim.x >> 5); ++w) {
+                value = sval[w] > value ? sval[w] : value;
+                bits |= sbit[w];
+            }
+            if (value) atomicMax(&s->value, value);
+            if (bits) atomicOr(&s->bits, bits);
+        }
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&g->arrived) : "memory");
+        const unsigned target = (round + 1u) * (gridDim.x + wait.extra);
+        bool done = false;
+        unsigned long long t0 = 0;
+        for (unsigned it = 0; it < (1u << 28); ++it) {
+            if (ld_acquire_gpu(&g->arrived) >= target) {
+                done = true;
+                break;
+            }
+            if ((it & 255u) == 255u) {
+                const unsigned long long t = global_ns();
+                if (t0 == 0) t0 = t;
+                else if (t - t0 > wait.limit_ns) break;
+            }
+        }
+        if constexpr (VALUES) {
+            rval = __ldcg(&s->value);
+            rbit = __ldcg(&s->bits);
+        }
+        if (blockIdx.x == 0 && done) {
+            GridSync::Slot *z = &g->slot[(round + 2u) % 3u];
+            z->value = 0;
+            z->bits = 0;
+        }
+        ok = done;
+    }
+    __syncthreads();
+    if constexpr (VALUES) {
+        value = rval;
+        bits = rbit;
+    }
+    return ok != 0;
+}
+
+}  // namespace lbg
