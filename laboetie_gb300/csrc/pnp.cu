@@ -24,6 +24,7 @@
 #include "lbgpu.h"
 #include "trace.h"
 #include "pnp.h"
+#include "pnp_args.cuh"
 #include "reduce.cuh"
 
 namespace lbg {
@@ -61,45 +62,6 @@ void pnp_release(lbgpu_ctx *ctx)
 }
 
 namespace {
-
-struct PnpArgs {
-    const uint32_t *mask;
-    const double *phi;
-    double *phi_out;
-    const double *cp, *cm;
-    double *fp, *fm;
-    double *partial;
-    PnpCtl *ctl;
-    long long N;
-    int lx, ly, lz;
-    double a0[3];
-    double factor, omega, one_minus_omega;
-    double eDp, eDm;
-    double delta_axis, delta_diag;
-    int color;        // multicolour SOR: the colour of this launch
-    int ncolor;       // colours per sweep (the last colour's launch decides the stopping test)
-    int gen;          // general colouring (some side odd): colour from k_sor_color_gen's rule
-    int kx, ky, kz;   // colours per axis of the general colouring (1, 2 or 3)
-    int loop_bug;     // just_eq_smolu.f90:68-70
-};
-
-__device__ __forceinline__ void coords(long long r, int lx, int ly, int &x, int &y, int &z)
-{
-    const unsigned nd = (unsigned)r;
-    x = (int)(nd % (unsigned)lx);
-    const unsigned yz = nd / (unsigned)lx;
-    y = (int)(yz % (unsigned)ly);
-    z = (int)(yz / (unsigned)ly);
-}
-
-// offset of (x + dx, y + dy, z + dz), periodic, dx.. in {-1,0,1}
-__device__ __forceinline__ long long nb(int x, int y, int z, int dx, int dy, int dz, int lx, int ly, int lz)
-{
-    const int xx = dx > 0 ? wrap_plus(x, lx) : (dx < 0 ? wrap_minus(x, lx) : x);
-    const int yy = dy > 0 ? wrap_plus(y, ly) : (dy < 0 ? wrap_minus(y, ly) : y);
-    const int zz = dz > 0 ? wrap_plus(z, lz) : (dz < 0 ? wrap_minus(z, lz) : z);
-    return xx + (long long)lx * (yy + (long long)ly * zz);
-}
 
 // Final sum of the 4-value block partials of the last kernel, in block order.
 // The control block of a solve, set on the device (a kernel parameter, no staged host copy).
@@ -142,37 +104,94 @@ __device__ __forceinline__ void block_partial4(double (&t)[4], double *partial)
     }
 }
 
-// sor.f90:48-70 one Jacobi sweep over every node (solid included), then the stopping test of
-// sor.f90:78 by the last block.
-__global__ void __launch_bounds__(PB) k_sor_jacobi(const PnpArgs a, double *phi0, double *phi1)
+// Sum of one value per thread over the grid, in a fixed order (32 strided lanes of the first warp,
+// then the blocks in order by the last one), to finish(total) in one thread.  The first warp alone
+// adds the block's values: a shuffle tree in each of its 8 warps would issue 40 FP64 instructions
+// against 12.
+template <typename Fin>
+__device__ __forceinline__ void grid_sum1(double v, double *partial, unsigned *counter, Fin &&finish)
 {
-    const volatile PnpCtl *vc = a.ctl;
-    if (vc->done) return;
-    const int par = vc->parity;
+    __shared__ double sh[PB];
+    __shared__ bool last;
+    auto warp_total = [&]() {
+        double s = 0.0;
+        for (unsigned k = threadIdx.x; k < PB; k += 32u) s = s + sh[k];
+        return warp_sum_fixed(s);
+    };
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const double s = warp_total();
+        if (threadIdx.x == 0) {
+            partial[blockIdx.x] = s;
+            __threadfence();
+            last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        }
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double t = 0.0;
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += PB) t += __ldcg(partial + i);
+    sh[threadIdx.x] = t;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        t = warp_total();
+        if (threadIdx.x == 0) {
+            *counter = 0;
+            finish(t);
+        }
+    }
+}
+
+// sor.f90:48-70 one Jacobi sweep over every node (solid included), then the stopping test of
+// sor.f90:78 by the last block.  The first sweep of a solve multiplies each neighbour's phi by its
+// weight and leaves w_axis phi (t) and the right-hand side for the others, which add t, or its exact
+// half for a diagonal neighbour (pnp_resident.cu): 26 FP64 instructions per node instead of 45.
+template <bool FIRST>
+__global__ void __launch_bounds__(PB) k_sor_jacobi(const PnpArgs a, double *phi0, double *phi1, double *t0, double *t1,
+                                                   double *rhs)
+{
+    if (a.ctl->done) return;   // written by the last block only, after every block has read it
+    const int par = a.ctl->parity;
     const double *__restrict__ src = par ? phi1 : phi0;
+    const double *__restrict__ tsrc = par ? t1 : t0;
     double *__restrict__ dst = par ? phi0 : phi1;
-    double t[3] = {0.0, 0.0, 0.0};
+    double *__restrict__ tdst = par ? t0 : t1;
+    double err = 0.0;
     for (long long r = (long long)blockIdx.x * PB + threadIdx.x; r < a.N; r += (long long)gridDim.x * PB) {
         int x, y, z;
         coords(r, a.lx, a.ly, x, y, z);
-        double phistar = 0.0;
-        static_for<0, Q>([&](auto L) {
+        const double phiold = src[r];
+        double phistar = a.a0[0] * phiold;
+        static_for<1, Q>([&](auto L) {
             constexpr int l = decltype(L)::value;
             constexpr Vel c = vel(l);
             // phi(pbc(i - c_l)) (sor.f90:54-57)
-            phistar = phistar + a.a0[wclass(l)] * src[nb(x, y, z, -c.x, -c.y, -c.z, a.lx, a.ly, a.lz)];
+            const long long s = nb(x, y, z, -c.x, -c.y, -c.z, a.lx, a.ly, a.lz);
+            if constexpr (FIRST) phistar = phistar + a.a0[wclass(l)] * src[s];
+            else if constexpr (wclass(l) == 1) phistar = phistar + tsrc[s];
+            else phistar = __fma_rn(0.5, tsrc[s], phistar);
         });
-        phistar = phistar + a.factor * (a.cp[r] - a.cm[r]);
-        const double phiold = src[r];
-        dst[r] = a.omega * phistar + a.one_minus_omega * phiold;
-        t[0] = t[0] + fabs(phistar - phiold);
+        double q;
+        if constexpr (FIRST) {
+            q = a.factor * (a.cp[r] - a.cm[r]);
+            rhs[r] = q;
+        } else {
+            q = rhs[r];
+        }
+        phistar = phistar + q;
+        const double phi = a.omega * phistar + a.one_minus_omega * phiold;
+        dst[r] = phi;
+        tdst[r] = a.a0[1] * phi;
+        err = err + fabs(phistar - phiold);
     }
-    grid_sum3(t, a.partial, &a.ctl->blocks_done, [&](const double (&tot)[3]) {
+    grid_sum1(err, a.partial, &a.ctl->blocks_done, [&](double tot) {
         PnpCtl *c = a.ctl;
-        c->anorm = tot[0];
+        c->anorm = tot;
         c->parity ^= 1;  // phi = phitmp (sor.f90:70)
         c->iter += 1;
-        if (tot[0] <= c->limit) {
+        if (tot <= c->limit) {
             c->converged = 1;
             c->done = 1;
         } else if (c->iter >= c->max_iter) {
@@ -317,12 +336,7 @@ __global__ void __launch_bounds__(PB) k_shift_phi(double *phi, long long N, doub
 __device__ __forceinline__ void link_flux(const PnpArgs &k, long long ra, long long rb, double delta,
                                           double &Jp, double &Jm)
 {
-    const double e = exp(k.phi[rb] - k.phi[ra]);
-    const double em = 1.0 / e;
-    Jp = 0.5 * (1.0 + em) * (k.cp[rb] * e - k.cp[ra]);
-    Jp = Jp * k.eDp / delta;
-    Jm = 0.5 * (1.0 + e) * (k.cm[rb] * em - k.cm[ra]);
-    Jm = Jm * k.eDm / delta;
+    link_flux_values(k, k.phi[ra], k.cp[ra], k.cm[ra], k.phi[rb], k.cp[rb], k.cm[rb], delta, Jp, Jm);
 }
 
 // flux_site_plus/minus of just_eq_smolu.f90:61-103 in gather form: every site adds the fluxes
@@ -587,6 +601,20 @@ int lbgpu_pnp_init(lbgpu_ctx *ctx, const lbgpu_pnp_params *p, double *anormf0)
         return rc;
     for (int q = 0; q < 3; ++q)
         if ((rc = alloc(&s->bak[q], N))) return rc;
+    const bool jacobi = p->solver != LBGPU_POISSON_SOR4;
+    if (jacobi) s->resident = plan_pnp_resident(N);
+    if (s->resident.blocks) {
+        double *d = nullptr;
+        if ((rc = alloc(&s->link, 18 * (size_t)ctx->p.lx)) ||
+            (rc = alloc(&s->rpartial, pnp_resident_partials(s->resident.blocks))) ||
+            (rc = alloc(&d, sizeof(GridSync) / sizeof(double))))
+            return rc;
+        s->gsync = reinterpret_cast<GridSync *>(d);
+        if ((rc = alloc(&d, (sizeof(PnpLoop) + 7) / sizeof(double)))) return rc;
+        s->loop = reinterpret_cast<PnpLoop *>(d);
+    } else if (jacobi) {
+        if ((rc = alloc(&s->rhs, N))) return rc;
+    }
     // partials: 4 per block, twice (two reductions read back together); results: 4, twice
     if ((rc = alloc(&s->partial, 8 * (size_t)MP_MAX_BLOCKS)) || (rc = alloc(&s->result, 8))) return rc;
     LBG_CK(ctx, cudaMalloc((void **)&s->ctl, sizeof(PnpCtl)));
@@ -672,6 +700,64 @@ int lbgpu_pnp_get(lbgpu_ctx *ctx, double *c_plus, double *c_minus, double *phi, 
 
 static int sor_solve(lbgpu_ctx *ctx, int *iters, bool defer_anorm);
 
+// omega, the stopping value and the sweep cap of a solve from the current anormf0
+static void solve_params(const PnpState *s, PnpArgs &a, PnpCtl &c)
+{
+    std::memset(&c, 0, sizeof(c));
+    c.parity = s->par;
+    const bool ref = s->p.solver == LBGPU_POISSON_REFERENCE;
+    a.omega = ref ? 1.4 : s->p.omega;                              // sor.f90:19
+    c.limit = (ref ? (double)1.0e-5f : s->p.tol) * s->anormf0;     // sor.f90:18,78
+    c.max_iter = s->p.max_iter > 0 ? s->p.max_iter : 500000;
+    a.one_minus_omega = 1.0 - a.omega;
+}
+
+static int solve_not_converged(lbgpu_ctx *ctx)
+{
+    return ctx_fail(ctx, LBGPU_ERR_STEP_CAP, "maximum iterations 500 000 reached without convergence in sor");
+}
+
+// The resident loop (pnp_resident.cu) from the current state: one solve (max_outer = 0), or up to
+// max_outer outer iterations (each launch some tens of milliseconds at most).
+static int run_resident(lbgpu_ctx *ctx, const PnpArgs &a, const PnpCtl &c, int max_outer, PnpLoop &h)
+{
+    PnpState *s = ctx->pnp;
+    cudaStream_t st = ctx->stream;
+    std::memset(&h, 0, sizeof(h));
+    h.limit = c.limit;
+    LBG_CK(ctx, cudaMemcpyAsync(s->loop, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+    PnpResidentArgs r;
+    std::memset(&r, 0, sizeof(r));
+    r.a = a;
+    r.sync = s->gsync;
+    r.loop = s->loop;
+    r.phi = s->phi[s->par];
+    r.cp = s->cp;
+    r.cm = s->cm;
+    r.t0 = s->fp;
+    r.t1 = s->fm;
+    for (int q = 0; q < 3; ++q) r.bak[q] = s->bak[q];
+    r.link = s->link;
+    r.partial = s->rpartial;
+    r.limit_factor = s->p.solver == LBGPU_POISSON_REFERENCE ? (double)1.0e-5f : s->p.tol;
+    r.max_iter = c.max_iter;
+    r.max_outer = max_outer;
+    r.max_sweeps = 4096;
+    r.outers_per_launch = 1024;
+    r.sigma = s->p.sigma;
+    r.rho_ch = s->rho_ch;
+    r.count_fluid = (double)ctx->counts[0];
+    do {
+        r.outer0 = h.outer;
+        LBG_CK(ctx, launch_pnp_resident(s->resident, r, st));
+        LBG_CK(ctx, cudaMemcpyAsync(&h, s->loop, sizeof(h), cudaMemcpyDeviceToHost, st));
+        LBG_CK(ctx, cudaStreamSynchronize(st));
+    } while (!h.done && !(h.status & LBGPU_ERR_TIMEOUT));
+    if (h.status & LBGPU_ERR_TIMEOUT)
+        return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, "Poisson-Nernst-Planck: a block did not reach the grid's barrier within its wait limit");
+    return LBGPU_OK;
+}
+
 int lbgpu_sor(lbgpu_ctx *ctx, int *iters)
 {
     TraceRange trace_("lbgpu_sor");
@@ -705,18 +791,15 @@ static int sor_solve(lbgpu_ctx *ctx, int *iters, bool defer_anorm)
     a.gen = multi && !four;
     a.ncolor = four ? 4 : std::max(a.kx, a.kz) * std::max(a.ky, a.kz);
     PnpCtl c;
-    std::memset(&c, 0, sizeof(c));
-    c.parity = s->par;
-    if (s->p.solver == LBGPU_POISSON_REFERENCE) {
-        a.omega = 1.4;                                  // sor.f90:19
-        c.limit = (double)1.0e-5f * s->anormf0;         // sor.f90:18,78
-        c.max_iter = s->p.max_iter > 0 ? s->p.max_iter : 500000;
-    } else {
-        a.omega = s->p.omega;
-        c.limit = s->p.tol * s->anormf0;
-        c.max_iter = s->p.max_iter > 0 ? s->p.max_iter : 500000;
+    solve_params(s, a, c);
+    if (s->resident.blocks) {
+        PnpLoop h;
+        if ((rc = run_resident(ctx, a, c, 0, h))) return rc;
+        if (iters) *iters = h.total;
+        if ((rc = anorm_begin(ctx))) return rc;                   // sor.f90:90
+        if (!defer_anorm && (rc = anorm_end(ctx))) return rc;
+        return h.converged ? LBGPU_OK : solve_not_converged(ctx);
     }
-    a.one_minus_omega = 1.0 - a.omega;
     k_ctl_set<<<1, 1, 0, st>>>(s->ctl, c);
     LBG_CK(ctx, cudaGetLastError());
     const unsigned grid = grid_for(ctx->N);
@@ -737,7 +820,8 @@ static int sor_solve(lbgpu_ctx *ctx, int *iters, bool defer_anorm)
                     else k_sor_color_gen<<<grid, PB, 0, st>>>(b, s->phi[s->par]);
                 }
             } else {
-                k_sor_jacobi<<<grid, PB, 0, st>>>(a, s->phi[0], s->phi[1]);
+                if (k == 0) k_sor_jacobi<true><<<grid, PB, 0, st>>>(a, s->phi[0], s->phi[1], s->fp, s->fm, s->rhs);
+                else k_sor_jacobi<false><<<grid, PB, 0, st>>>(a, s->phi[0], s->phi[1], s->fp, s->fm, s->rhs);
             }
         }
         cudaError_t ce = cudaStreamEndCapture(st, &g);
@@ -775,9 +859,7 @@ static int sor_solve(lbgpu_ctx *ctx, int *iters, bool defer_anorm)
     if (iters) *iters = s->p.solver == LBGPU_POISSON_SOR4 ? c.iter : c.iter - 1;  // sor.f90:87
     if ((rc = anorm_begin(ctx))) return rc;                       // sor.f90:90
     if (!defer_anorm && (rc = anorm_end(ctx))) return rc;
-    if (!c.converged)
-        return ctx_fail(ctx, LBGPU_ERR_STEP_CAP, "maximum iterations 500 000 reached without convergence in sor");
-    return LBGPU_OK;
+    return c.converged ? LBGPU_OK : solve_not_converged(ctx);
 }
 
 int lbgpu_just_eq_smolu(lbgpu_ctx *ctx, int *iters)
@@ -871,6 +953,26 @@ int lbgpu_poisson_nernst_planck(lbgpu_ctx *ctx, int max_outer, int *outer, int *
         lbgpu_ctx *ctx;
         ~AnormDone() { anorm_end(ctx); }
     } anorm_done_{ctx};
+    if (s->resident.blocks) {
+        if ((rc = anorm_end(ctx))) return rc;
+        PnpArgs a;
+        PnpCtl c;
+        PnpLoop h;
+        fill_pnp_args(ctx, a);
+        solve_params(s, a, c);
+        if ((rc = run_resident(ctx, a, c, max_outer > 0 ? max_outer : 0x7fffffff, h))) return rc;
+        if ((rc = anorm_begin(ctx))) return rc;   // anormf0 of the last solve in the reference's order
+        if (h.status & LBGPU_ERR_STEP_CAP) return solve_not_converged(ctx);
+        if (h.status & LBGPU_ERR_FLUX_SUM)
+            return ctx_fail(ctx, LBGPU_ERR_FLUX_SUM, "the sum of all flux does not add up. problem in just_eq_smolu.f90");
+        if (outer) *outer = h.outer;
+        if (sor_iters_total) *sor_iters_total = h.total;
+        if (!h.equilibrium)
+            return ctx_fail(ctx, LBGPU_ERR_STEP_CAP, "Equilibrium distribution of salts not found");
+        if ((rc = anorm_end(ctx))) return rc;
+        double sc, fc;
+        return lbgpu_charge_test(ctx, &sc, &fc);   // poisson_nernst_planck.f90:50
+    }
     while (!converged) {
         if (max_outer > 0 && n >= max_outer) {
             if (outer) *outer = n;

@@ -22,11 +22,24 @@ struct PnpCtl {
     double anorm, limit;  // stop when anorm <= limit
 };
 
+// The resident loop of a small box (pnp_resident.cu): blocks 0 when the box is not run so.
+struct PnpResidentPlan {
+    unsigned blocks, threads;
+};
+struct PnpResidentArgs;
+struct PnpLoop;
+struct GridSync;
+PnpResidentPlan plan_pnp_resident(long long N);
+size_t pnp_resident_partials(unsigned blocks);   // doubles of PnpResidentArgs::partial
+cudaError_t launch_pnp_resident(const PnpResidentPlan &plan, PnpResidentArgs &r, cudaStream_t s);
+
 struct PnpState {
     lbgpu_pnp_params p{};
     double *phi[2] = {nullptr, nullptr};
     double *cp = nullptr, *cm = nullptr;
-    double *fp = nullptr, *fm = nullptr;    // flux_site_plus / flux_site_minus
+    // flux_site_plus / flux_site_minus; during a Jacobi solve, w_axis phi by sweep parity
+    double *fp = nullptr, *fm = nullptr;
+    double *rhs = nullptr;                  // Jacobi solve: 4 pi bjl kBT/2 (c+ - c-)
     double *bak[3] = {nullptr, nullptr, nullptr};  // phi_old, c_plus_old, c_minus_old
     double *partial = nullptr;              // 4 per block
     double *result = nullptr;               // 4 reduced sums
@@ -35,7 +48,11 @@ struct PnpState {
     double anormf0 = 0.0, rho_ch = 0.0;
     bool charged = false;
     std::vector<void *> allocs;
-    // CUDA graphs of 8 and of 64 sweeps, captured at the first solve and replayed by every later
+    PnpResidentPlan resident{};             // with its own buffers:
+    GridSync *gsync = nullptr;
+    PnpLoop *loop = nullptr;
+    double *link = nullptr, *rpartial = nullptr;
+    // CUDA graphs of 1 and of 64 sweeps, captured at the first solve and replayed by every later
     // one (their arguments are fixed until the state is released)
     cudaGraphExec_t sor_exec[2] = {nullptr, nullptr};
     // electrokinetic operators (ek.cu), allocated at their first use: the total potential
