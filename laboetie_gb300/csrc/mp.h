@@ -122,6 +122,32 @@ cudaError_t launch_mp_step_f32(const MpArgs32 &a, unsigned grid, const CUtensorM
 bool mp32_tensor_map(CUtensorMap *tm, const float4 *field, int lx, int ly, int lz);
 // blocks of the slab step resident on the current device at once (SMs x blocks per SM)
 unsigned mp32_slab_resident();
+
+// Many steps of a small box in one launch (mp_resident.cu); blocks 0 when the box is not run so.
+struct MpResidentPlan {
+    unsigned blocks, threads;
+    bool cluster;
+};
+struct MpResident {
+    MpResidentPlan plan;
+    unsigned Nf;
+    const uint32_t *fidx;    // lattice indices of the fluid nodes
+    const uint32_t *place;   // lattice index -> fluid node (cluster only)
+    void *sync;              // mp_resident_sync_bytes
+    void *scratch;           // grid only: one more P buffer (N float4, or 3 N doubles)
+    double *part;            // max_steps * blocks * threads / 32 * 3 doubles
+    unsigned *failed;        // 1 after a launch whose wait ran out
+    int max_steps;           // most steps per launch
+};
+MpResidentPlan plan_mp_resident(unsigned Nf, bool f64);
+size_t mp_resident_sync_bytes();
+cudaError_t launch_mp_place(const uint32_t *fidx, unsigned nf, uint32_t *place, cudaStream_t s);
+cudaError_t launch_mp_fidx(const uint32_t *cpos, unsigned nf, int lx, int ly, int xbits, int ybits, uint32_t *fidx,
+                           cudaStream_t s);
+// nsteps steps from P[par] (left as it is) into P[par ^ 1], and VACF of each step (3 doubles) in
+// vacf; a64 or a32 is null
+cudaError_t launch_mp_resident(const MpResident &m, const MpArgs64 *a64, const MpArgs32 *a32, int par, int nsteps,
+                               double *vacf, cudaStream_t s);
 cudaError_t launch_mp_init_f32(const MpArgs32 &a, float bw, unsigned grid, cudaStream_t s);
 
 }  // namespace lbg

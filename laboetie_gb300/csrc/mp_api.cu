@@ -28,6 +28,8 @@ struct MpState {
     MpArgs64 a64{};
     MpArgs32 a32{};
     std::vector<void *> allocs;
+    MpResident res{};             // many steps per launch (mp_resident.cu) where the box is small
+    double *res_vacf = nullptr;   // VACF of one launch's steps
     unsigned nblocks = 0;
     int it_next = 1;
     int converged = 0;
@@ -56,6 +58,44 @@ int alloc_zero(lbgpu_ctx *ctx, MpState *s, T **p, size_t count)
 }
 
 constexpr double EPS = 2.220446049250313e-16;  // epsilon(1._dp)
+
+// The resident form of a neutral tracer (mp_resident.cu): its tables and workspace, in one allocation.
+int resident_init(lbgpu_ctx *ctx, MpState *s)
+{
+    const bool f64 = s->prec == LBGPU_FP64;
+    if (!f64 && !ctx->d_cpos) return LBGPU_OK;   // two-buffer FP32 layout: no list of fluid nodes
+    const long long N = ctx->N;
+    const unsigned nf = (unsigned)ctx->counts[0];
+    // LBGPU_MP_SLAB / LBGPU_MP_TMA choose among the launch-per-step kernels
+    if (std::getenv("LBGPU_MP_SLAB") || std::getenv("LBGPU_MP_TMA")) return LBGPU_OK;
+    MpResident m{};
+    m.plan = plan_mp_resident(nf, f64);
+    if (!m.plan.blocks) return LBGPU_OK;
+    m.Nf = nf;
+    const size_t step = (size_t)m.plan.blocks * (m.plan.threads / 32) * 3 * sizeof(double);
+    m.max_steps = (int)std::min<size_t>(1024, std::max<size_t>(16, (16u << 20) / step));
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t b_part = up(step * m.max_steps), b_vacf = up(sizeof(double) * 3 * m.max_steps),
+                 b_sync = up(mp_resident_sync_bytes()), b_idx = up(sizeof(uint32_t) * (f64 ? 1 : nf)),
+                 b_place = up(sizeof(uint32_t) * (m.plan.cluster ? N : 1)),
+                 b_scratch = up(m.plan.cluster ? 1 : (f64 ? 3 * sizeof(double) : sizeof(float4)) * (size_t)N);
+    char *mem = nullptr;
+    int rc = alloc_zero(ctx, s, &mem, b_part + b_vacf + b_sync + 256 + b_idx + b_place + b_scratch);
+    if (rc) return rc;
+    m.part = reinterpret_cast<double *>(mem);
+    s->res_vacf = reinterpret_cast<double *>(mem += b_part);
+    m.sync = mem += b_vacf;
+    m.failed = reinterpret_cast<unsigned *>(mem += b_sync);
+    uint32_t *idx = reinterpret_cast<uint32_t *>(mem += 256);
+    uint32_t *place = reinterpret_cast<uint32_t *>(mem += b_idx);
+    m.scratch = mem + b_place;
+    if (!f64) LBG_CK(ctx, launch_mp_fidx(ctx->d_cpos, nf, ctx->p.lx, ctx->p.ly, ctx->xbits, ctx->ybits, idx, ctx->stream));
+    m.fidx = f64 ? ctx->d_fidx : idx;
+    if (m.plan.cluster) LBG_CK(ctx, launch_mp_place(m.fidx, nf, place, ctx->stream));
+    m.place = place;
+    s->res = m;
+    return LBGPU_OK;
+}
 
 // refresh ctx->d_rho / d_j with the moments of the current flow state
 int flow_moments_on_device(lbgpu_ctx *ctx)
@@ -275,6 +315,8 @@ int mp_init_impl(lbgpu_ctx *ctx, const lbgpu_tracer *tr, const double *density, 
                     mp32_tensor_map(&s->tm[1], b.P[0], a.lx, a.ly, a.lz) &&
                     mp32_tensor_map(&s->tm[2], b.P[1], a.lx, a.ly, a.lz);
     }
+    if (!charged)
+        if ((rc = resident_init(ctx, s))) return rc;
     LBG_CK(ctx, launch_mp_reduce_init(a.partial, s->nblocks, a.ctl, st));
     if (tmp) LBG_CK(ctx, cudaFreeAsync(tmp, st));
     // the ρ/j pointers of the init are not used by the steps
@@ -293,6 +335,60 @@ int mp_init_impl(lbgpu_ctx *ctx, const lbgpu_tracer *tr, const double *density, 
 }  // namespace lbg
 
 extern "C" {
+
+// The steps of mp_run as resident launches: `c` is the control block as the call starts (its
+// thresholds set).  A launch that meets the convergence test before its last step is repeated up to
+// that step from the P it started from.
+static int mp_run_resident(lbgpu_ctx *ctx, MpCtl &c, int nsteps, double *vacf_out, bool timing, float *ms)
+{
+    MpState *s = ctx->mp;
+    cudaStream_t st = ctx->stream;
+    const MpArgs64 *a64 = s->prec == LBGPU_FP64 ? &s->a64 : nullptr;
+    const MpArgs32 *a32 = a64 ? nullptr : &s->a32;
+    std::vector<double> rows((size_t)3 * std::min(nsteps, s->res.max_steps));
+    unsigned failed = 0;
+    int done = 0;
+    if (timing) LBG_CK(ctx, cudaEventRecord(ctx->ev0, st));
+    while (done < nsteps && !c.converged) {
+        int n = std::min(nsteps - done, s->res.max_steps);
+        LBG_CK(ctx, launch_mp_resident(s->res, a64, a32, c.parity, n, s->res_vacf, st));
+        LBG_CK(ctx, cudaMemcpyAsync(rows.data(), s->res_vacf, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st));
+        LBG_CK(ctx, cudaMemcpyAsync(&failed, s->res.failed, sizeof(failed), cudaMemcpyDeviceToHost, st));
+        LBG_CK(ctx, cudaStreamSynchronize(st));
+        if (failed) {
+            c.status |= LBGPU_ERR_TIMEOUT;
+            return LBGPU_OK;
+        }
+        for (int k = 0; k < n && !c.converged; ++k) {
+            bool conv = c.it + k > 2;
+            for (int d = 0; d < 3; ++d) {
+                const double v = std::fabs(rows[3 * k + d]);
+                if (!(v < c.thr1) || !(v < c.thr2)) conv = false;
+            }
+            if (!conv) continue;
+            c.converged = 1;
+            if (k + 1 < n) {
+                n = k + 1;
+                LBG_CK(ctx, launch_mp_resident(s->res, a64, a32, c.parity, n, s->res_vacf, st));
+            }
+        }
+        if (vacf_out) std::memcpy(vacf_out + 3 * (size_t)done, rows.data(), sizeof(double) * 3 * n);
+        for (int d = 0; d < 3; ++d) c.vacf[d] = rows[3 * (n - 1) + d];
+        c.parity ^= 1;
+        c.it += n;
+        c.last_it = c.it - 1;
+        done += n;
+    }
+    c.done = 1;
+    if (timing) {
+        LBG_CK(ctx, cudaEventRecord(ctx->ev1, st));
+        LBG_CK(ctx, cudaEventSynchronize(ctx->ev1));
+        LBG_CK(ctx, cudaEventElapsedTime(ms, ctx->ev0, ctx->ev1));
+    }
+    LBG_CK(ctx, cudaMemcpyAsync(s->a64.ctl, &c, sizeof(c), cudaMemcpyHostToDevice, st));
+    LBG_CK(ctx, cudaStreamSynchronize(st));
+    return LBGPU_OK;
+}
 
 static int mp_run(lbgpu_ctx *ctx, int nsteps, double *vacf_out, int *steps_done, int *is_converged,
                   bool timing, float *ms)
@@ -322,6 +418,17 @@ static int mp_run(lbgpu_ctx *ctx, int nsteps, double *vacf_out, int *steps_done,
         const volatile double den = 2.0 * ctx->p.lx * ctx->p.ly * ctx->p.lz / s->tr.Db;
         c.thr1 = 1.0 / den;
         c.thr2 = (double)1.e-12f;
+    }
+    if (s->res.plan.blocks) {
+        if (int rc = mp_run_resident(ctx, c, nsteps, vacf_out, timing, ms)) return rc;
+        if (c.status & LBGPU_ERR_TIMEOUT)
+            return ctx_fail(ctx, LBGPU_ERR_TIMEOUT,
+                            "moment propagation: a block did not reach the grid's barrier within its wait limit");
+        s->it_next = c.last_it + 1;
+        s->converged = c.converged;
+        if (steps_done) *steps_done = c.last_it - c.it_base + 1;
+        if (is_converged) *is_converged = c.converged;
+        return LBGPU_OK;
     }
     LBG_CK(ctx, cudaMemcpyAsync(s->a64.ctl, &c, sizeof(c), cudaMemcpyHostToDevice, st));
     double *hist = nullptr;
