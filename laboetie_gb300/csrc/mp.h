@@ -111,7 +111,7 @@ inline unsigned mp32_slab_grid(int lx, int ly, int lz, unsigned resident, int *z
 }
 
 cudaError_t launch_mp_init_f64(const MpArgs64 &a, unsigned grid, cudaStream_t s);
-cudaError_t launch_mp_step_f64(const MpArgs64 &a, unsigned grid, cudaStream_t s);
+cudaError_t launch_mp_step_f64(const MpArgs64 &a, cudaStream_t s);
 cudaError_t launch_mp_reduce_init(double *partial, unsigned nblocks, MpCtl *ctl, cudaStream_t s);
 cudaError_t launch_mp_v32(const MpArgs64 &a64, float4 *V, cudaStream_t s);
 // tm: the tensor maps of V, P[0], P[1] for the slab step's bulk tensor copies, or null (the slab

@@ -247,7 +247,7 @@ int mp_init_impl(lbgpu_ctx *ctx, const lbgpu_tracer *tr, const double *density, 
     int zc = 0;
     const unsigned resident = s->prec == LBGPU_FP64 ? 0u : mp32_slab_resident();
     const unsigned slab = s->prec == LBGPU_FP64 ? 0u : mp32_slab_grid(a.lx, a.ly, a.lz, resident, &zc);
-    if ((rc = alloc_zero(ctx, s, &a.partial, 3 * (size_t)std::max(s->nblocks, slab)))) return rc;
+    if ((rc = alloc_zero(ctx, s, &a.partial, 3 * (size_t)std::max(std::max(s->nblocks, slab), 2 * MP_MAX_BLOCKS)))) return rc;
     if ((rc = alloc_zero(ctx, s, &a.ctl, 1))) return rc;
 
     if (s->prec == LBGPU_FP64) {
@@ -440,13 +440,9 @@ static int mp_run(lbgpu_ctx *ctx, int nsteps, double *vacf_out, int *steps_done,
     cudaGraphExec_t exec;
     LBG_CK(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < G; ++k) {
-        // the FP64 step walks the fluid-node list: one thread per fluid node
-        const unsigned grid = std::min(s->prec == LBGPU_FP64 && s->a64.fidx
-                                           ? (unsigned)((s->a64.Nf + MP_BLOCK - 1) / MP_BLOCK)
-                                           : s->nblocks,
-                                       MP_MAX_BLOCKS);
-        cudaError_t e = s->prec == LBGPU_FP64 ? launch_mp_step_f64(s->a64, grid, st)
-                                              : launch_mp_step_f32(s->a32, grid, s->tma_ok ? s->tm : nullptr, st);
+        cudaError_t e = s->prec == LBGPU_FP64
+                            ? launch_mp_step_f64(s->a64, st)
+                            : launch_mp_step_f32(s->a32, std::min(s->nblocks, MP_MAX_BLOCKS), s->tma_ok ? s->tm : nullptr, st);
         if (e != cudaSuccess) {
             cudaStreamEndCapture(st, &g);
             return ctx_cuda(ctx, e, "capture moment propagation");

@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(MP_BLOCK) k_mp32(const MpArgs32 a, float bw)
             for (int d = 0; d < 3; ++d) a.partial[3 * blockIdx.x + d] = v[d];
         if (bad) atomicOr(&a.ctl->status, bad);
     } else {
-        grid_sum3(v, a.partial, &a.ctl->blocks_done,
+        grid_sum3<false>(v, a.partial, &a.ctl->blocks_done,
                   [&](const double (&tot)[3]) { mp_control(a.ctl, a.hist, tot); });
     }
 }
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(MP_BLOCK, 4)
     mp_slab_planes(a, par, (tile % tiles_x) * MPS_TX, (tile / tiles_x) * MPS_TY, z0, min(z0 + zc, a.lz), sm4, vt,
                    use_tma ? &tmV : nullptr, use_tma ? (par ? &tmP1 : &tmP0) : nullptr, &a.ctl->status);
     double v[3] = {(double)vt[0], (double)vt[1], (double)vt[2]};
-    grid_sum3(v, a.partial, &a.ctl->blocks_done,
+    grid_sum3<false>(v, a.partial, &a.ctl->blocks_done,
               [&](const double (&tot)[3]) { mp_control(a.ctl, a.hist, tot); });
 }
 

@@ -8,6 +8,8 @@
 // reference's sweep does (module_moment_propagation.f90:207-253): the propagated quantities are
 // bit-identical to the reference; only the VACF node sum runs in a different (fixed) order.
 // Storing the table instead of recomputing it matters on GB300, whose FP64 rate is low.
+#include <algorithm>
+
 #include "common.cuh"
 #include "lbgpu.h"
 #include "mp.h"
@@ -168,14 +170,18 @@ __global__ void __launch_bounds__(MP_BLOCK) k_mp_init(const MpArgs64 a)
 // module_moment_propagation.f90:164-289, one step.  Grid-stride over the nodes.  The gathers
 // are branch-free: a link to a solid neighbour has coefficient 0 and the neighbour's P is 0, so
 // it adds an exact zero where the reference skips it (only the sign of an exact zero can differ).
+// Bound by the FP64 pipe: 143 FP64 instructions per warp and step at 60 % porosity with adsorption
+// (108 of them the links), 19 SM cycles each.  97 % of that at 675 k fluid nodes (192 us per step);
+// 201 k fluid nodes 80.4 us per step with a shuffle tree per warp, 256-thread blocks and separate
+// branches for adsorbing nodes, 66.6 now (64 registers: 51 or 42 keep fewer gathers in flight, 68.1
+// and 71.4 us).
 // FUSED (LBGPU_FP64_FUSED): each link's gather and the remaining-fraction terms as fused
 // multiply-adds, in the same order (within 1e-12 relative of the separately rounded form).
 template <bool FUSED>
-__global__ void __launch_bounds__(MP_BLOCK) k_mp_step(const MpArgs64 a)
+__global__ void __launch_bounds__(MP_BLOCK, 4) k_mp_step(const MpArgs64 a)
 {
-    const volatile MpCtl *vc = a.ctl;
-    if (vc->done) return;
-    const int par = vc->parity;
+    if (a.ctl->done) return;   // written by the last block only, after every block has read it
+    const int par = a.ctl->parity;
     const long long N = a.N;
     const double *__restrict__ Px = a.P[par][0];
     const double *__restrict__ Py = a.P[par][1];
@@ -183,8 +189,8 @@ __global__ void __launch_bounds__(MP_BLOCK) k_mp_step(const MpArgs64 a)
     double v[3] = {0.0, 0.0, 0.0};
     // the fluid nodes through their list (every lane of a warp does work), else every lattice node
     const long long n_it = a.fidx ? a.Nf : N;
-    for (long long i = (long long)blockIdx.x * MP_BLOCK + threadIdx.x; i < n_it;
-         i += (long long)gridDim.x * MP_BLOCK) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_it;
+         i += (long long)gridDim.x * blockDim.x) {
         const long long r = a.fidx ? (long long)a.fidx[i] : i;
         const uint32_t m = a.mask[r];
         if (!(m & FLUID_BIT)) continue;
@@ -211,20 +217,23 @@ __global__ void __launch_bounds__(MP_BLOCK) k_mp_step(const MpArgs64 a)
         v[1] = v[1] + p1 * a.us[1][r];
         v[2] = v[2] + p2 * a.us[2][r];
         const double frac = a.frac[r];
-        if (FUSED && (!a.ads || !(m & INTERFACIAL_BIT))) {
+        const bool inter = a.ads && (m & INTERFACIAL_BIT);
+        if (FUSED && !inter) {
             n0 = __fma_rn(frac, p0, n0);
             n1 = __fma_rn(frac, p1, n1);
             n2 = __fma_rn(frac, p2, n2);
-        } else if (!a.ads || !(m & INTERFACIAL_BIT)) {
-            n0 = n0 + frac * p0;
-            n1 = n1 + frac * p1;
-            n2 = n2 + frac * p2;
         } else {
-            const double f2 = frac - a.ka;
+            // one sequence for the lanes of a warp with and without adsorption (frac - 0 is frac)
+            const double f2 = inter ? frac - a.ka : frac;
+            n0 = n0 + f2 * p0;
+            n1 = n1 + f2 * p1;
+            n2 = n2 + f2 * p2;
+        }
+        if (inter) {
             const double q0 = a.A[par][0][r], q1 = a.A[par][1][r], q2 = a.A[par][2][r];
-            n0 = n0 + f2 * p0 + q0 * a.kd;
-            n1 = n1 + f2 * p1 + q1 * a.kd;
-            n2 = n2 + f2 * p2 + q2 * a.kd;
+            n0 = n0 + q0 * a.kd;
+            n1 = n1 + q1 * a.kd;
+            n2 = n2 + q2 * a.kd;
             a.A[par ^ 1][0][r] = q0 * a.one_minus_kd + p0 * a.ka;
             a.A[par ^ 1][1][r] = q1 * a.one_minus_kd + p1 * a.ka;
             a.A[par ^ 1][2][r] = q2 * a.one_minus_kd + p2 * a.ka;
@@ -233,7 +242,7 @@ __global__ void __launch_bounds__(MP_BLOCK) k_mp_step(const MpArgs64 a)
         a.P[par ^ 1][1][r] = n1;
         a.P[par ^ 1][2][r] = n2;
     }
-    grid_sum3(v, a.partial, &a.ctl->blocks_done,
+    grid_sum3<true>(v, a.partial, &a.ctl->blocks_done,
               [&](const double (&tot)[3]) { mp_control(a.ctl, a.hist, tot); });
 }
 
@@ -259,10 +268,16 @@ cudaError_t launch_mp_init_f64(const MpArgs64 &a, unsigned grid, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t launch_mp_step_f64(const MpArgs64 &a, unsigned grid, cudaStream_t s)
+cudaError_t launch_mp_step_f64(const MpArgs64 &a, cudaStream_t s)
 {
-    if (a.fused) k_mp_step<true><<<grid, MP_BLOCK, 0, s>>>(a);
-    else k_mp_step<false><<<grid, MP_BLOCK, 0, s>>>(a);
+    // Four-warp blocks, so that a few blocks per SM come out even (201 k fluid nodes: 10.3 blocks of
+    // 128 threads per SM run as 11, 5.2 blocks of 256 as 6), until eight-warp blocks fill the SMs
+    // many times over; then a grid-stride over as many as the partial sums hold.
+    const long long n = a.fidx ? a.Nf : a.N;
+    const unsigned block = n <= 128ll * 2 * MP_MAX_BLOCKS ? 128u : (unsigned)MP_BLOCK;
+    const unsigned grid = (unsigned)std::min<long long>((n + block - 1) / block, block == 128u ? 2 * MP_MAX_BLOCKS : MP_MAX_BLOCKS);
+    if (a.fused) k_mp_step<true><<<grid, block, 0, s>>>(a);
+    else k_mp_step<false><<<grid, block, 0, s>>>(a);
     return cudaGetLastError();
 }
 

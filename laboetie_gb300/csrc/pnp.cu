@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(PB) k_sor_color(const PnpArgs a, double *phi)
         const long long r = x + (long long)a.lx * (y + (long long)a.ly * z);
         t[0] = t[0] + sor_node(a, phi, x, y, z, r);
     }
-    grid_sum3(t, a.partial, &a.ctl->blocks_done, [&](const double (&tot)[3]) { sor_colour_done(a, tot); });
+    grid_sum3<true>(t, a.partial, &a.ctl->blocks_done, [&](const double (&tot)[3]) { sor_colour_done(a, tot); });
 }
 
 // One colour of the multicolour SOR of any box (some side odd or one wide).  With gx, gy, gz the
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(PB) k_sor_color_gen(const PnpArgs a, double *p
         if (colour != a.color) continue;
         t[0] = t[0] + sor_node(a, phi, x, y, z, r);
     }
-    grid_sum3(t, a.partial, &a.ctl->blocks_done, [&](const double (&tot)[3]) { sor_colour_done(a, tot); });
+    grid_sum3<true>(t, a.partial, &a.ctl->blocks_done, [&](const double (&tot)[3]) { sor_colour_done(a, tot); });
 }
 
 // Sum of the reference's stopping measure |phi* - phi| over every node at the current phi (no

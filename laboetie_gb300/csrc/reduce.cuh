@@ -53,15 +53,44 @@ __device__ __forceinline__ void block_sum3_fixed(double (&v)[3])
     }
 }
 
+// The same for any block of up to MP_BLOCK threads (a multiple of 32), for kernels bound by the FP64
+// pipe: one warp per value adds the block's values through shared memory, 12 FP64 instructions per
+// value for 256 threads against 5 in each of 8 warps and 5 more (an FP64 instruction occupies its
+// quarter of the SM for 64 cycles).  It takes 6 KB of shared memory, which would cost the FP32 slab
+// step a resident block (77 -> 83 us per step at 160^3).
+__device__ __forceinline__ void block_sum3_shared(double (&v)[3])
+{
+    __shared__ double sh[3][MP_BLOCK];
+    __shared__ double tot[3];
+    const unsigned lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    __syncthreads();  // sh may still be read by a previous call
+#pragma unroll
+    for (int d = 0; d < 3; ++d) sh[d][threadIdx.x] = v[d];
+    __syncthreads();
+    for (unsigned d = wid; d < 3; d += nw) {
+        double s = sh[d][lane];
+        for (unsigned k = lane + 32; k < blockDim.x; k += 32) s = s + sh[d][k];
+        s = warp_sum_fixed(s);
+        if (lane == 0) tot[d] = s;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) v[d] = tot[d];
+    }
+}
+
 // Every block stores its 3 partial sums; the last block to finish adds the partials in block
 // order and runs `finish(total)` in thread 0.
-template <typename Fin>
+// SHARED: the blocks' sums as block_sum3_shared's.
+template <bool SHARED, typename Fin>
 __device__ __forceinline__ void grid_sum3(const double (&v)[3], double *partial, unsigned *counter,
                                           Fin &&finish)
 {
     __shared__ bool last;
     double b[3] = {v[0], v[1], v[2]};
-    block_sum3_fixed(b);
+    if constexpr (SHARED) block_sum3_shared(b);
+    else block_sum3_fixed(b);
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) partial[3 * blockIdx.x + d] = b[d];
@@ -72,12 +101,13 @@ __device__ __forceinline__ void grid_sum3(const double (&v)[3], double *partial,
     if (!last) return;
     __threadfence();
     double t[3] = {0.0, 0.0, 0.0};
-    for (unsigned i = threadIdx.x; i < gridDim.x; i += MP_BLOCK) {
-        const volatile double *p = partial + 3 * i;
+#pragma unroll 4
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) t[d] += p[d];
+        for (int d = 0; d < 3; ++d) t[d] += __ldcg(partial + 3 * i + d);
     }
-    block_sum3_fixed(t);
+    if constexpr (SHARED) block_sum3_shared(t);
+    else block_sum3_fixed(t);
     if (threadIdx.x == 0) {
         *counter = 0;
         finish(t);
