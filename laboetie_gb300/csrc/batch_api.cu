@@ -23,6 +23,7 @@
 #include "batch.h"
 #include "compact.cuh"
 #include "ctx.h"
+#include "fields.h"
 #include "flow.h"
 #include "lbgpu.h"
 #include "trace.h"
@@ -147,6 +148,9 @@ struct lbgpu_batch {
     BatchTicket *d_ticket = nullptr;
     bool aa_tuned = false;
     bool smem_tuned = false;
+    // workspace of the calls that hand fields back, grown to the largest box asked for
+    double *d_ws = nullptr;
+    size_t ws_bytes = 0;
     std::vector<int> desc_slot;   // descriptor index -> slot
     std::vector<GraphEntry> graphs;
 };
@@ -169,6 +173,18 @@ int grow(T **p, int &cap, int need, cudaStream_t s)
     if (*p) LBB_CK(cudaFreeAsync(*p, s));
     LBB_CK(cudaMallocAsync((void **)p, sizeof(T) * nc, s));
     cap = nc;
+    return LBGPU_OK;
+}
+
+int workspace(lbgpu_batch *b, size_t bytes)
+{
+    if (bytes <= b->ws_bytes) return LBGPU_OK;
+    LBB_CK(cudaStreamSynchronize(b->stream));
+    cudaFree(b->d_ws);
+    b->d_ws = nullptr;
+    b->ws_bytes = 0;
+    LBB_CK(cudaMalloc((void **)&b->d_ws, bytes));
+    b->ws_bytes = bytes;
     return LBGPU_OK;
 }
 
@@ -729,6 +745,7 @@ void lbgpu_batch_destroy(lbgpu_batch *b)
     cudaFree(b->d_du);
     cudaFree(b->d_counts);
     cudaFree(b->d_ticket);
+    cudaFree(b->d_ws);
     for (cudaEvent_t ev : {b->ev0, b->ev1, b->fork, b->join, b->join2, b->fork_mp, b->join_mp})
         if (ev) cudaEventDestroy(ev);
     if (b->side) cudaStreamDestroy(b->side);
@@ -969,15 +986,14 @@ int lbgpu_batch_moments(lbgpu_batch *b, int id, double *rho, double *jx, double 
     const BatchInst &d = b->slots[id].d;
     const int N = d.N;
     cudaStream_t s = b->stream;
-    double *tmp = nullptr;
-    LBB_CK(cudaMallocAsync((void **)&tmp, sizeof(double) * 4 * (size_t)N, s));
+    if ((rc = workspace(b, sizeof(double) * 4 * (size_t)N))) return rc;
+    double *tmp = b->d_ws;
     if (d.compact) LBB_CK(cudaMemsetAsync(tmp, 0, sizeof(double) * 4 * (size_t)N, s));   // solid nodes: zeros
     LBB_CK(launch_batch_moments(b->d_insts, desc, batch_units(d), tmp, tmp + N, tmp + 2 * (size_t)N,
                                 tmp + 3 * (size_t)N, s));
     double *out[4] = {rho, jx, jy, jz};
     for (int q = 0; q < 4; ++q)
         LBB_CK(cudaMemcpyAsync(out[q], tmp + q * (size_t)N, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
-    LBB_CK(cudaFreeAsync(tmp, s));
     LBB_CK(cudaStreamSynchronize(s));
     return LBGPU_OK;
 }
@@ -1032,22 +1048,17 @@ int lbgpu_batch_mp_fields(lbgpu_batch *b, int id, double *P, double *P_ads)
     const Slot &sl = b->slots[id];
     if (sl.d.phase != BATCH_MP) return bfail(LBGPU_ERR_INVALID, "lbgpu_batch_mp_fields: no tracer phase");
     const size_t N = (size_t)sl.d.N;
-    std::vector<float4> f(N);
     double *outs[2] = {P, P_ads};
     for (int q = 0; q < 2; ++q) {
         if (!outs[q]) continue;
-        const float4 *src = q == 0 ? sl.d.P[0] : sl.d.A[0];   // a call runs an even number of steps
-        if (!src) {
+        Field3 f{};
+        f.rec = q == 0 ? sl.d.P[0] : sl.d.A[0];   // a call runs an even number of steps
+        if (!f.rec) {
             std::memset(outs[q], 0, sizeof(double) * 3 * N);
             continue;
         }
-        LBB_CK(cudaMemcpyAsync(f.data(), src, sizeof(float4) * N, cudaMemcpyDeviceToHost, b->stream));
-        LBB_CK(cudaStreamSynchronize(b->stream));
-        for (size_t i = 0; i < N; ++i) {
-            outs[q][3 * i] = f[i].x;
-            outs[q][3 * i + 1] = f[i].y;
-            outs[q][3 * i + 2] = f[i].z;
-        }
+        if (int rc = workspace(b, sizeof(double) * 3 * field_chunk_nodes((long long)N))) return rc;
+        LBB_CK(field_to_host(f, (long long)N, b->d_ws, outs[q], b->stream));
     }
     return LBGPU_OK;
 }

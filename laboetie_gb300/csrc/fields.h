@@ -1,0 +1,22 @@
+// fields.h -- transfers of tracer fields (fields.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+namespace lbg {
+
+// A three-component field on the device: float4 records (rec), or three arrays of doubles (comp).
+struct Field3 {
+    float4 *rec;
+    double *comp[3];
+};
+
+// nodes converted at a time; `stage` below holds 3 doubles of each
+size_t field_chunk_nodes(long long N);
+// host[3 i + d] = component d of node i (and back), waiting for the stream
+cudaError_t field_to_host(const Field3 &f, long long N, double *stage, double *host, cudaStream_t s);
+cudaError_t field_from_host(const Field3 &f, long long N, double *stage, const double *host, cudaStream_t s);
+
+}  // namespace lbg

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "fields.h"
 #include "flow.h"
 #include "lbgpu.h"
 #include "trace.h"
@@ -30,6 +31,7 @@ struct MpState {
     std::vector<void *> allocs;
     MpResident res{};             // many steps per launch (mp_resident.cu) where the box is small
     double *res_vacf = nullptr;   // VACF of one launch's steps
+    double *stage = nullptr;      // staging of lbgpu_mp_get / _set, at most 96 MiB
     unsigned nblocks = 0;
     int it_next = 1;
     int converged = 0;
@@ -58,6 +60,24 @@ int alloc_zero(lbgpu_ctx *ctx, MpState *s, T **p, size_t count)
 }
 
 constexpr double EPS = 2.220446049250313e-16;  // epsilon(1._dp)
+
+int stage_init(lbgpu_ctx *ctx, MpState *s)
+{
+    if (s->stage) return LBGPU_OK;
+    LBG_CK(ctx, cudaMalloc((void **)&s->stage, sizeof(double) * 3 * field_chunk_nodes(ctx->N)));
+    s->allocs.push_back(s->stage);
+    return LBGPU_OK;
+}
+
+// P (q = 0) or the adsorbed part (q = 1) in the buffers of parity par
+Field3 field_of(const MpState *s, int par, int q)
+{
+    Field3 f{};
+    if (s->prec == LBGPU_FP64)
+        for (int d = 0; d < 3; ++d) f.comp[d] = q == 0 ? s->a64.P[par][d] : s->a64.A[par][d];
+    else f.rec = q == 0 ? s->a32.P[par] : s->a32.A[par];
+    return f;
+}
 
 // The resident form of a neutral tracer (mp_resident.cu): its tables and workspace, in one allocation.
 int resident_init(lbgpu_ctx *ctx, MpState *s)
@@ -523,26 +543,8 @@ int lbgpu_mp_get(lbgpu_ctx *ctx, double *P, double *P_ads)
             std::memset(outs[q], 0, sizeof(double) * 3 * N);
             continue;
         }
-        std::vector<double> comp((size_t)3 * N);
-        for (int d = 0; d < 3; ++d) {
-            if (s->prec == LBGPU_FP64) {
-                const double *src = q == 0 ? s->a64.P[par][d] : s->a64.A[par][d];
-                LBG_CK(ctx, cudaMemcpyAsync(comp.data() + d * N, src, sizeof(double) * N, cudaMemcpyDeviceToHost, st));
-            } else if (d == 0) {
-                std::vector<float4> f(N);
-                const float4 *src = q == 0 ? s->a32.P[par] : s->a32.A[par];
-                LBG_CK(ctx, cudaMemcpyAsync(f.data(), src, sizeof(float4) * N, cudaMemcpyDeviceToHost, st));
-                LBG_CK(ctx, cudaStreamSynchronize(st));
-                for (long long i = 0; i < N; ++i) {
-                    comp[i] = f[i].x;
-                    comp[N + i] = f[i].y;
-                    comp[2 * N + i] = f[i].z;
-                }
-            }
-        }
-        LBG_CK(ctx, cudaStreamSynchronize(st));
-        for (long long i = 0; i < N; ++i)
-            for (int d = 0; d < 3; ++d) outs[q][3 * i + d] = comp[d * N + i];
+        if (int rc = stage_init(ctx, s)) return rc;
+        LBG_CK(ctx, field_to_host(field_of(s, par, q), N, s->stage, outs[q], st));
     }
     return LBGPU_OK;
 }
@@ -563,23 +565,8 @@ int lbgpu_mp_set(lbgpu_ctx *ctx, const double *P, const double *P_ads, int it_ne
     const double *ins[2] = {P, s->ads ? P_ads : nullptr};
     for (int q = 0; q < 2; ++q) {
         if (!ins[q]) continue;
-        if (s->prec == LBGPU_FP64) {
-            std::vector<double> comp((size_t)3 * N);
-            for (long long i = 0; i < N; ++i)
-                for (int d = 0; d < 3; ++d) comp[d * N + i] = ins[q][3 * i + d];
-            for (int d = 0; d < 3; ++d) {
-                double *dst = q == 0 ? s->a64.P[par][d] : s->a64.A[par][d];
-                LBG_CK(ctx, cudaMemcpyAsync(dst, comp.data() + d * N, sizeof(double) * N, cudaMemcpyHostToDevice, st));
-            }
-            LBG_CK(ctx, cudaStreamSynchronize(st));   // comp goes out of scope
-        } else {
-            std::vector<float4> f(N);
-            for (long long i = 0; i < N; ++i)
-                f[i] = make_float4((float)ins[q][3 * i], (float)ins[q][3 * i + 1], (float)ins[q][3 * i + 2], 0.0f);
-            float4 *dst = q == 0 ? s->a32.P[par] : s->a32.A[par];
-            LBG_CK(ctx, cudaMemcpyAsync(dst, f.data(), sizeof(float4) * N, cudaMemcpyHostToDevice, st));
-            LBG_CK(ctx, cudaStreamSynchronize(st));
-        }
+        if (int rc = stage_init(ctx, s)) return rc;
+        LBG_CK(ctx, field_from_host(field_of(s, par, q), N, s->stage, ins[q], st));
     }
     s->it_next = it_next;
     s->converged = 0;

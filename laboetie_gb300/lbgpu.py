@@ -250,9 +250,10 @@ class Box:
                   "flow_set")
 
     def flow_get(self, populations=True):
-        n = np.zeros((19,) + self.shape) if populations else None
-        rho = np.zeros(self.shape)
-        j = [np.zeros(self.shape) for _ in range(3)]
+        # np.empty: the call writes every node (a zeroed array would be written twice)
+        n = np.empty((19,) + self.shape) if populations else None
+        rho = np.empty(self.shape)
+        j = [np.empty(self.shape) for _ in range(3)]
         self._chk(self.L.lbgpu_flow_get(self.ctx, _ptr(n), _ptr(rho), *(_ptr(x) for x in j)),
                   "flow_get")
         return n, rho, tuple(j)
@@ -338,7 +339,7 @@ def _mp_init(self, moments=None, charged=False, **tracer):
 
 def _mp_propagate(self, nsteps):
     """Returns (vacf (steps,3), converged)."""
-    v = np.zeros((max(nsteps, 1), 3))
+    v = np.empty((max(nsteps, 1), 3))
     done, conv = C.c_int(0), C.c_int(0)
     rc = self.L.lbgpu_mp_propagate(self.ctx, nsteps, _ptr(v), C.byref(done), C.byref(conv))
     self._chk(rc, "mp_propagate")
@@ -346,8 +347,8 @@ def _mp_propagate(self, nsteps):
 
 
 def _mp_get(self):
-    P = np.zeros(self.shape + (3,))
-    A = np.zeros(self.shape + (3,))
+    P = np.empty(self.shape + (3,))
+    A = np.empty(self.shape + (3,))
     self._chk(self.L.lbgpu_mp_get(self.ctx, _ptr(P), _ptr(A)), "mp_get")
     return P, A
 
@@ -394,7 +395,7 @@ def _pnp_init(self, bjl=0.4, sigma=0.0, lambda_D=4.0, D_plus=0.05, D_minus=0.05,
 
 
 def _pnp_get(self):
-    cp, cm, phi = (np.zeros(self.shape) for _ in range(3))
+    cp, cm, phi = (np.empty(self.shape) for _ in range(3))
     an = C.c_double(0)
     self._chk(self.L.lbgpu_pnp_get(self.ctx, _ptr(cp), _ptr(cm), _ptr(phi), C.byref(an)), "pnp_get")
     return cp, cm, phi, an.value
@@ -705,7 +706,7 @@ class Batch:
 
     def moments(self, box: int):
         shape = self._shapes[box]
-        out = [np.zeros(shape) for _ in range(4)]
+        out = [np.empty(shape) for _ in range(4)]
         self._chk(self.L.lbgpu_batch_moments(self.b, box, *(_ptr(x) for x in out)), "batch_moments")
         return out[0], tuple(out[1:])
 
@@ -723,7 +724,7 @@ class Batch:
     def mp_fields(self, box: int):
         """(P, P_ads) of a box in its tracer phase, shape (lz, ly, lx, 3), as Box.mp_get."""
         shape = self._shapes[box] + (3,)
-        P, A = np.zeros(shape), np.zeros(shape)
+        P, A = np.empty(shape), np.empty(shape)
         self._chk(self.L.lbgpu_batch_mp_fields(self.b, box, _ptr(P), _ptr(A)), "batch_mp_fields")
         return P, A
 
