@@ -3,8 +3,8 @@
 //
 // Large boxes are stored in the fluid-only layout of compact.cuh and cut into tiles of
 // BATCH_BLOCK consecutive fluid nodes; one launch steps every tile of every large box in a phase
-// (a tile never straddles two boxes, so a block reads one descriptor).  In the tracer phase,
-// large boxes at least 32 x 8 wide run shared-memory slab tiles (mp_slab.cuh).  Small boxes are
+// (a tile never straddles two boxes, so a block reads one descriptor).  In the tracer phase, large
+// dense boxes run shared-memory slab tiles (mp_slab.cuh; the rule is in batch_api.cu).  Small boxes are
 // stepped by a persistent block each that loads the whole box (lattice layout) into shared
 // memory, runs all the steps of a call there with a block barrier between steps, and writes it
 // back: HBM is touched twice per call instead of twice per step.  Every box is updated by its
@@ -128,7 +128,7 @@ template <bool INIT>
 __device__ __forceinline__ void mp_node(const float4 *V, const float4 *Pn, float4 *Pnext,
                                         const float4 *An, float4 *Anext, float4 *aux, unsigned r, int x,
                                         int y, int z, uint32_t m, const BatchInst &I, float (&vt)[3],
-                                        unsigned &bad)
+                                        unsigned &bad, float *S = nullptr, unsigned k = 0)
 {
     const int lx = I.lx, ly = I.ly, lz = I.lz;
     const int sy = lx, sz = lx * ly;
@@ -159,6 +159,7 @@ __device__ __forceinline__ void mp_node(const float4 *V, const float4 *Pn, float
         const float spp = INIT ? mp32_scatter(blocked, I.a1[w], mp32_cdot<-c.x, -c.y, -c.z>(vn), I.lwh[w])
                                : mp32_scatter_flag(I.a1[w], mp32_cdot<-c.x, -c.y, -c.z>(vn), __fmul_rn(I.lwh[w], vn.w));
         if constexpr (INIT) {
+            if (S) S[(size_t)(l - 1) * I.Nf + k] = spp;
             const float sp = mp32_scatter(blocked, I.a1[w], mp32_cdot<c.x, c.y, c.z>(vr), I.lwh[w]);
             frac -= sp;
             ux += c.x * sp;
@@ -191,6 +192,74 @@ __device__ __forceinline__ void mp_node(const float4 *V, const float4 *Pn, float
         if (I.ads && (m & INTERFACIAL_BIT)) Anext[r] = mp32_adsorb(p, An[r], I.ka, I.kd, I.one_minus_kd, n0, n1, n2);
         Pnext[r] = make_float4(n0, n1, n2, 0.0f);
     }
+}
+
+// A word that is used once per step: kept out of L1, which holds the rows of P that the next tiles of
+// the SM read again.
+__device__ __forceinline__ float ld_once(const float *p)
+{
+    float v;
+    asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+// One tracer step at fluid node r (compact index k) with its 18 incoming probabilities read from the
+// box's table S[(l-1) Nf + k], which the start of the phase filled with what mp_node forms from V:
+// the same operations on the same values.  A link costs one coalesced word and the neighbour's P
+// instead of two 16-byte gathers, by whose L1 wavefronts (13 each over the rows of a tube) the step
+// was bound.  Of the neighbours' P only the 8 neighbouring columns are loaded: consecutive lanes
+// hold consecutive fluid nodes, so where the lane before (after) holds the node x - 1 (x + 1) of the
+// row, the value at x -+ 1 of a column's row is that lane's; only a lane at the end of a run of
+// fluid nodes loads its own.  Every lane of the warp calls it (lanes beyond the box's nodes with
+// its last node and store = false).
+__device__ __forceinline__ void mp_node_table(const float *__restrict__ S, const float4 *__restrict__ Pn,
+                                              float4 *__restrict__ Pnext, const float4 *An, float4 *Anext,
+                                              const float4 *__restrict__ aux, unsigned k, unsigned r, int x, int y,
+                                              int z, uint32_t m, bool store, const BatchInst &I, float (&vt)[3])
+{
+    const int lx = I.lx, ly = I.ly, lz = I.lz;
+    const unsigned Nf = I.Nf;
+    const int sy = lx, sz = lx * ly;
+    const int Y[3] = {wrap_minus(y, ly) * sy, y * sy, wrap_plus(y, ly) * sy};
+    const int Z[3] = {wrap_minus(z, lz) * sz, z * sz, wrap_plus(z, lz) * sz};
+    const int lane = threadIdx.x & 31;
+    const unsigned before = __shfl_up_sync(0xffffffffu, r, 1), after = __shfl_down_sync(0xffffffffu, r, 1);
+    const bool near_l = lane > 0 && x > 0 && before + 1u == r, near_r = lane < 31 && x < lx - 1 && r + 1u == after;
+    float4 col[9];   // P(x, y + dy, z + dz) at 3 (dz + 1) + dy + 1
+    static_for<0, 9>([&](auto K) {
+        constexpr int q = decltype(K)::value;
+        col[q] = __ldg(Pn + (unsigned)(x + Y[q % 3] + Z[q / 3]));
+    });
+    const float4 p = col[4], ax = __ldg(aux + r);
+    float n0 = 0.0f, n1 = 0.0f, n2 = 0.0f;
+    static_for<1, Q>([&](auto L) {
+        constexpr int l = mp_link_order(decltype(L)::value);
+        constexpr Vel c = vel(l);
+        float4 pn = col[3 * (c.z + 1) + c.y + 1];
+        if constexpr (c.x != 0) {
+            const bool near = c.x < 0 ? near_l : near_r;
+            if constexpr (c.x < 0) {
+                pn.x = __shfl_up_sync(0xffffffffu, pn.x, 1);
+                pn.y = __shfl_up_sync(0xffffffffu, pn.y, 1);
+                pn.z = __shfl_up_sync(0xffffffffu, pn.z, 1);
+            } else {
+                pn.x = __shfl_down_sync(0xffffffffu, pn.x, 1);
+                pn.y = __shfl_down_sync(0xffffffffu, pn.y, 1);
+                pn.z = __shfl_down_sync(0xffffffffu, pn.z, 1);
+            }
+            // a blocked link (probability 0) may keep whatever finite P the shuffle gave
+            if (!near && !((m >> inv(l)) & 1u))
+                pn = __ldg(Pn + (unsigned)((c.x < 0 ? wrap_minus(x, lx) : wrap_plus(x, lx)) + Y[c.y + 1] + Z[c.z + 1]));
+        }
+        mp32_link(ld_once(S + (size_t)(l - 1) * Nf + k), pn, p, n0, n1, n2);
+    });
+    if (!store) return;
+    vt[0] += p.x * ax.x;
+    vt[1] += p.y * ax.y;
+    vt[2] += p.z * ax.z;
+    mp32_finish(p, ax.w, n0, n1, n2);
+    if (I.ads && (m & INTERFACIAL_BIT)) Anext[r] = mp32_adsorb(p, An[r], I.ka, I.kd, I.one_minus_kd, n0, n1, n2);
+    Pnext[r] = make_float4(n0, n1, n2, 0.0f);
 }
 
 __device__ __forceinline__ void lattice_xyz(const BatchInst &I, unsigned r, int &x, int &y, int &z)
@@ -257,6 +326,28 @@ __device__ __forceinline__ void block_sum3(double (&v)[3])
             for (int k = 0; k < nw; ++k) s += sh[d][k];
             v[d] = s;
         }
+}
+
+// Sum of 3 values over a block of BATCH_BLOCK threads; valid in threads 0..2, thread d its value d in
+// v[0].  A warp's 32 terms are added by an FP32 tree (5 roundings; a thread of a slab tile adds up to
+// BATCH_SLAB_ZC terms in FP32 in sequence), the warps in FP64: 5 FP64 additions per value in every
+// warp would take a third of a node tile's time (19 SM cycles each).
+__device__ __forceinline__ double tile_sum3(const float (&t)[3])
+{
+    __shared__ float sh[3][BATCH_BLOCK / 32];
+    float v[3] = {t[0], t[1], t[2]};
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[d] += __shfl_down_sync(0xffffffffu, v[d], o);
+    if ((threadIdx.x & 31) == 0)
+        for (int d = 0; d < 3; ++d) sh[d][threadIdx.x >> 5] = v[d];
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x < 3)
+#pragma unroll
+        for (int k = 0; k < BATCH_BLOCK / 32; ++k) s += (double)sh[threadIdx.x][k];
+    return s;
 }
 
 __device__ __forceinline__ unsigned *status_word(const BatchInst &I)
@@ -389,21 +480,38 @@ __global__ void __launch_bounds__(BATCH_BLOCK, MINB) k_batch_aa_list(const Batch
     release_ticket(tk);
 }
 
-// One tracer step of every tiled box in the tracer phase; with INIT (one box, the tiles of
-// `inst` in order), the start of its tracer phase.  Each tile keeps its own running sums.
+// One tracer step of every tiled box in the tracer phase (inst: the number of SMs); with INIT (one
+// box, the tiles of `inst` in order), the start of its tracer phase.  Each tile keeps its own running
+// sums.  Bound by L2 and memory traffic (the table's 72 B, P of the neighbouring rows, (u*, D)) at
+// large sizes.  16 tubes of 32^2 x L (846 k fluid nodes), per step: 54.9 us as slab tiles, 48.5 as
+// node tiles forming the probabilities from V, 41 with the table, 35.5 with each SM on a run of
+// consecutive tiles (42 registers: 51, 64 and 85 take 39.9, 42.5 and 46.6 us); 82 us before the FP64
+// shuffles of the VACF terms were taken out of the node tiles.
 template <bool INIT>
-__global__ void __launch_bounds__(BATCH_BLOCK) k_batch_mp(const BatchInst *__restrict__ insts,
+__global__ void __launch_bounds__(BATCH_BLOCK, 6) k_batch_mp(const BatchInst *__restrict__ insts,
                                                           const BatchTile *__restrict__ tiles,
                                                           int inst, int par)
 {
     BatchTile t;
-    if constexpr (INIT) t = BatchTile{inst, (int)blockIdx.x * BATCH_BLOCK};
-    else t = tiles[blockIdx.x];
+    if constexpr (INIT) {
+        t = BatchTile{inst, (int)blockIdx.x * BATCH_BLOCK};
+    } else {
+        // blocks are handed out to the SMs in turn: each SM's share is a run of consecutive tiles,
+        // whose neighbours' rows it has in L1
+        const unsigned sms = (unsigned)inst, sm = blockIdx.x % sms, q = gridDim.x / sms, rem = gridDim.x % sms;
+        t = tiles[sm * q + min(sm, rem) + blockIdx.x / sms];
+    }
     const BatchInst &I = insts[t.inst];
     const unsigned k = (unsigned)t.start + threadIdx.x;   // node in the box's layout
     float vt32[3] = {0.0f, 0.0f, 0.0f};
     unsigned bad = 0;
-    if (k < batch_units(I)) {
+    if (!INIT && I.S) {   // whole warps: their lanes exchange neighbours
+        const unsigned kk = min(k, I.Nf - 1u);
+        int x, y, z;
+        const unsigned r = compact_xyz(I, __ldg(I.cpos + kk), x, y, z);
+        mp_node_table(I.S, I.P[par], I.P[par ^ 1], I.A[par], I.A[par ^ 1], I.aux, kk, r, x, y, z, __ldg(I.cmask + kk),
+                      k < I.Nf, I, vt32);
+    } else if (k < batch_units(I)) {
         uint32_t m;
         unsigned r;
         int x, y, z;
@@ -416,73 +524,31 @@ __global__ void __launch_bounds__(BATCH_BLOCK) k_batch_mp(const BatchInst *__res
             lattice_xyz(I, r, x, y, z);
         }
         if (m & FLUID_BIT) {
-            if constexpr (INIT) mp_node<true>(I.V, nullptr, I.P[0], nullptr, nullptr, I.aux, r, x, y, z, m, I, vt32, bad);
+            if constexpr (INIT)
+                mp_node<true>(I.V, nullptr, I.P[0], nullptr, nullptr, I.aux, r, x, y, z, m, I, vt32, bad, I.S, k);
             else mp_node<false>(I.V, I.P[par], I.P[par ^ 1], I.A[par], I.A[par ^ 1], I.aux, r, x, y, z, m, I, vt32, bad);
         }
     }
-    double vt[3] = {(double)vt32[0], (double)vt32[1], (double)vt32[2]};
-    block_sum3(vt);
-    if (threadIdx.x == 0) {
-        double *acc = I.tacc + (size_t)(t.start / BATCH_BLOCK) * BATCH_TACC;
-        if constexpr (INIT) {
+    double *acc = I.tacc + (size_t)(t.start / BATCH_BLOCK) * BATCH_TACC;
+    if constexpr (INIT) {
+        double vt[3] = {(double)vt32[0], (double)vt32[1], (double)vt32[2]};
+        block_sum3(vt);
+        if (threadIdx.x == 0)
             for (int d = 0; d < 3; ++d) {
                 acc[d] = vt[d] * (double)I.bw;
                 acc[3 + d] = 0.0;
                 acc[6 + d] = 0.0;
             }
-        } else {
-            for (int d = 0; d < 3; ++d) {
-                acc[3 + d] += vt[d];
-                acc[6 + d] = vt[d];
-            }
+    } else {
+        const double v = tile_sum3(vt32);
+        if (threadIdx.x < 3) {
+            acc[3 + threadIdx.x] += v;
+            acc[6 + threadIdx.x] = v;
         }
     }
     if constexpr (INIT) {
         if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(status_word(I), (unsigned)LBGPU_ERR_FRACTION);
     }
-}
-
-// The work-list form of the tiled tracer step (see k_batch_aa_list).
-__global__ void __launch_bounds__(BATCH_BLOCK) k_batch_mp_list(const BatchInst *__restrict__ insts,
-                                                               const BatchTile *__restrict__ tiles,
-                                                               int ntiles, int tpc, int par, BatchTicket *tk)
-{
-    unsigned b0, b1;
-    while (claim_tiles(tk, ntiles, tpc, b0, b1)) {
-        for (unsigned kt = b0; kt < b1; ++kt) {
-            const BatchTile t = tiles[kt];
-            const BatchInst &I = insts[t.inst];
-            const unsigned k = (unsigned)t.start + threadIdx.x;
-            float vt32[3] = {0.0f, 0.0f, 0.0f};
-            unsigned bad = 0;
-            if (k < batch_units(I)) {
-                uint32_t m;
-                unsigned r;
-                int x, y, z;
-                if (I.compact) {
-                    m = __ldg(I.cmask + k);
-                    r = compact_xyz(I, __ldg(I.cpos + k), x, y, z);
-                } else {
-                    m = __ldg(I.mask + k);
-                    r = k;
-                    lattice_xyz(I, r, x, y, z);
-                }
-                if (m & FLUID_BIT)
-                    mp_node<false>(I.V, I.P[par], I.P[par ^ 1], I.A[par], I.A[par ^ 1], I.aux, r, x, y, z, m, I,
-                                   vt32, bad);
-            }
-            double vt[3] = {(double)vt32[0], (double)vt32[1], (double)vt32[2]};
-            block_sum3(vt);
-            if (threadIdx.x == 0) {
-                double *acc = I.tacc + (size_t)(t.start / BATCH_BLOCK) * BATCH_TACC;
-                for (int d = 0; d < 3; ++d) {
-                    acc[3 + d] += vt[d];
-                    acc[6 + d] = vt[d];
-                }
-            }
-        }
-    }
-    release_ticket(tk);
 }
 
 // One tracer step of the slab tiles of boxes in the tracer phase (mp_slab.cuh); each tile keeps
@@ -703,11 +769,11 @@ cudaError_t launch_batch_aa(const BatchInst *insts, const BatchTile *tiles, int 
     return cudaGetLastError();
 }
 
-cudaError_t launch_batch_mp(const BatchInst *insts, const BatchTile *tiles, int ntiles, int par,
+cudaError_t launch_batch_mp(const BatchInst *insts, const BatchTile *tiles, int ntiles, int par, int sms,
                             cudaStream_t s)
 {
     if (ntiles <= 0) return cudaSuccess;
-    k_batch_mp<false><<<ntiles, BATCH_BLOCK, 0, s>>>(insts, tiles, 0, par);
+    k_batch_mp<false><<<ntiles, BATCH_BLOCK, 0, s>>>(insts, tiles, sms, par);
     return cudaGetLastError();
 }
 
@@ -728,15 +794,6 @@ cudaError_t launch_batch_aa_list(const BatchInst *insts, const BatchTile *tiles,
     else if (minb == 4) batch_aa_list<4>(insts, tiles, ntiles, odd, grid, tpc, tk, s);
     else if (minb == 5) batch_aa_list<5>(insts, tiles, ntiles, odd, grid, tpc, tk, s);
     else batch_aa_list<6>(insts, tiles, ntiles, odd, grid, tpc, tk, s);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_batch_mp_list(const BatchInst *insts, const BatchTile *tiles, int ntiles, int par, int grid,
-                                 int tpc, BatchTicket *tk, cudaStream_t s)
-{
-    if (ntiles <= 0) return cudaSuccess;
-    grid = std::max(1, std::min(grid, (ntiles + tpc - 1) / tpc));
-    k_batch_mp_list<<<grid, BATCH_BLOCK, 0, s>>>(insts, tiles, ntiles, tpc, par, tk);
     return cudaGetLastError();
 }
 

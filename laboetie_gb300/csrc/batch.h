@@ -33,6 +33,9 @@ struct BatchInst {
     float4 *V;              // tracer phase: (j + f_ext)/rho per node (0 on solid nodes)
     float4 *P[2], *A[2];    // propagated quantity / adsorbed part, by step parity
     float4 *aux;            // per fluid node, fixed for the tracer phase: (u*, D) of mp_f32.cu
+    // tracer phase of a box with node tiles, where the batch's budget has room: the 18 incoming
+    // scattering probabilities of every fluid node, S[(l-1) Nf + i]; else null (formed from V)
+    float *S;
     double *tacc;           // BATCH_TACC doubles per tile of BATCH_BLOCK nodes, then a status word
     int lx, ly, lz, N;
     int phase, ads;
@@ -82,10 +85,8 @@ cudaError_t launch_batch_aa(const BatchInst *insts, const BatchTile *tiles, int 
 cudaError_t launch_batch_aa_list(const BatchInst *insts, const BatchTile *tiles, int ntiles, bool odd, int minb,
                                  int grid, int tpc, BatchTicket *tk, cudaStream_t s);
 // one tracer step of the tiled boxes: P[par] -> P[par^1]
-cudaError_t launch_batch_mp(const BatchInst *insts, const BatchTile *tiles, int ntiles, int par,
+cudaError_t launch_batch_mp(const BatchInst *insts, const BatchTile *tiles, int ntiles, int par, int sms,
                             cudaStream_t s);
-cudaError_t launch_batch_mp_list(const BatchInst *insts, const BatchTile *tiles, int ntiles, int par, int grid,
-                                 int tpc, BatchTicket *tk, cudaStream_t s);
 // the same for boxes with slab tiles (tile start = slab tile index within the box)
 cudaError_t launch_batch_mp_slab(const BatchInst *insts, const BatchTile *tiles, int ntiles, int par,
                                  cudaStream_t s);

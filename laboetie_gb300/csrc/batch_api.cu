@@ -122,6 +122,9 @@ struct lbgpu_batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, fork = nullptr, join = nullptr, join2 = nullptr;
     cudaEvent_t fork_mp = nullptr, join_mp = nullptr;
     size_t budget = 0, used = 0;
+    // bytes of the boxes' probability tables (BatchInst::S): taken from what the budget leaves, given
+    // back as soon as a box needs the room, and not part of a box's footprint
+    size_t tables = 0;
     int smem_max = BATCH_SMEM_BYTES_MAX;
     std::vector<Slot> slots;
     unsigned long long *d_counts = nullptr;
@@ -175,6 +178,8 @@ int grow(T **p, int &cap, int need, cudaStream_t s)
     cap = nc;
     return LBGPU_OK;
 }
+
+size_t table_bytes(const BatchInst &d) { return sizeof(float) * (Q - 1) * (size_t)d.Nf; }
 
 int workspace(lbgpu_batch *b, size_t bytes)
 {
@@ -291,6 +296,21 @@ int rebuild(lbgpu_batch *b)
     return LBGPU_OK;
 }
 
+// Frees the tables of boxes (their steps form the probabilities from V again, with the same bits)
+// until `need` more bytes fit the budget.
+int make_room(lbgpu_batch *b, size_t need)
+{
+    for (auto &sl : b->slots) {
+        if (b->used + b->tables + need <= b->budget) break;
+        if (!sl.active || !sl.d.S) continue;
+        LBB_CK(cudaFreeAsync(sl.d.S, b->stream));
+        sl.d.S = nullptr;
+        b->tables -= table_bytes(sl.d);
+        b->dirty = true;
+    }
+    return LBGPU_OK;
+}
+
 // One AA launch of the flow-phase tiles in the variant the tuner chose (descriptors insts: the
 // batch's, or the tuner's scratch copies).
 int launch_aa(lbgpu_batch *b, const BatchInst *insts, int odd, cudaStream_t s)
@@ -358,7 +378,7 @@ int enqueue_steps(lbgpu_batch *b, int nsteps, bool check, bool smem)
         if (flow_tiles)
             if (int rc = launch_aa(b, b->d_insts, t & 1, s)) return rc;
         if (mp_tiles) {
-            LBB_CK(launch_batch_mp(b->d_insts, b->d_tiles + b->nflow, b->nmp, t & 1, ms));
+            LBB_CK(launch_batch_mp(b->d_insts, b->d_tiles + b->nflow, b->nmp, t & 1, b->sms, ms));
             LBB_CK(launch_batch_mp_slab(b->d_insts, b->d_tiles + b->nflow + b->nmp, b->nslab, t & 1, ms));
         }
     }
@@ -737,8 +757,10 @@ void lbgpu_batch_destroy(lbgpu_batch *b)
     if (b->side2) cudaStreamSynchronize(b->side2);
     if (b->side3) cudaStreamSynchronize(b->side3);
     drop_graphs(b);
-    for (auto &sl : b->slots)
+    for (auto &sl : b->slots) {
         if (sl.active) cudaFree(sl.mem);
+        if (sl.active) cudaFree(sl.d.S);
+    }
     cudaFree(b->d_insts);
     cudaFree(b->d_tiles);
     cudaFree(b->d_smem);
@@ -801,27 +823,45 @@ int lbgpu_batch_add(lbgpu_batch *b, const lbgpu_cell *c, const int8_t *nature, i
         return bfail(LBGPU_ERR_INVALID, "lbgpu_batch_add: box shape beyond the packed-position limits");
     if (compact && pos.empty()) return bfail(LBGPU_ERR_INVALID, "All nodes are solid: no fluid, no fluid dynamics!");
     const long long units = compact ? (long long)pos.size() : N;
-    // LBGPU_BATCH_SLAB=0: tiled boxes take node tiles in the tracer phase too (same bits)
+    // Slab tiles (mp_slab.cuh) or node tiles in the tracer phase: the same P, so a matter of speed, and
+    // decided by the box alone (its VACF sums are grouped by its tiles, and a box gives the same bits
+    // in any batch).  A slab tile sweeps 16 planes in about 27 us however few tiles there are, and
+    // visits solid nodes; a node tile costs 0.04 ns per fluid node at any porosity.  us per step of
+    // 1 / 4 / 40 boxes, slab against node tiles: touching spheres 64^3 (0.32 fluid) 27 / 34 / 212
+    // against 6.3 / 14 / 144, porous 64^3 (0.60) 28 / 37 / 223 against 7.2 / 24 / 255, cylinder
+    // 96^2 x 32 (0.72) 27 / 35 / 229 against 8.6 / 29 / 329, all fluid 64^3 23 / 29 / 188 against
+    // 11 / 34 / 368.  LBGPU_BATCH_SLAB=0 / 1: node / slab tiles for every box.
     const char *slab_env = std::getenv("LBGPU_BATCH_SLAB");
-    const bool slab_ok = !(slab_env && std::string(slab_env) == "0");
-    const int nslab = compact && tracer && slab_ok ? batch_slab_tiles(c->lx, c->ly, c->lz) : 0;
-    const int ntacc = std::max((int)((units + BATCH_BLOCK - 1) / BATCH_BLOCK), nslab);
+    const std::string slab_mode = slab_env ? slab_env : "";
+    int nslab = compact && tracer && slab_mode != "0" ? batch_slab_tiles(c->lx, c->ly, c->lz) : 0;
     sl.slab_live.clear();
     if (nslab) {   // slab tile k: column tile k % nxy (MPS_TX x MPS_TY), planes [zc (k / nxy), + zc)
         const int tx = (c->lx + MPS_TX - 1) / MPS_TX, nxy = tx * ((c->ly + MPS_TY - 1) / MPS_TY);
+        long long nodes = 0;   // lattice nodes of the live tiles
         for (int k = 0; k < nslab; ++k) {
             const int t = k % nxy, x0 = (t % tx) * MPS_TX, y0 = (t / tx) * MPS_TY, z0 = (k / nxy) * BATCH_SLAB_ZC;
+            const int x1 = std::min(x0 + MPS_TX, c->lx), y1 = std::min(y0 + MPS_TY, c->ly),
+                      z1 = std::min(z0 + BATCH_SLAB_ZC, c->lz);
             bool fluid = false;
-            for (int z = z0; z < std::min(z0 + BATCH_SLAB_ZC, c->lz) && !fluid; ++z)
-                for (int y = y0; y < std::min(y0 + MPS_TY, c->ly) && !fluid; ++y)
-                    for (int x = x0; x < std::min(x0 + MPS_TX, c->lx); ++x)
+            for (int z = z0; z < z1 && !fluid; ++z)
+                for (int y = y0; y < y1 && !fluid; ++y)
+                    for (int x = x0; x < x1; ++x)
                         if (nature[(size_t)x + (size_t)c->lx * ((size_t)y + (size_t)c->ly * z)] == 0) {
                             fluid = true;
                             break;
                         }
-            if (fluid) sl.slab_live.push_back(k);
+            if (!fluid) continue;
+            sl.slab_live.push_back(k);
+            nodes += (long long)(x1 - x0) * (y1 - y0) * (z1 - z0);
+        }
+        const double share = (double)units / (double)nodes;
+        const size_t live = sl.slab_live.size();
+        if (slab_mode != "1" && !((share >= 0.65 && live >= 64) || (share >= 0.5 && live >= 256))) {
+            nslab = 0;
+            sl.slab_live.clear();
         }
     }
+    const int ntacc = std::max((int)((units + BATCH_BLOCK - 1) / BATCH_BLOCK), nslab);
     const Layout L = layout(N, units, (long long)tab.size(), ntacc, compact, tracer, ads);
     if (b->used + L.total > b->budget)
         return bfail(LBGPU_ERR_OOM, "lbgpu_batch_add: box needs " + std::to_string(L.total >> 20) +
@@ -829,7 +869,14 @@ int lbgpu_batch_add(lbgpu_batch *b, const lbgpu_cell *c, const int8_t *nature, i
     cudaStream_t s = b->stream;
     sl.bytes = L.total;
     sl.ntile = ntacc;
-    LBB_CK(cudaMallocAsync(&sl.mem, L.total, s));
+    if (int rc = make_room(b, L.total)) return rc;
+    cudaError_t me = cudaMallocAsync(&sl.mem, L.total, s);
+    if (me == cudaErrorMemoryAllocation && b->tables) {   // others use the device too: without tables
+        cudaGetLastError();
+        if (int rc = make_room(b, b->budget)) return rc;
+        me = cudaMallocAsync(&sl.mem, L.total, s);
+    }
+    LBB_CK(me);
     char *base = static_cast<char *>(sl.mem);
     BatchInst &d = sl.d;
     std::memset(&d, 0, sizeof(d));
@@ -914,6 +961,10 @@ int lbgpu_batch_remove(lbgpu_batch *b, int id)
     if (!valid_slot(b, id)) return bfail(LBGPU_ERR_INVALID, "lbgpu_batch_remove: no such box");
     Slot &sl = b->slots[id];
     LBB_CK(cudaFreeAsync(sl.mem, b->stream));
+    if (sl.d.S) {
+        LBB_CK(cudaFreeAsync(sl.d.S, b->stream));
+        b->tables -= table_bytes(sl.d);
+    }
     b->used -= sl.bytes;
     sl = Slot();
     b->dirty = true;
@@ -1005,9 +1056,19 @@ int lbgpu_batch_mp_start(lbgpu_batch *b, int id)
     Slot &sl = b->slots[id];
     if (!sl.tracer) return bfail(LBGPU_ERR_INVALID, "lbgpu_batch_mp_start: the box has no tracer (tracer.Db = 0)");
     if (sl.d.phase != BATCH_FLOW) return bfail(LBGPU_ERR_INVALID, "lbgpu_batch_mp_start: tracer phase already started");
+    cudaStream_t s = b->stream;
+    const size_t tb = table_bytes(sl.d);
+    if (sl.d.compact && sl.d.zc == 0 && !sl.d.S && b->used + b->tables + tb <= b->budget) {
+        if (cudaMallocAsync((void **)&sl.d.S, tb, s) == cudaSuccess) {
+            b->tables += tb;
+            b->dirty = true;
+        } else {
+            cudaGetLastError();   // no room on the device: without a table
+            sl.d.S = nullptr;
+        }
+    }
     int rc = rebuild(b);
     if (rc) return rc;
-    cudaStream_t s = b->stream;
     LBB_CK(launch_batch_mp_start(b->d_insts, desc_of(b, id), batch_units(sl.d), s));
     unsigned st = 0;
     LBB_CK(cudaMemcpyAsync(&st, sl.d.tacc + (size_t)sl.ntile * BATCH_TACC, sizeof(st), cudaMemcpyDeviceToHost, s));
