@@ -88,11 +88,20 @@ cudaError_t launch_finalize_f64(const FlowArgs64 &a, bool field, cudaStream_t s)
 // init_simu.f90:31-39: raw n = w*rho0 into buffer (parity), rho, j = 0
 cudaError_t launch_init_f64(const FlowArgs64 &a, double rho0, cudaStream_t s);
 
+// the same for a small FP64 box (flow_f64_resident.cu): nsteps steps of the reference loop on the
+// control block a.ctl, or fixed steps from a.parity with a.force_moment / a.force_collide in the
+// first and fon in the moments of the later ones
+struct ResidentPlan;
+ResidentPlan plan_resident64(unsigned long long Nf, long long N, int fmask, bool fused);
+cudaError_t launch_resident64(const ResidentPlan &plan, const FlowArgs64 &a, int fmask, void *sync, int nsteps, bool loop,
+                              int fon, cudaStream_t s);
+
 // FP32 deviation ------------------------------------------------------------------------
 // many steps of one box in one launch (flow_f32_resident.cu): blocks 0 when the box is not run so
 struct ResidentPlan {
     unsigned blocks, threads;
-    bool cluster;
+    bool cluster;   // FP32: one thread-block cluster
+    bool split;     // FP64: four warps per node
 };
 ResidentPlan plan_resident32(unsigned Nf, bool wide, bool loop);   // fixed steps, or the reference loop
 size_t grid_sync_bytes();   // device bytes of `sync` below

@@ -148,6 +148,8 @@ int ctx_init_device(lbgpu_ctx *ctx, const int8_t *nature)
         LBG_CK(ctx, cudaMemcpyAsync(ctx->d_fidx, fidx.data(), sizeof(uint32_t) * fidx.size(),
                                     cudaMemcpyHostToDevice, ctx->stream));
         LBG_CK(ctx, cudaStreamSynchronize(ctx->stream));   // the host list goes out of scope
+        ctx->resident = plan_resident64(ctx->counts[0], N, force_mask(p.f_ext), p.precision == LBGPU_FP64_FUSED);
+        if (ctx->resident.blocks) LBG_CK(ctx, cudaMalloc(&ctx->d_gsync, grid_sync_bytes()));
     } else {
         const char *mode = std::getenv("LBGPU_FP32_STREAMING");
         ctx->aa = !(mode && std::string(mode) == "ab");
@@ -326,6 +328,7 @@ int lbgpu_flow_get(lbgpu_ctx *ctx, double *n, double *density, double *jx, doubl
     if (ctx->p.precision == LBGPU_FP32_DEV) return f32_flow_get(ctx, n, density, jx, jy, jz);
     if (ctx->prev_kind == PREV_NONE)
         return ctx_fail(ctx, LBGPU_ERR_INVALID, "lbgpu_flow_get: no flow state (call lbgpu_flow_init)");
+    if (int rc = resident_status(ctx)) return rc;
     const long long N = ctx->N;
     cudaStream_t s = ctx->stream;
     const int prev = 1 - ctx->cur;
@@ -496,27 +499,32 @@ int lbgpu_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int h
     a.Fx = ctx->d_F[0];
     a.Fy = ctx->d_F[1];
     a.Fz = ctx->d_F[2];
-    // one CUDA graph of G launches; the control block makes launches after the exit no-ops
-    const long long N = ctx->N;
-    int G = (int)std::min<long long>(512, std::max<long long>(8, (1LL << 24) / std::max<long long>(N, 1)));
-    if (max_steps > 0) G = std::min(G, max_steps + 8);
-    cudaGraph_t graph;
-    cudaGraphExec_t exec;
-    LBG_CK(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    for (int g = 0; g < G; ++g) {
-        cudaError_t e = launch_flow_step_f64(a, fmask, field, true, true, s);
-        if (e != cudaSuccess) {
-            cudaStreamEndCapture(s, &graph);
-            return ctx_cuda(ctx, e, "capture flow step");
+    const bool resident = ctx->resident.blocks > 0 && !field;
+    cudaGraphExec_t exec = nullptr;
+    if (!resident) {
+        // one CUDA graph of G launches; the control block makes launches after the exit no-ops
+        const long long N = ctx->N;
+        int G = (int)std::min<long long>(512, std::max<long long>(8, (1LL << 24) / std::max<long long>(N, 1)));
+        if (max_steps > 0) G = std::min(G, max_steps + 8);
+        cudaGraph_t graph;
+        LBG_CK(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        for (int g = 0; g < G; ++g) {
+            cudaError_t e = launch_flow_step_f64(a, fmask, field, true, true, s);
+            if (e != cudaSuccess) {
+                cudaStreamEndCapture(s, &graph);
+                return ctx_cuda(ctx, e, "capture flow step");
+            }
         }
+        LBG_CK(ctx, cudaStreamEndCapture(s, &graph));
+        LBG_CK(ctx, cudaGraphInstantiate(&exec, graph, 0));
+        cudaGraphDestroy(graph);
     }
-    LBG_CK(ctx, cudaStreamEndCapture(s, &graph));
-    LBG_CK(ctx, cudaGraphInstantiate(&exec, graph, 0));
-    cudaGraphDestroy(graph);
     FlowCtl h;
     int rc = LBGPU_OK;
     for (;;) {
-        cudaError_t e = cudaGraphLaunch(exec, s);
+        constexpr int RES_CHUNK = 1024;   // steps of a resident launch: some 10 ms
+        cudaError_t e = resident ? launch_resident64(ctx->resident, a, fmask, ctx->d_gsync, RES_CHUNK, true, 0, s)
+                                 : cudaGraphLaunch(exec, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h, ctx->d_ctl, sizeof(h), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
@@ -525,8 +533,13 @@ int lbgpu_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int h
         }
         if (h.done) break;
     }
-    cudaGraphExecDestroy(exec);
+    if (exec) cudaGraphExecDestroy(exec);
     if (rc) return rc;
+    if (h.status & LBGPU_ERR_TIMEOUT) {
+        LBG_CK(ctx, cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(h.status), s));
+        if (d_hist) cudaFreeAsync(d_hist, s);
+        return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, "equilibration: a block did not reach the grid's barrier within its wait limit");
+    }
     ctx->cur = h.parity;
     ctx->prev_kind = PREV_POST;
     ctx->prev_force_moment = h.exit_force_moment;
@@ -549,6 +562,28 @@ int lbgpu_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int h
     return LBGPU_OK;
 }
 
+// Fixed steps of a small box as resident launches; fewer than RES_MIN are not worth their set-up.
+static constexpr int RES_MIN = 4;
+static int resident_steps64(lbgpu_ctx *ctx, FlowArgs64 &a, int fmask, int nsteps, int force_on)
+{
+    a.ctl = ctx->d_ctl;   // where a wait that runs out is reported
+    for (int left = nsteps; left > 0;) {
+        const int n = std::min(left, 1024);
+        left -= n;
+        a.parity = ctx->cur;
+        a.force_moment = ctx->force_last_collide;
+        a.force_collide = force_on;
+        LBG_CK(ctx, launch_resident64(ctx->resident, a, fmask, ctx->d_gsync, n, false, force_on, ctx->stream));
+        ctx->prev_force_moment = n >= 2 ? force_on : ctx->force_last_collide;
+        ctx->force_last_collide = force_on;
+        ctx->cur ^= n & 1;
+    }
+    ctx->prev_kind = PREV_POST;
+    ctx->moments_valid = false;
+    ctx->resident_unchecked = true;
+    return LBGPU_OK;
+}
+
 int lbgpu_flow_steps(lbgpu_ctx *ctx, int nsteps, int force_on)
 {
     TraceRange trace_("lbgpu_flow_steps");
@@ -559,6 +594,7 @@ int lbgpu_flow_steps(lbgpu_ctx *ctx, int nsteps, int force_on)
     FlowArgs64 a;
     fill_args64(ctx, a);
     const int fmask = force_mask(ctx->p.f_ext);
+    if (ctx->resident.blocks && nsteps >= RES_MIN) return resident_steps64(ctx, a, fmask, nsteps, force_on ? 1 : 0);
     for (int t = 0; t < nsteps; ++t) {
         a.parity = ctx->cur;
         a.force_moment = ctx->force_last_collide;
