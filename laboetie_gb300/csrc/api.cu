@@ -88,6 +88,13 @@ LbConst64 make_const64(double tau)
         K.c2a2cs2[w] = K.c2a2[w] * csq;
         K.c3a1[w] = K.c3 * K.a1[w];
     }
+    K.fix_c2 = std::llrint(std::ldexp(K.c2, 61));   // tau >= 1/2: at most 2^62
+    K.fix_c1 = (1ll << 62) - 2 * K.fix_c2;
+    K.fix_c3 = (1ll << 62) - K.fix_c2;
+    __int128 sum = std::llrint(std::ldexp(K.c1, 62));
+    for (int w = 0; w < 3; ++w) sum += (__int128)(w == 0 ? 1 : 6 * w) * std::llrint(std::ldexp(K.c2a0[w], 62));
+    K.fix_loss = (int)(2 * (((__int128)1 << 62) - sum));
+    K.fix_c2_36 = (long long)(((unsigned __int128)K.fix_c2 * 8 + 4) / 9);
     return K;
 }
 

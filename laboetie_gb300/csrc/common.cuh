@@ -85,6 +85,10 @@ struct LbConst64 {
     // the pair-symmetric collision of LBGPU_FP64_FUSED, per weight class: c2 a0, c2 a1, c2 a2,
     // c2 a2 cs^2, c3 a1
     double c2a0[3], c2a1[3], c2a2[3], c2a2cs2[3], c3a1[3];
+    // and its fixed-point form (flow64.cuh): c1 2^62 = 2^62 - 2 fix_c2, c2 2^61, c3 2^62 = 2^62 -
+    // fix_c2, c2/36 2^66, 2^63 (1 - c1 - sum of c2 a0)
+    long long fix_c1, fix_c2, fix_c3, fix_c2_36;
+    int fix_loss;
 };
 
 // Device-resident control block of the reference flow loop (equilibration.f90:143-491).

@@ -248,6 +248,214 @@ __device__ __forceinline__ void collide_node_fused(double (&n)[Q], const double 
     });
 }
 
+// ---- LBGPU_FP64_FUSED in 64-bit fixed point
+//
+// The FP64 pipe issues one warp instruction per 19 cycles of an SM, a 64-bit integer addition takes
+// 0.3 and the high half of a 64 x 64-bit product 4.4, and the integer pipes are otherwise idle here.
+// So the fused step of an ordinary node runs in fixed point: its populations become integers on a
+// grid 60 bits below the largest one's binade (exact while they are within 2^7 of it, and finer
+// than its rounding below), moments are exact integer sums, and each result is rounded once to a
+// double.  j and what is made of it carry 3 more bits, so that the rounding down of a product's high
+// half leaves no bias worth a tenth of a unit (a bias in j, unlike a random error, adds up like a
+// force).  With c at the scale of a diagonal link (a0 = 1/36, a1 = 1/12, a2 = 1/8;
+// an axis link has twice each, the rest velocity 12 times a0), per pair of opposite velocities:
+//   H = c2 j/8 + c3 F/4,  b = (c2 j + c3 F)/12,  Q = sum_a u_a H_a,  base = c2 rho/36 - Q/3
+//   n'(l, inv l) = [c1 s/2 + base + (c.u)(c.H)] +- [c1 d/2 + c.b],   s, d = n_l +- n_inv
+// the same regrouping as collide_node_fused's.  (c.u)(c.H) of the two pairs of a plane comes from
+// one product and the squares; the rest population takes what the others leave of rho.  The rounded
+// constants of the FP64 form do not quite sum to 1 (at tau = 1 as the weights in the reference's
+// code: 1/3 + 6/18 + 12/36 = 1 - 2^-54), so a step changes a node's mass by a fixed share of it: the
+// rest population takes that too (fix_loss; 4e-13 of rho after 7000 steps, and the tracer sums
+// depend on rho).  Nodes outside the fixed-point range -- a negative or non-finite
+// population, the largest one below 2^-895, rho from 8 times the largest one's binade up, |j| from
+// a quarter of it up, a force from a sixteenth of it up -- take the FP64 form.
+// Porous medium of 128^3 (1.26 M fluid nodes), tau 0.8: 400 -> 165 us a step (57 us of HBM traffic;
+// now bound by the integer pipes).  Error of j against binary128 after 120 steps of 24^3, tau 0.62 /
+// 0.8 / 1.3: 1.4e-13 / 5e-13 / 3.5e-13 of its norm where the FP64 form has 6e-13 / 8e-13 / 9e-13.
+
+__device__ __forceinline__ long long mulhi(long long a, long long b) { return __mul64hi(a, b); }
+
+// value of v units of 2^(emax - 1082), rounded to nearest even
+__device__ __forceinline__ double fixed_to_double(long long v, int emax)
+{
+    const int hi = (int)(v >> 32);
+    const int sh = 11 - __clz(hi);   // drops v to 53 bits
+    if (hi <= 0 || sh < 1) {         // negative or small: by conversion, its exponent shifted
+        if (v == 0) return 0.0;
+        const double r = (double)v;
+        return __hiloint2double(__double2hiint(r) + (emax - 1082) * (1 << 20), __double2loint(r));
+    }
+    const unsigned lo = (unsigned)v, half = 1u << (sh - 1);
+    const unsigned long long m = ((unsigned long long)v + (half - 1u) + ((lo >> sh) & 1u)) >> sh;
+    // the leading 1 of m adds one to the exponent field
+    return __longlong_as_double((long long)(m + ((unsigned long long)(unsigned)(emax - 8 + sh) << 52)));
+}
+
+// j: units of 2^(emax - 1085), of either sign and any size
+__device__ __forceinline__ double signed_fixed(long long v, int emax)
+{
+    const double r = (double)v;
+    return v == 0 ? 0.0 : __hiloint2double(__double2hiint(r) + (emax - 1085) * (1 << 20), __double2loint(r));
+}
+
+// |x| for a comparison (a NaN or infinity compares above every finite bound as its bits do)
+__device__ __forceinline__ unsigned long long fabs_bits(double x)
+{
+    return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+
+// F in units of 2^(emax - 1085), to nearest; |F| must lie below the largest population's binade
+__device__ __forceinline__ long long force_to_fixed(double F, int emax)
+{
+    const unsigned hi = (unsigned)__double2hiint(F), lo = (unsigned)__double2loint(F);
+    const int e = (int)((hi >> 20) & 0x7ffu), sh = 10 - (emax - e);
+    const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | (e ? 0x100000u : 0u)) << 32) | lo;
+    const int down = min(-sh, 62);
+    const long long v = (long long)(sh >= 0 ? m << sh : (m + (1ull << (down - 1))) >> down);
+    return (int)hi < 0 ? -v : v;
+}
+
+// One fused step of a node: n, after streaming, becomes the collided populations.  Returns false,
+// with n untouched, for a node outside the fixed-point range.  WANT_J: its j, as doubles.
+template <int FMASK, bool WANT_J>
+__device__ __forceinline__ bool fused_fixed(double (&n)[Q], const bool fm, const bool fc, const double fx,
+                                            const double fy, const double fz, const FlowArgs64 &a, double &ox,
+                                            double &oy, double &oz)
+{
+    const LbConst64 &K = a.K;
+    int emax = 0;
+    unsigned sign = 0;
+#pragma unroll
+    for (int l = 0; l < Q; ++l) {
+        const unsigned hi = (unsigned)__double2hiint(n[l]);
+        sign |= hi;
+        emax = max(emax, (int)(hi >> 20));
+    }
+    if ((int)sign < 0 || emax >= 0x7ff || emax < 128) return false;
+    long long v[Q];
+#pragma unroll
+    for (int l = 0; l < Q; ++l) {
+        const unsigned hi = (unsigned)__double2hiint(n[l]), lo = (unsigned)__double2loint(n[l]);
+        const int e = (int)(hi >> 20), sh = 7 - (emax - e);
+        const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
+        v[l] = e == 0 ? 0ll : (long long)(sh >= 0 ? m << sh : m >> min(-sh, 63));
+    }
+    // rho in three parts that cannot overflow (each v < 2^60)
+    const long long r0 = v[0] + v[1] + v[2] + v[3] + v[4] + v[5] + v[6];
+    const long long r1 = v[7] + v[8] + v[9] + v[10] + v[11] + v[12];
+    const long long r2 = v[13] + v[14] + v[15] + v[16] + v[17] + v[18];
+    const long long R = r0 + r1 + r2;
+    constexpr long long LO = 1ll << 59, HI = 1ll << 62;
+    if (r0 >= HI || r1 >= HI / 2 || r2 >= HI / 2 || R < LO || R >= HI) return false;
+    long long jx = 0, jy = 0, jz = 0, gx = 0, gy = 0, gz = 0, sx = 0, sy = 0, sz = 0;
+    if constexpr (FMASK != 0) {
+        if (fm || fc) {
+            // a force of the populations' size lies outside the range
+            const unsigned long long big = (unsigned long long)(unsigned)(emax - 4) << 52;
+            if (fabs_bits(fx) >= big || fabs_bits(fy) >= big || fabs_bits(fz) >= big) return false;
+            if constexpr (FMASK & 1) gx = force_to_fixed(fx, emax);
+            if constexpr (FMASK & 2) gy = force_to_fixed(fy, emax);
+            if constexpr (FMASK & 4) gz = force_to_fixed(fz, emax);
+            if (fm) {
+                jx = (gx + 1) >> 1;
+                jy = (gy + 1) >> 1;
+                jz = (gz + 1) >> 1;
+            }
+        }
+    }
+    static_for<0, 9>([&](auto P) {
+        constexpr int l = pair_l(decltype(P)::value);
+        constexpr Vel c = vel(l);
+        const long long s = v[l] + v[inv(l)], d = v[l] - v[inv(l)];
+        v[l] = s;
+        v[inv(l)] = d;
+        if constexpr (c.x != 0) sx += c.x > 0 ? d : -d;
+        if constexpr (c.y != 0) sy += c.y > 0 ? d : -d;
+        if constexpr (c.z != 0) sz += c.z > 0 ? d : -d;
+    });
+    constexpr unsigned long long JR = 1ull << 57;   // no sum wraps: every |d| < R < 2^62, all n >= 0
+    if ((unsigned long long)(sx + (long long)JR) >= 2 * JR || (unsigned long long)(sy + (long long)JR) >= 2 * JR ||
+        (unsigned long long)(sz + (long long)JR) >= 2 * JR)
+        return false;
+    jx += 8 * sx;   // in eighths of a unit, |j| < 2^61
+    jy += 8 * sy;
+    jz += 8 * sz;
+    if constexpr (WANT_J) {
+        ox = signed_fixed(jx, emax);
+        oy = signed_fixed(jy, emax);
+        oz = signed_fixed(jz, emax);
+    }
+    // r = 2^121 / R: the reciprocal of R's 32 leading bits in FP32, then two Newton-Raphson steps
+    // r <- r + r (1 - R r), which double its 23 bits to 46 and to the product's 57
+    const float q = __frcp_rn((float)(unsigned)(R >> 30));
+    long long r = (long long)((unsigned long long)((__float_as_uint(q) & 0x7fffffu) | 0x800000u)
+                              << ((__float_as_uint(q) >> 23) - 59u));
+#pragma unroll
+    for (int k = 0; k < 2; ++k) r += mulhi(r, ((1ll << 57) - mulhi(R, r)) << 7);
+    const long long ux = mulhi(jx << 2, r), uy = mulhi(jy << 2, r), uz = mulhi(jz << 2, r);   // u 2^62
+    // c2 j / 8, c3 F / 4 and all that follows in eighths of a unit
+    const long long px = mulhi(jx, K.fix_c2), py = mulhi(jy, K.fix_c2), pz = mulhi(jz, K.fix_c2);
+    long long fqx = 0, fqy = 0, fqz = 0;
+    if constexpr (FMASK != 0) {
+        if (fc) {
+            if constexpr (FMASK & 1) fqx = mulhi(gx, K.fix_c3);
+            if constexpr (FMASK & 2) fqy = mulhi(gy, K.fix_c3);
+            if constexpr (FMASK & 4) fqz = mulhi(gz, K.fix_c3);
+        }
+    }
+    constexpr long long THIRD = 0x2aaaaaaaaaaaaaabll;   // 2^63 / 3
+    const long long hx = px + fqx, hy = py + fqy, hz = pz + fqz;
+    const long long bx = mulhi((2 * px + fqx) * 2, THIRD), by = mulhi((2 * py + fqy) * 2, THIRD),
+                    bz = mulhi((2 * pz + fqz) * 2, THIRD);
+    const long long qx = mulhi(ux, hx * 4), qy = mulhi(uy, hy * 4), qz = mulhi(uz, hz * 4);
+    const long long base = 2 * mulhi(R, K.fix_c2_36) - mulhi((qx + qy + qz) * 2, THIRD);
+    const long long base_axis = 2 * base;
+    long long rest = R - __mulhi((int)(R >> 31), K.fix_loss);
+    const bool relax = K.fix_c1 != 0;
+    // (s, d) of a pair in v[l], v[inv l] -> its collided populations; A, B to nearest, and half a
+    // unit more for the rounding down of the c1 products
+    const long long half = relax ? 8 : 4;
+    auto pair = [&](auto P, long long A, long long B) {
+        constexpr int l = pair_l(decltype(P)::value);
+        constexpr int li = inv(l);
+        long long e = (A + half) >> 3, o = (B + half) >> 3;
+        if (relax) {
+            e += mulhi(v[l] * 2, K.fix_c1);
+            o += mulhi(v[li] * 2, K.fix_c1);
+        }
+        rest -= 2 * e;
+        n[l] = fixed_to_double(e + o, emax);
+        n[li] = fixed_to_double(e - o, emax);
+    };
+    pair(std::integral_constant<int, 0>{}, base_axis + 2 * qx, 2 * bx);
+    pair(std::integral_constant<int, 1>{}, base_axis + 2 * qy, 2 * by);
+    pair(std::integral_constant<int, 2>{}, base_axis + 2 * qz, 2 * bz);
+    const long long mxy = mulhi(ux + uy, (hx + hy) * 4), mxz = mulhi(ux + uz, (hx + hz) * 4),
+                    myz = mulhi(uy + uz, (hy + hz) * 4);
+    pair(std::integral_constant<int, 3>{}, base + mxy, bx + by);                        // (1, 1, 0)
+    pair(std::integral_constant<int, 4>{}, base + 2 * (qx + qy) - mxy, by - bx);        // (-1, 1, 0)
+    pair(std::integral_constant<int, 5>{}, base + mxz, bx + bz);                        // (1, 0, 1)
+    pair(std::integral_constant<int, 6>{}, base + 2 * (qx + qz) - mxz, bz - bx);        // (-1, 0, 1)
+    pair(std::integral_constant<int, 7>{}, base + myz, by + bz);                        // (0, 1, 1)
+    pair(std::integral_constant<int, 8>{}, base + 2 * (qy + qz) - myz, bz - by);        // (0, -1, 1)
+    n[0] = fixed_to_double(rest, emax);
+    return true;
+}
+
+// One fused step of a node, in fixed point or, outside its range, in FP64.
+template <int FMASK, bool UCF, bool WANT_J>
+__device__ __forceinline__ void fused_step(double (&n)[Q], const bool fm, const bool fc, const double fx,
+                                           const double fy, const double fz, const FlowArgs64 &a, double &jx,
+                                           double &jy, double &jz)
+{
+    if (fused_fixed<FMASK, WANT_J>(n, fm, fc, fx, fy, fz, a, jx, jy, jz)) return;
+    double rho;
+    if (fm) moments19_pairs(n, fx / 2.0, fy / 2.0, fz / 2.0, rho, jx, jy, jz);
+    else moments19_pairs(n, 0.0, 0.0, 0.0, rho, jx, jy, jz);
+    if (fc) collide_node_fused<FMASK, UCF>(n, rho, jx, jy, jz, fx, fy, fz, a);
+    else collide_node_fused<0, true>(n, rho, jx, jy, jz, 0.0, 0.0, 0.0, a);
+}
+
 // density = SUM(n,4); j = F/2 + sum_l n_l c_l   (equilibration.f90:254,293-300)
 __device__ __forceinline__ void moments19(const double (&n)[Q], double fhx, double fhy,
                                           double fhz, double &rho, double &jx, double &jy,

@@ -1,5 +1,5 @@
 // flow_f64.cu -- FP64 D3Q19 kernels (compiled with -fmad=false): the strict form, and the fused
-// step of LBGPU_FP64_FUSED (explicit fused multiply-adds, collide_node_fused).
+// step of LBGPU_FP64_FUSED (64-bit fixed point, or explicit fused multiply-adds; flow64.cuh).
 //
 // Bit-exactness with the reference.  Every product and sum is evaluated in the operand order
 // of the Fortran source with separate roundings (no fused multiply-add in this translation
@@ -144,8 +144,10 @@ __global__ void __launch_bounds__(BLOCK) k_flow_step(const FlowArgs64 a)
                 fy = a.F[1];
                 fz = a.F[2];
             }
-            double rho, jx, jy, jz;
-            if constexpr (FUSED) {
+            double rho, jx = 0.0, jy = 0.0, jz = 0.0;
+            if constexpr (FUSED && !FIELD) {
+                fused_step<FMASK, true, CHECK>(n, fm != 0, fc != 0, fx, fy, fz, a, jx, jy, jz);
+            } else if constexpr (FUSED) {
                 if (fm) moments19_pairs(n, fx / 2.0, fy / 2.0, fz / 2.0, rho, jx, jy, jz);
                 else moments19_pairs(n, 0.0, 0.0, 0.0, rho, jx, jy, jz);
             } else {
@@ -159,10 +161,10 @@ __global__ void __launch_bounds__(BLOCK) k_flow_step(const FlowArgs64 a)
                 a.jy[node] = jy;
                 a.jz[node] = jz;
             }
-            if constexpr (FUSED) {
-                if (fc) collide_node_fused<FMASK, !FIELD>(n, rho, jx, jy, jz, fx, fy, fz, a);
+            if constexpr (FUSED && FIELD) {
+                if (fc) collide_node_fused<FMASK, false>(n, rho, jx, jy, jz, fx, fy, fz, a);
                 else collide_node_fused<0, true>(n, rho, jx, jy, jz, 0.0, 0.0, 0.0, a);
-            } else {
+            } else if constexpr (!FUSED) {
                 collide_strict<FMASK, !FIELD>(n, rho, jx, jy, jz, fx, fy, fz, a, fc != 0);
             }
 #pragma unroll

@@ -94,8 +94,8 @@ __global__ void __launch_bounds__(SPLIT ? 128 : RT, 1) k_flow64_resident(const R
 #pragma unroll
             for (int l = 0; l < Q; ++l) n[l] = __ldcg(src + off[l]);
             if (r.loop) bad = check19(n);
-            double rho, jx, jy, jz;
-            if constexpr (FUSED) moments19_pairs(n, fm ? fx / 2.0 : 0.0, fm ? fy / 2.0 : 0.0, fm ? fz / 2.0 : 0.0, rho, jx, jy, jz);
+            double rho, jx = 0.0, jy = 0.0, jz = 0.0;
+            if constexpr (FUSED) fused_step<FMASK, true, true>(n, fm, fc, fx, fy, fz, a, jx, jy, jz);
             else moments19(n, fm ? fx / 2.0 : 0.0, fm ? fy / 2.0 : 0.0, fm ? fz / 2.0 : 0.0, rho, jx, jy, jz);
             if (r.loop) {
                 const double e = max_nonneg(max_nonneg(fabs(jx - jold[0]), fabs(jy - jold[1])), fabs(jz - jold[2]));
@@ -104,12 +104,7 @@ __global__ void __launch_bounds__(SPLIT ? 128 : RT, 1) k_flow64_resident(const R
                 jold[1] = jy;
                 jold[2] = jz;
             }
-            if constexpr (FUSED) {
-                if (fc) collide_node_fused<FMASK, true>(n, rho, jx, jy, jz, fx, fy, fz, a);
-                else collide_node_fused<0, true>(n, rho, jx, jy, jz, 0.0, 0.0, 0.0, a);
-            } else {
-                collide_strict<FMASK, true>(n, rho, jx, jy, jz, fx, fy, fz, a, fc);
-            }
+            if constexpr (!FUSED) collide_strict<FMASK, true>(n, rho, jx, jy, jz, fx, fy, fz, a, fc);
 #pragma unroll
             for (int l = 0; l < Q; ++l) dst[(size_t)l * N + node] = n[l];
         } else {
