@@ -25,6 +25,7 @@
 #include "ctx.h"
 #include "fields.h"
 #include "flow.h"
+#include "host_pages.h"
 #include "lbgpu.h"
 #include "trace.h"
 
@@ -1043,8 +1044,15 @@ int lbgpu_batch_moments(lbgpu_batch *b, int id, double *rho, double *jx, double 
     LBB_CK(launch_batch_moments(b->d_insts, desc, batch_units(d), tmp, tmp + N, tmp + 2 * (size_t)N,
                                 tmp + 3 * (size_t)N, s));
     double *out[4] = {rho, jx, jy, jz};
-    for (int q = 0; q < 4; ++q)
-        LBB_CK(cudaMemcpyAsync(out[q], tmp + q * (size_t)N, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
+    const size_t bytes = sizeof(double) * N;
+    if (jx == rho + N && jy == jx + N && jz == jy + N) {   // one array (4, N): one copy
+        ready_pages({{rho, 4 * bytes}});
+        LBB_CK(cudaMemcpyAsync(rho, tmp, 4 * bytes, cudaMemcpyDeviceToHost, s));
+    } else {
+        ready_pages({{rho, bytes}, {jx, bytes}, {jy, bytes}, {jz, bytes}});
+        for (int q = 0; q < 4; ++q)
+            LBB_CK(cudaMemcpyAsync(out[q], tmp + q * (size_t)N, bytes, cudaMemcpyDeviceToHost, s));
+    }
     LBB_CK(cudaStreamSynchronize(s));
     return LBGPU_OK;
 }
@@ -1110,6 +1118,14 @@ int lbgpu_batch_mp_fields(lbgpu_batch *b, int id, double *P, double *P_ads)
     if (sl.d.phase != BATCH_MP) return bfail(LBGPU_ERR_INVALID, "lbgpu_batch_mp_fields: no tracer phase");
     const size_t N = (size_t)sl.d.N;
     double *outs[2] = {P, P_ads};
+    if (P && P_ads && sl.d.A[0] && N <= field_chunk_nodes((long long)N)) {
+        if (int rc = workspace(b, sizeof(double) * 6 * N)) return rc;
+        Field3 f[2] = {};
+        f[0].rec = sl.d.P[0];
+        f[1].rec = sl.d.A[0];
+        LBB_CK(fields_to_host(f[0], f[1], (long long)N, b->d_ws, P, P_ads, b->stream));
+        return LBGPU_OK;
+    }
     for (int q = 0; q < 2; ++q) {
         if (!outs[q]) continue;
         Field3 f{};

@@ -83,6 +83,9 @@ struct lbgpu_ctx {
     // many steps per launch (flow_f32_resident.cu) where the box is small enough (blocks > 0)
     lbg::ResidentPlan resident{}, resident_loop{};   // fixed steps, reference loop
     void *d_gsync = nullptr;
+    // per-step results of one call (l2err, VACF): kept up to HIST_KEPT bytes, see hist_take
+    double *d_hist = nullptr;
+    size_t hist_bytes = 0;
     bool resident_unchecked = false;   // a grid launch whose waits' outcome has not been read
     uint32_t *d_cpos = nullptr, *d_cmask = nullptr;
     uint2 *d_rowtab = nullptr;
@@ -117,6 +120,11 @@ void pnp_release(lbgpu_ctx *ctx);
 const double *pnp_potential(const lbgpu_ctx *ctx);
 // LBGPU_ERR_TIMEOUT if a wait of a resident launch since the last call ran out (waits for the stream)
 int resident_status(lbgpu_ctx *ctx);
+// A zeroed device array of n doubles for the per-step results of a call, and its return.  The
+// context keeps it between calls up to 1 MiB (cudaMallocAsync and cudaFreeAsync around every call
+// gave the memory back to the system at the next synchronisation: some 100 us a call).
+int hist_take(lbgpu_ctx *ctx, size_t n, double **p);
+void hist_return(lbgpu_ctx *ctx, double *p);
 // The device address of the host range [p, p + bytes) if it lies inside one range page-locked by
 // lbgpu_host_register (kernels may then read it in place), else null.
 const void *pinned_device_view(const void *p, size_t bytes);

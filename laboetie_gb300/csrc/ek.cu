@@ -328,8 +328,7 @@ int need_charges(lbgpu_ctx *ctx, const char *fn)
 int alloc_zero(lbgpu_ctx *ctx, double **p, size_t n)
 {
     if (*p) return LBGPU_OK;
-    LBG_CK(ctx, cudaMalloc((void **)p, n * sizeof(double)));
-    ctx->pnp->allocs.push_back(*p);
+    LBG_CK(ctx, ctx->pnp->allocs.get((void **)p, n * sizeof(double)));
     LBG_CK(ctx, cudaMemsetAsync(*p, 0, n * sizeof(double), ctx->stream));
     return LBGPU_OK;
 }

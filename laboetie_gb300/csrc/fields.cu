@@ -4,6 +4,7 @@
 // P of a 160^3 box took 20 ms, against 6 ms for the transfer into fresh pages.
 #include "common.cuh"
 #include "fields.h"
+#include "host_pages.h"
 
 namespace lbg {
 namespace {
@@ -50,14 +51,40 @@ unsigned blocks(size_t n) { return (unsigned)((n + BLOCK - 1) / BLOCK); }
 
 size_t field_chunk_nodes(long long N) { return (size_t)(N < (1ll << 22) ? N : (1ll << 22)); }
 
+namespace {
+cudaError_t pack(const Field3 &f, size_t at, unsigned n, double *stage, cudaStream_t s)
+{
+    if (f.rec) k_pack32<<<blocks(3 * (size_t)n), BLOCK, 0, s>>>(f.rec + at, stage, n);
+    else k_pack64<<<blocks(3 * (size_t)n), BLOCK, 0, s>>>(f.comp[0] + at, f.comp[1] + at, f.comp[2] + at, stage, n);
+    return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t fields_to_host(const Field3 &a, const Field3 &b, long long N, double *stage, double *host_a, double *host_b,
+                           cudaStream_t s)
+{
+    const size_t doubles = 3 * (size_t)N, bytes = sizeof(double) * doubles;
+    cudaError_t e = pack(a, 0, (unsigned)N, stage, s);
+    if (e == cudaSuccess) e = pack(b, 0, (unsigned)N, stage + doubles, s);
+    if (e != cudaSuccess) return e;
+    if (host_b == host_a + doubles) {   // one array: one copy
+        ready_pages({{host_a, 2 * bytes}});
+        e = cudaMemcpyAsync(host_a, stage, 2 * bytes, cudaMemcpyDeviceToHost, s);
+    } else {
+        ready_pages({{host_a, bytes}, {host_b, bytes}});
+        e = cudaMemcpyAsync(host_a, stage, bytes, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(host_b, stage + doubles, bytes, cudaMemcpyDeviceToHost, s);
+    }
+    return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+}
+
 cudaError_t field_to_host(const Field3 &f, long long N, double *stage, double *host, cudaStream_t s)
 {
     const size_t chunk = field_chunk_nodes(N);
     for (size_t at = 0; at < (size_t)N; at += chunk) {
         const unsigned n = (unsigned)((size_t)N - at < chunk ? (size_t)N - at : chunk);
-        if (f.rec) k_pack32<<<blocks(3 * (size_t)n), BLOCK, 0, s>>>(f.rec + at, stage, n);
-        else k_pack64<<<blocks(3 * (size_t)n), BLOCK, 0, s>>>(f.comp[0] + at, f.comp[1] + at, f.comp[2] + at, stage, n);
-        cudaError_t e = cudaGetLastError();
+        cudaError_t e = pack(f, at, n, stage, s);
+        ready_pages({{host + 3 * at, sizeof(double) * 3 * n}});
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(host + 3 * at, stage, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) return e;

@@ -17,6 +17,9 @@ struct Field3 {
 size_t field_chunk_nodes(long long N);
 // host[3 i + d] = component d of node i (and back), waiting for the stream
 cudaError_t field_to_host(const Field3 &f, long long N, double *stage, double *host, cudaStream_t s);
+// both fields of a box of one chunk at once (a: host_a, b: host_b), with 6 doubles of stage per node
+cudaError_t fields_to_host(const Field3 &a, const Field3 &b, long long N, double *stage, double *host_a, double *host_b,
+                           cudaStream_t s);
 cudaError_t field_from_host(const Field3 &f, long long N, double *stage, const double *host, cudaStream_t s);
 
 }  // namespace lbg

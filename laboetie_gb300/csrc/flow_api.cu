@@ -13,6 +13,7 @@
 #include "compact.cuh"
 #include "ctx.h"
 #include "flow.h"
+#include "host_pages.h"
 #include "lbgpu.h"
 #include "trace.h"
 
@@ -188,6 +189,32 @@ int ctx_init_device(lbgpu_ctx *ctx, const int8_t *nature)
 }
 
 
+int hist_take(lbgpu_ctx *ctx, size_t n, double **p)
+{
+    constexpr size_t HIST_KEPT = 1u << 20;
+    const size_t bytes = sizeof(double) * n;
+    cudaStream_t s = ctx->stream;
+    if (bytes > HIST_KEPT) {
+        LBG_CK(ctx, cudaMallocAsync((void **)p, bytes, s));
+    } else {
+        if (bytes > ctx->hist_bytes) {
+            if (ctx->d_hist) LBG_CK(ctx, cudaFreeAsync(ctx->d_hist, s));
+            ctx->d_hist = nullptr;
+            ctx->hist_bytes = 0;
+            LBG_CK(ctx, cudaMallocAsync((void **)&ctx->d_hist, bytes, s));
+            ctx->hist_bytes = bytes;
+        }
+        *p = ctx->d_hist;
+    }
+    LBG_CK(ctx, cudaMemsetAsync(*p, 0, bytes, s));
+    return LBGPU_OK;
+}
+
+void hist_return(lbgpu_ctx *ctx, double *p)
+{
+    if (p && p != ctx->d_hist) cudaFreeAsync(p, ctx->stream);
+}
+
 void ctx_release_device(lbgpu_ctx *ctx)
 {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
@@ -204,6 +231,7 @@ void ctx_release_device(lbgpu_ctx *ctx)
     cudaFree(ctx->d_cmask);
     cudaFree(ctx->d_rowtab);
     cudaFree(ctx->d_gsync);
+    if (ctx->d_hist) cudaFree(ctx->d_hist);
     for (int b = 0; b < 2; ++b) {
         cudaFree(ctx->d_f[b]);
         cudaFree(ctx->d_g[b]);
@@ -355,6 +383,8 @@ int lbgpu_flow_get(lbgpu_ctx *ctx, double *n, double *density, double *jx, doubl
         a.Fz = ctx->d_F[2];
         LBG_CK(ctx, launch_finalize_f64(a, field, s));
     }
+    const size_t bytes = sizeof(double) * N;
+    ready_pages({{n, Q * bytes}, {density, bytes}, {jx, bytes}, {jy, bytes}, {jz, bytes}});
     if (n) LBG_CK(ctx, cudaMemcpyAsync(n, nsrc, sizeof(double) * Q * N, cudaMemcpyDeviceToHost, s));
     if (density) LBG_CK(ctx, cudaMemcpyAsync(density, ctx->d_rho, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
     double *j[3] = {jx, jy, jz};
@@ -452,6 +482,7 @@ int lbgpu_moments(lbgpu_ctx *ctx, const double *n, const double *f_ext_x, const 
     a.Fz = ob->F[2];
     LBG_CK(ctx, launch_moments_f64(a, true, s));
     double *out[4] = {density, jx, jy, jz};
+    ready_pages({{density, sizeof(double) * N}, {jx, sizeof(double) * N}, {jy, sizeof(double) * N}, {jz, sizeof(double) * N}});
     for (int q = 0; q < 4; ++q)
         LBG_CK(ctx, cudaMemcpyAsync(out[q], ob->m[q], sizeof(double) * N, cudaMemcpyDeviceToHost, s));
     Scratch sc;
@@ -477,8 +508,8 @@ int lbgpu_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int h
     cudaStream_t s = ctx->stream;
     double *d_hist = nullptr;
     if (hist_cap > 0) {
-        LBG_CK(ctx, cudaMallocAsync(&d_hist, sizeof(double) * hist_cap, s));
-        LBG_CK(ctx, cudaMemsetAsync(d_hist, 0, sizeof(double) * hist_cap, s));
+        if (int rc = hist_take(ctx, (size_t)hist_cap, &d_hist)) return rc;
+        ready_pages({{l2err_hist, sizeof(double) * hist_cap}});
     }
     FlowCtl c;
     std::memset(&c, 0, sizeof(c));
@@ -537,7 +568,7 @@ int lbgpu_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int h
     if (rc) return rc;
     if (h.status & LBGPU_ERR_TIMEOUT) {
         LBG_CK(ctx, cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(h.status), s));
-        if (d_hist) cudaFreeAsync(d_hist, s);
+        hist_return(ctx, d_hist);
         return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, "equilibration: a block did not reach the grid's barrier within its wait limit");
     }
     ctx->cur = h.parity;
@@ -548,7 +579,7 @@ int lbgpu_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int h
     if (steps_out) *steps_out = h.exit_step;
     if (d_hist) {
         LBG_CK(ctx, cudaMemcpyAsync(l2err_hist, d_hist, sizeof(double) * hist_cap, cudaMemcpyDeviceToHost, s));
-        LBG_CK(ctx, cudaFreeAsync(d_hist, s));
+        hist_return(ctx, d_hist);
     }
     LBG_CK(ctx, cudaStreamSynchronize(s));
     if (h.status & LBGPU_ERR_NEGATIVE_POPULATION)

@@ -8,6 +8,7 @@
 
 #include "ctx.h"
 #include "flow.h"
+#include "host_pages.h"
 #include "lbgpu.h"
 
 namespace lbg {
@@ -171,6 +172,8 @@ int f32_flow_get(lbgpu_ctx *ctx, double *n, double *density, double *jx, double 
         LBG_CK(ctx, launch_aa_finalize_f32(a, ctx->aa_phase == 1, s));
     }
     else LBG_CK(ctx, launch_finalize_f32(a, ctx->prev_kind == PREV_POST, s));
+    const size_t bytes = sizeof(double) * N;
+    ready_pages({{n, Q * bytes}, {density, bytes}, {jx, bytes}, {jy, bytes}, {jz, bytes}});
     if (n) LBG_CK(ctx, cudaMemcpyAsync(n, tmp, sizeof(double) * Q * N, cudaMemcpyDeviceToHost, s));
     if (density) LBG_CK(ctx, cudaMemcpyAsync(density, ctx->d_rho, sizeof(double) * N, cudaMemcpyDeviceToHost, s));
     double *j[3] = {jx, jy, jz};
@@ -332,8 +335,8 @@ int f32_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int his
     cudaStream_t s = ctx->stream;
     double *d_hist = nullptr;
     if (hist_cap > 0) {
-        LBG_CK(ctx, cudaMallocAsync(&d_hist, sizeof(double) * hist_cap, s));
-        LBG_CK(ctx, cudaMemsetAsync(d_hist, 0, sizeof(double) * hist_cap, s));
+        if ((rc = hist_take(ctx, (size_t)hist_cap, &d_hist))) return rc;
+        ready_pages({{l2err_hist, sizeof(double) * hist_cap}});
     }
     FlowCtl c;
     std::memset(&c, 0, sizeof(c));
@@ -396,7 +399,7 @@ int f32_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int his
     if (rc) return rc;
     if (h.status & LBGPU_ERR_TIMEOUT) {
         LBG_CK(ctx, cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(h.status), s));
-        if (d_hist) cudaFreeAsync(d_hist, s);
+        hist_return(ctx, d_hist);
         return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, "equilibration: a block did not reach the grid's barrier within its wait limit");
     }
     ctx->aa_phase = h.exit_phase;
@@ -406,7 +409,7 @@ int f32_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int his
     if (steps_out) *steps_out = h.exit_step;
     if (d_hist) {
         LBG_CK(ctx, cudaMemcpyAsync(l2err_hist, d_hist, sizeof(double) * hist_cap, cudaMemcpyDeviceToHost, s));
-        LBG_CK(ctx, cudaFreeAsync(d_hist, s));
+        hist_return(ctx, d_hist);
     }
     LBG_CK(ctx, cudaStreamSynchronize(s));
     if (h.status & LBGPU_ERR_NEGATIVE_POPULATION)

@@ -12,6 +12,8 @@
 #include "ctx.h"
 #include "fields.h"
 #include "flow.h"
+#include "host_pages.h"
+#include "kept_allocs.h"
 #include "lbgpu.h"
 #include "trace.h"
 #include "mp.h"
@@ -28,7 +30,7 @@ struct MpState {
     double K = 0, lambda = 0, bw = 0;
     MpArgs64 a64{};
     MpArgs32 a32{};
-    std::vector<void *> allocs;
+    KeptAllocs allocs;
     MpResident res{};             // many steps per launch (mp_resident.cu) where the box is small
     double *res_vacf = nullptr;   // VACF of one launch's steps
     double *stage = nullptr;      // staging of lbgpu_mp_get / _set, at most 96 MiB
@@ -43,7 +45,7 @@ void mp_release(lbgpu_ctx *ctx)
 {
     if (!ctx->mp) return;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    for (void *p : ctx->mp->allocs) cudaFree(p);
+    ctx->mp->allocs.free_all();
     delete ctx->mp;
     ctx->mp = nullptr;
 }
@@ -53,8 +55,7 @@ namespace {
 template <typename T>
 int alloc_zero(lbgpu_ctx *ctx, MpState *s, T **p, size_t count)
 {
-    LBG_CK(ctx, cudaMalloc((void **)p, count * sizeof(T)));
-    s->allocs.push_back(*p);
+    LBG_CK(ctx, s->allocs.get((void **)p, count * sizeof(T)));
     LBG_CK(ctx, cudaMemsetAsync(*p, 0, count * sizeof(T), ctx->stream));
     return LBGPU_OK;
 }
@@ -64,8 +65,7 @@ constexpr double EPS = 2.220446049250313e-16;  // epsilon(1._dp)
 int stage_init(lbgpu_ctx *ctx, MpState *s)
 {
     if (s->stage) return LBGPU_OK;
-    LBG_CK(ctx, cudaMalloc((void **)&s->stage, sizeof(double) * 3 * field_chunk_nodes(ctx->N)));
-    s->allocs.push_back(s->stage);
+    LBG_CK(ctx, s->allocs.get((void **)&s->stage, sizeof(double) * 3 * field_chunk_nodes(ctx->N)));
     return LBGPU_OK;
 }
 
@@ -198,9 +198,14 @@ int mp_init_impl(lbgpu_ctx *ctx, const lbgpu_tracer *tr, const double *density, 
             if ((msk[r] & FLUID_BIT) && (msk[r] & INTERFACIAL_BIT)) s2 = s2 + std::exp(-(tr->z * phi[r])) * K;
         Pstat = s1 + s2;
     }
-    mp_release(ctx);
     MpState *s = new MpState();
+    KeptAllocs::SpareGuard guard{s->allocs};
+    const bool had_stage = ctx->mp && ctx->mp->stage;
+    if (ctx->mp) s->allocs.take(ctx->mp->allocs);
+    mp_release(ctx);
     ctx->mp = s;
+    if (had_stage)
+        if (int rc = stage_init(ctx, s)) return rc;
     // the fused FP64 mode runs the FP64 tracer with fused gathers (a64.fused)
     s->prec = ctx->p.precision == LBGPU_FP32_DEV ? LBGPU_FP32_DEV : LBGPU_FP64;
     s->tr = *tr;
@@ -452,7 +457,10 @@ static int mp_run(lbgpu_ctx *ctx, int nsteps, double *vacf_out, int *steps_done,
     }
     LBG_CK(ctx, cudaMemcpyAsync(s->a64.ctl, &c, sizeof(c), cudaMemcpyHostToDevice, st));
     double *hist = nullptr;
-    if (!timing) LBG_CK(ctx, cudaMallocAsync(&hist, sizeof(double) * 3 * (size_t)nsteps, st));
+    if (!timing) {
+        if (int rc = hist_take(ctx, 3 * (size_t)nsteps, &hist)) return rc;
+        ready_pages({{vacf_out, sizeof(double) * 3 * (size_t)nsteps}});
+    }
     s->a64.hist = hist;
     s->a32.hist = hist;
     const int G = std::min(nsteps, 256);
@@ -502,7 +510,7 @@ static int mp_run(lbgpu_ctx *ctx, int nsteps, double *vacf_out, int *steps_done,
         if (vacf_out && done > 0)
             LBG_CK(ctx, cudaMemcpyAsync(vacf_out, hist, sizeof(double) * 3 * (size_t)done,
                                         cudaMemcpyDeviceToHost, st));
-        LBG_CK(ctx, cudaFreeAsync(hist, st));
+        hist_return(ctx, hist);
         LBG_CK(ctx, cudaStreamSynchronize(st));
     }
     s->a64.hist = s->a32.hist = nullptr;

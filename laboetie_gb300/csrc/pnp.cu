@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "ctx.h"
+#include "host_pages.h"
 #include "lbgpu.h"
 #include "trace.h"
 #include "pnp.h"
@@ -55,7 +56,7 @@ void pnp_release(lbgpu_ctx *ctx)
     if (ps->anorm_ev) cudaEventDestroy(ps->anorm_ev);
     for (cudaGraphExec_t g : ctx->pnp->sor_exec)
         if (g) cudaGraphExecDestroy(g);
-    for (void *p : ctx->pnp->allocs) cudaFree(p);
+    ctx->pnp->allocs.free_all();
     if (ctx->pnp->phi_host) cudaFreeHost(ctx->pnp->phi_host);
     delete ctx->pnp;
     ctx->pnp = nullptr;
@@ -581,15 +582,16 @@ int lbgpu_pnp_init(lbgpu_ctx *ctx, const lbgpu_pnp_params *p, double *anormf0)
     if (p->solver != LBGPU_POISSON_REFERENCE && p->solver != LBGPU_POISSON_SOR4 &&
         p->solver != LBGPU_POISSON_JACOBI)
         return ctx_fail(ctx, LBGPU_ERR_INVALID, "lbgpu_pnp_init: unknown solver");
-    pnp_release(ctx);
     PnpState *s = new PnpState();
+    KeptAllocs::SpareGuard guard{s->allocs};
+    if (ctx->pnp) s->allocs.take(ctx->pnp->allocs);
+    pnp_release(ctx);
     ctx->pnp = s;
     s->p = *p;
     const long long N = ctx->N;
     cudaStream_t st = ctx->stream;
     auto alloc = [&](double **q, size_t n) -> int {
-        LBG_CK(ctx, cudaMalloc((void **)q, n * sizeof(double)));
-        s->allocs.push_back(*q);
+        LBG_CK(ctx, s->allocs.get((void **)q, n * sizeof(double)));
         LBG_CK(ctx, cudaMemsetAsync(*q, 0, n * sizeof(double), st));
         return LBGPU_OK;
     };
@@ -617,8 +619,7 @@ int lbgpu_pnp_init(lbgpu_ctx *ctx, const lbgpu_pnp_params *p, double *anormf0)
     }
     // partials: 4 per block, twice (two reductions read back together); results: 4, twice
     if ((rc = alloc(&s->partial, 8 * (size_t)MP_MAX_BLOCKS)) || (rc = alloc(&s->result, 8))) return rc;
-    LBG_CK(ctx, cudaMalloc((void **)&s->ctl, sizeof(PnpCtl)));
-    s->allocs.push_back(s->ctl);
+    LBG_CK(ctx, s->allocs.get((void **)&s->ctl, sizeof(PnpCtl)));
     LBG_CK(ctx, cudaMemsetAsync(s->ctl, 0, sizeof(PnpCtl), st));
 
     // charges_init.f90:23-135 on the host, node by node in the reference's order
@@ -691,6 +692,7 @@ int lbgpu_pnp_get(lbgpu_ctx *ctx, double *c_plus, double *c_minus, double *phi, 
     if (rc) return rc;
     PnpState *s = ctx->pnp;
     const size_t b = sizeof(double) * ctx->N;
+    ready_pages({{c_plus, b}, {c_minus, b}, {phi, b}});
     if (c_plus) LBG_CK(ctx, cudaMemcpyAsync(c_plus, s->cp, b, cudaMemcpyDeviceToHost, ctx->stream));
     if (c_minus) LBG_CK(ctx, cudaMemcpyAsync(c_minus, s->cm, b, cudaMemcpyDeviceToHost, ctx->stream));
     if (phi) LBG_CK(ctx, cudaMemcpyAsync(phi, s->phi[s->par], b, cudaMemcpyDeviceToHost, ctx->stream));

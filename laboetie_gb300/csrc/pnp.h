@@ -11,6 +11,7 @@
 #include <thread>
 #include <vector>
 
+#include "kept_allocs.h"
 #include "lbgpu.h"
 
 namespace lbg {
@@ -47,7 +48,7 @@ struct PnpState {
     int par = 0;                            // buffer holding phi
     double anormf0 = 0.0, rho_ch = 0.0;
     bool charged = false;
-    std::vector<void *> allocs;
+    KeptAllocs allocs;
     PnpResidentPlan resident{};             // with its own buffers:
     GridSync *gsync = nullptr;
     PnpLoop *loop = nullptr;

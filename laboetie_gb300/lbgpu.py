@@ -705,8 +705,7 @@ class Batch:
         return ms.value
 
     def moments(self, box: int):
-        shape = self._shapes[box]
-        out = [np.empty(shape) for _ in range(4)]
+        out = np.empty((4,) + self._shapes[box])   # one array: one copy from the device
         self._chk(self.L.lbgpu_batch_moments(self.b, box, *(_ptr(x) for x in out)), "batch_moments")
         return out[0], tuple(out[1:])
 
@@ -723,8 +722,7 @@ class Batch:
 
     def mp_fields(self, box: int):
         """(P, P_ads) of a box in its tracer phase, shape (lz, ly, lx, 3), as Box.mp_get."""
-        shape = self._shapes[box] + (3,)
-        P, A = np.empty(shape), np.empty(shape)
+        P, A = np.empty((2,) + self._shapes[box] + (3,))   # one array: one copy from the device
         self._chk(self.L.lbgpu_batch_mp_fields(self.b, box, _ptr(P), _ptr(A)), "batch_mp_fields")
         return P, A
 
