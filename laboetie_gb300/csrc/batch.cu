@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(BATCH_BLOCK, 6) k_batch_mp(const BatchInst *__
 
 // One tracer step of the slab tiles of boxes in the tracer phase (mp_slab.cuh); each tile keeps
 // its own running sums.
-__global__ void __launch_bounds__(BATCH_BLOCK, 4) k_batch_mp_slab(const BatchInst *__restrict__ insts,
+__global__ void __launch_bounds__(MPS_THREADS, 4) k_batch_mp_slab(const BatchInst *__restrict__ insts,
                                                                const BatchTile *__restrict__ tiles, int par)
 {
     extern __shared__ float4 sm4[];
@@ -563,10 +563,9 @@ __global__ void __launch_bounds__(BATCH_BLOCK, 4) k_batch_mp_slab(const BatchIns
     const int nxy = tiles_x * tiles_y;
     const int tile = t.start % nxy, chunk = t.start / nxy;
     const int z0 = chunk * I.zc;
-    float vt[3] = {0.0f, 0.0f, 0.0f};
+    double v[3];
     mp_slab_planes(I, par, (tile % tiles_x) * MPS_TX, (tile / tiles_x) * MPS_TY, z0, min(z0 + I.zc, I.lz), sm4,
-                   vt, nullptr, nullptr, nullptr);
-    double v[3] = {(double)vt[0], (double)vt[1], (double)vt[2]};
+                   v, nullptr, nullptr, nullptr);
     block_sum3(v);
     if (threadIdx.x == 0) {
         double *acc = I.tacc + (size_t)t.start * BATCH_TACC;
@@ -801,7 +800,7 @@ cudaError_t launch_batch_mp_slab(const BatchInst *insts, const BatchTile *tiles,
                                  cudaStream_t s)
 {
     if (ntiles <= 0) return cudaSuccess;
-    k_batch_mp_slab<<<ntiles, BATCH_BLOCK, MPS_SMEM, s>>>(insts, tiles, par);
+    k_batch_mp_slab<<<ntiles, MPS_THREADS, MPS_SMEM, s>>>(insts, tiles, par);
     return cudaGetLastError();
 }
 

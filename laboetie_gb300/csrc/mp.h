@@ -95,7 +95,9 @@ struct MpArgs32 {
 // Shared-memory slab variant of the FP32 step (mp_f32.cu): 32 x 8 column tiles sweeping a chunk
 // of z planes.  Used when lx >= 32, ly >= 8 and lz >= 3.  Returns the grid (0: not eligible) and
 // the planes per block in *zc.  A chunk reads two planes beyond its own, so the chunks are as long
-// as filling the device once allows (resident: blocks resident at once), and at least 8 planes.
+// as filling the device once allows (resident: blocks resident at once), and at least 4 planes: a
+// plane costs a block of a half-empty device about 1 us whatever the box (64^3 porous: 17.0 us a step
+// with at least 8 planes, 16.3 with 6, 15.7 with 4 or 3, 17.4 with 2; 96^3: 26.2, 25.4, 25.4).
 // resident 0 (the step's shared memory could not be granted): not eligible.
 constexpr int MPS_TX = 32, MPS_TY = 8;
 inline unsigned mp32_slab_grid(int lx, int ly, int lz, unsigned resident, int *zc)
@@ -103,7 +105,7 @@ inline unsigned mp32_slab_grid(int lx, int ly, int lz, unsigned resident, int *z
     if (lx < MPS_TX || ly < MPS_TY || lz < 3 || resident == 0) return 0;
     const int nxy = ((lx + MPS_TX - 1) / MPS_TX) * ((ly + MPS_TY - 1) / MPS_TY);
     int nz = (int)(resident / (unsigned)nxy);
-    if (nz > lz / 8) nz = lz / 8;
+    if (nz > lz / 4) nz = lz / 4;
     if (nz < 1) nz = 1;
     const int c = (lz + nz - 1) / nz;
     *zc = c;

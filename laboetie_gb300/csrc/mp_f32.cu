@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(MP_BLOCK) k_mp32(const MpArgs32 a, float bw)
 // One tracer step of a box with V and P staged in shared memory (mp_slab.cuh): a block owns a
 // 32 x 8 column tile and a chunk of zc planes.  With use_tma, interior tiles stage their planes
 // by bulk tensor copies through the tensor maps of V and P[0], P[1] (kernel parameters).
-__global__ void __launch_bounds__(MP_BLOCK, 4)
+__global__ void __launch_bounds__(MPS_THREADS, 4)
     k_mp32_slab(const MpArgs32 a, int tiles_x, int tiles_y, int zc, const __grid_constant__ CUtensorMap tmV,
                 const __grid_constant__ CUtensorMap tmP0, const __grid_constant__ CUtensorMap tmP1, int use_tma)
 {
@@ -183,10 +183,9 @@ __global__ void __launch_bounds__(MP_BLOCK, 4)
     const int nxy = tiles_x * tiles_y;
     const int tile = (int)blockIdx.x % nxy, chunk = (int)blockIdx.x / nxy;
     const int z0 = chunk * zc;
-    float vt[3] = {0.0f, 0.0f, 0.0f};
-    mp_slab_planes(a, par, (tile % tiles_x) * MPS_TX, (tile / tiles_x) * MPS_TY, z0, min(z0 + zc, a.lz), sm4, vt,
+    double v[3];
+    mp_slab_planes(a, par, (tile % tiles_x) * MPS_TX, (tile / tiles_x) * MPS_TY, z0, min(z0 + zc, a.lz), sm4, v,
                    use_tma ? &tmV : nullptr, use_tma ? (par ? &tmP1 : &tmP0) : nullptr, &a.ctl->status);
-    double v[3] = {(double)vt[0], (double)vt[1], (double)vt[2]};
     grid_sum3<false>(v, a.partial, &a.ctl->blocks_done,
               [&](const double (&tot)[3]) { mp_control(a.ctl, a.hist, tot); });
 }
@@ -251,7 +250,7 @@ unsigned mp32_slab_resident()
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaFuncSetAttribute(k_mp32_slab, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MPS_SMEM) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mp32_slab, MP_BLOCK, MPS_SMEM) != cudaSuccess) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mp32_slab, MPS_THREADS, MPS_SMEM) != cudaSuccess) {
         cudaGetLastError();
         return 0u;
     }
@@ -266,7 +265,7 @@ cudaError_t launch_mp_step_f32(const MpArgs32 &a, unsigned grid, const CUtensorM
         const int tx = (a.lx + MPS_TX - 1) / MPS_TX, ty = (a.ly + MPS_TY - 1) / MPS_TY;
         CUtensorMap none;
         std::memset(&none, 0, sizeof(none));
-        k_mp32_slab<<<sg, MP_BLOCK, MPS_SMEM, s>>>(a, tx, ty, zc, tm ? tm[0] : none, tm ? tm[1] : none,
+        k_mp32_slab<<<sg, MPS_THREADS, MPS_SMEM, s>>>(a, tx, ty, zc, tm ? tm[0] : none, tm ? tm[1] : none,
                                                    tm ? tm[2] : none, tm ? 1 : 0);
     } else {
         if (a.charged) k_mp32<false, true><<<grid, MP_BLOCK, 0, s>>>(a, 0.0f);

@@ -6,7 +6,15 @@
 // V and P value is fetched from L2/HBM about 1.3 times (halo) per step; the column's flag words
 // (and the node's fixed (u*, D)) are loaded into registers ahead of use, and an interfacial
 // node's adsorbed part is copied into a slot of the thread's own two steps before it finishes.
-// One block barrier per plane.  mp_slab_planes is the difference form of mp_f32.cu:k_mp32 (same operations in the same
+// One block barrier per plane.  A thread steps two columns, neighbours in y: half of their
+// neighbourhoods' points are common (24 shared-memory reads of V and P a plane instead of 36), and
+// barrier, ring and addresses are paid once for both.
+// 160^3 porous medium, 2.46 M fluid nodes, adsorbing: one column a thread and addresses formed for
+// each copied record 75.3 us a step (441 instructions a node, 66 % of the issue slots), addresses
+// kept 72.3, two columns 69.9 (324).  What is left is memory: 0.45 GB from L2 (27 % of it halo),
+// 0.29 GB from HBM, 52 % of its rate, behind a barrier every plane; a third fewer instructions per
+// column changed little, a ring of 3 planes (5 blocks an SM instead of 4) took 128 us.
+// mp_slab_planes is the difference form of mp_f32.cu:k_mp32 (same operations in the same
 // order, so P is bit-identical) visiting each plane once, for single boxes and batched ones alike.
 // The argument struct provides V (its w component: the node's fluid flag, 1 or 0), P[2], A[2],
 // aux, mask, lx, ly, lz, ads, ka, kd, one_minus_kd, a1[3], lwh[3], wait_ns, skip_copies.
@@ -27,9 +35,11 @@ constexpr int SHX = MPS_TX + 2, SHY = MPS_TY + 2, SPL = SHX * SHY;  // a plane w
 // 128-byte boundary)
 constexpr int SPLP = (SPL * 16 + 127) / 128 * 8;
 constexpr unsigned MPS_TMA_BYTES = SPL * 16;                        // one plane of V or of P
-// 4 planes of V and of P, 4 mbarriers, two adsorbed-part slots per thread, and slack to align the
+// nodes of a plane that a thread steps (neighbours in y), and the threads of a block
+constexpr int MPS_ROWS = 2, MPS_THREADS = MPS_TX * MPS_TY / MPS_ROWS;
+// 4 planes of V and of P, 4 mbarriers, two adsorbed-part slots per column, and slack to align the
 // ring to 128 bytes
-constexpr size_t MPS_SMEM = 128 + sizeof(float4) * 8 * SPLP + 4 * sizeof(uint64_t) + 2 * MP_BLOCK * sizeof(float4);
+constexpr size_t MPS_SMEM = 128 + sizeof(float4) * 8 * SPLP + 4 * sizeof(uint64_t) + 2 * MPS_TX * MPS_TY * sizeof(float4);
 
 // Scattering probability of a link, a1 (c.V) + lambda w / 2 rounded once, or 0 across a
 // bounce-back link (blocked).  The reference multiplies by a 0/1 factor instead; the sums it
@@ -136,13 +146,29 @@ __host__ __device__ constexpr bool plane_order_is_link_order()
 }
 static_assert(plane_order_is_link_order(), "plane-wise visit order differs from mp_link_order");
 
+// Whether visit k of column q is the first to read its point (dx, j = dy + q) of the neighbourhood:
+// the columns of a thread visit their nine points in step, and a point they share is read once.
+__host__ __device__ constexpr bool slab_visits(int k, bool da, bool db, bool dc)
+{
+    const bool axis = pt_dx(k) * pt_dx(k) + pt_dy(k) * pt_dy(k) <= 1;
+    return ((dc || da) && axis) || (db && (pt_dx(k) != 0 || pt_dy(k) != 0));
+}
+__host__ __device__ constexpr bool slab_first_use(int k, int q, bool da, bool db, bool dc)
+{
+    for (int k2 = 0; k2 <= k; ++k2)
+        for (int q2 = 0; q2 < MPS_ROWS; ++q2) {
+            if (k2 == k && q2 >= q) break;
+            if (slab_visits(k2, da, db, dc) && pt_dx(k2) == pt_dx(k) && pt_dy(k2) + q2 == pt_dy(k) + q) return false;
+        }
+    return true;
+}
+
 // Difference-form sweep of one tile (a box's FP32 step, mp_f32.cu:k_mp32's arithmetic in
 // mp_link_order): P(par) -> P(par^1) (and A) for its fluid nodes, P(r) + [sum_l sp_in(l)
 // (P(r+c_l) - P(r)) + D P(r)] with the node's fixed (u*, D) from a.aux; vt += the VACF terms.
 //
 // Plane-wise: each plane zz = z0-1 .. z1 is read once.  A thread reads the nine points
-// (x+dx, y+dy, zz) of its column's neighbourhood (V and P: 18 shared-memory reads instead of the
-// 37 a node-wise step makes) and adds each point's incoming links to the nodes of its column that
+// (x+dx, y+dy, zz) of each column's neighbourhood (V and P) and adds each point's incoming links to the nodes of its column that
 // they reach: (dx, dy, -1) to node zz+1, (dx, dy, 0) to node zz, (dx, dy, +1) to node zz-1.  The
 // three nodes in flight keep their sums, P and flag words in registers; node zz-1 is complete
 // after plane zz and is written.  Ring of 4 plane slots: at step zz plane zz+1 has arrived (its
@@ -154,7 +180,7 @@ static_assert(plane_order_is_link_order(), "plane-wise visit order differs from 
 // runs out of its bound sets LBGPU_ERR_TIMEOUT in *status and the tile's nodes are left alone.
 template <typename Args>
 __device__ __forceinline__ void mp_slab_planes(const Args &a, int par, int x0, int y0, int z0, int z1,
-                                               float4 *sm_raw, float (&vt)[3], const CUtensorMap *tmV,
+                                               float4 *sm_raw, double (&vacf)[3], const CUtensorMap *tmV,
                                                const CUtensorMap *tmP, unsigned *status)
 {
     // align the ring to 128 bytes by offsetting the shared-memory pointer itself (rounding its
@@ -163,7 +189,8 @@ __device__ __forceinline__ void mp_slab_planes(const Args &a, int par, int x0, i
     float4 *sm = sm_raw + ((128u - (smem_addr(sm_raw) & 127u)) & 127u) / 16u;
     float4 *sV = sm, *sP = sm + 4 * SPLP;
     uint64_t *bars = reinterpret_cast<uint64_t *>(sm + 8 * SPLP);   // one per ring slot
-    // this thread's adsorbed-part slots (node z in slot z & 1), filled by its own cp.async
+    // this thread's adsorbed-part slots (row q, node z in slot 2 q + (z & 1)), filled by its own
+    // cp.async
     float4 *sA = sm + 8 * SPLP + 2 + threadIdx.x;
     const int lx = a.lx, ly = a.ly, lz = a.lz;
     const float4 *__restrict__ Vg = a.V;
@@ -177,6 +204,20 @@ __device__ __forceinline__ void mp_slab_planes(const Args &a, int par, int x0, i
         __syncthreads();
     }
     auto slot = [&](int zz) { return (zz - z0 + 1) & 3; };
+    // the records of a plane that this thread copies (per-thread copies): their offsets in a plane of
+    // the box, the same for every plane
+    constexpr int COPIES = (SPL + MPS_THREADS - 1) / MPS_THREADS;
+    unsigned halo[COPIES];
+    if (!tma) {
+#pragma unroll
+        for (int q = 0; q < COPIES; ++q) {
+            const int k = (int)threadIdx.x + q * MPS_THREADS, hx = k % SHX, hy = k / SHX;
+            int gx = x0 + hx - 1, gy = y0 + hy - 1;
+            gx = gx < 0 ? gx + lx : (gx >= lx ? gx - lx : gx);   // lx >= 32: one wrap at most
+            gy = gy < 0 ? gy + ly : (gy >= ly ? gy - ly : gy);   // ly >= 8
+            halo[q] = (unsigned)gx + (unsigned)lx * (unsigned)gy;
+        }
+    }
     const unsigned long long wait_ns = a.wait_ns ? a.wait_ns : 2000000000ull;
     const bool skip_copies = a.skip_copies != 0;
     int last_issued = z0 - 2, last_waited = z0 - 2;   // bulk-copied planes issued / arrived
@@ -196,14 +237,13 @@ __device__ __forceinline__ void mp_slab_planes(const Args &a, int par, int x0, i
                 }
                 last_issued = zz;
             } else {
-                for (int k = threadIdx.x; k < SPL; k += MP_BLOCK) {
-                    const int hx = k % SHX, hy = k / SHX;
-                    int gx = x0 + hx - 1, gy = y0 + hy - 1;
-                    gx = gx < 0 ? gx + lx : (gx >= lx ? gx - lx : gx);   // lx >= 32: one wrap at most
-                    gy = gy < 0 ? gy + ly : (gy >= ly ? gy - ly : gy);   // ly >= 8
-                    const size_t idx = (size_t)gx + (size_t)lx * ((size_t)gy + (size_t)ly * gz);
-                    cp_async16(dv + k, Vg + idx);
-                    cp_async16(dp + k, Pg + idx);
+                const unsigned at = (unsigned)lx * (unsigned)ly * (unsigned)gz;
+#pragma unroll
+                for (int q = 0; q < COPIES; ++q) {
+                    const int k = (int)threadIdx.x + q * MPS_THREADS;
+                    if ((q + 1) * MPS_THREADS > SPL && k >= SPL) break;
+                    cp_async16(dv + k, Vg + (at + halo[q]));
+                    cp_async16(dp + k, Pg + (at + halo[q]));
                 }
             }
         }
@@ -220,69 +260,92 @@ __device__ __forceinline__ void mp_slab_planes(const Args &a, int par, int x0, i
         if (done) last_waited = zz;
         return done;
     };
-    const int tx = threadIdx.x % MPS_TX, ty = threadIdx.x / MPS_TX;
-    const int x = x0 + tx, y = y0 + ty;
-    const bool col = x < lx && y < ly;
+    const int tx = threadIdx.x % MPS_TX, ty = MPS_ROWS * (threadIdx.x / MPS_TX);
+    const int x = x0 + tx;
+    bool col[MPS_ROWS];
+    for (int q = 0; q < MPS_ROWS; ++q) col[q] = x < lx && y0 + ty + q < ly;
     const int c0 = (ty + 1) * SHX + (tx + 1);
-    // node offsets in 32 bits (a box holds fewer than 2^31 nodes); the column's arrays are
+    // node offsets in 32 bits (a box holds fewer than 2^31 nodes); the first column's arrays are
     // addressed from its first node
-    const unsigned col0 = (unsigned)x + (unsigned)lx * (unsigned)y, plane = (unsigned)lx * (unsigned)ly;
+    const unsigned col0 = (unsigned)x + (unsigned)lx * (unsigned)(y0 + ty), plane = (unsigned)lx * (unsigned)ly;
     const uint32_t *__restrict__ mcol = a.mask + col0;
     const float4 *__restrict__ auxcol = a.aux + col0;
     float4 *__restrict__ Pout = a.P[par ^ 1] + col0;
-    // flag word of the column's node z; 0 (no fluid bit, no work) outside the tile's nodes
-    auto mask_at = [&](int z) { return (col && z < z1) ? __ldg(mcol + plane * (unsigned)z) : 0u; };
+    // flag word of node z of column q; 0 (no fluid bit, no work) outside the tile's nodes
+    auto mask_at = [&](int q, int z) {
+        return (col[q] && z < z1) ? __ldg(mcol + (plane * (unsigned)z + (unsigned)(q * lx))) : 0u;
+    };
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     bool ok = true;   // false once a wait for a bulk copy ran out
-    // a node of the column in flight: P (also the centre point of its plane for the links of
-    // the nodes above and below), running sums (x and y as one packed pair), flag word
+    // a node of a column in flight: P (also the centre point of its plane for the links of
+    // the nodes above and below), running sums, flag word
     struct Node {
         float4 p;
-        float2 nxy;
-        float nz;
+        float n0, n1, n2;
         uint32_t m;
     };
-    Node S0, S1, S2;
-    S0.m = S1.m = S2.m = 0u;
-    S0.p = S1.p = S2.p = zero;
-    S0.nxy = S1.nxy = S2.nxy = make_float2(0.0f, 0.0f);
-    S0.nz = S1.nz = S2.nz = 0.0f;
-    uint32_t m_next = mask_at(z0);   // flag word of node zz+1 at the start of step zz
-    // Step zz with A = node zz-1, B = node zz, C = node zz+1 (DA, DB, DC: which of them can be
+    struct Nodes {
+        Node q[MPS_ROWS];
+    };
+    Nodes S0, S1, S2;
+    float vt[MPS_ROWS][3];
+    uint32_t m_next[MPS_ROWS];   // flag words of the nodes zz+1 at the start of step zz
+    for (int q = 0; q < MPS_ROWS; ++q) {
+        S0.q[q] = S1.q[q] = S2.q[q] = Node{zero, 0.0f, 0.0f, 0.0f, 0u};
+        vt[q][0] = vt[q][1] = vt[q][2] = 0.0f;
+        m_next[q] = mask_at(q, z0);
+    }
+    // Step zz with A = nodes zz-1, B = nodes zz, C = nodes zz+1 (DA, DB, DC: which of them can be
     // nodes of the tile: the first step zz = z0-1 has only C, the last zz = z1 only A, and each
     // computes only their links).
-    auto step = [&](auto DA, auto DB, auto DC, Node &A, Node &B, Node &C, int zz) {
+    auto step = [&](auto DA, auto DB, auto DC, Nodes &A, Nodes &B, Nodes &C, int zz) {
         constexpr bool da = decltype(DA)::value, db = decltype(DB)::value, dc = decltype(DC)::value;
-        // node zz-1's fixed (u*, D), needed at the end of this step: loaded before the links, so
-        // that they hide its latency
-        float4 axA = zero;
-        if constexpr (da)
-            if (A.m & FLUID_BIT) axA = __ldg(auxcol + plane * (unsigned)(zz - 1));
+        // the fixed (u*, D) of the nodes zz-1, needed at the end of this step: loaded before the
+        // links, so that they hide its latency
+        float4 axA[MPS_ROWS];
+#pragma unroll
+        for (int q = 0; q < MPS_ROWS; ++q) {
+            axA[q] = zero;
+            if constexpr (da)
+                if (A.q[q].m & FLUID_BIT) axA[q] = __ldg(auxcol + (plane * (unsigned)(zz - 1) + (unsigned)(q * lx)));
+        }
         if (dc && ok) ok = wait_plane(zz + 1);
         // one verdict for the block: once a wait has run out, no thread uses the ring and no new
         // copy is issued (the per-thread path never fails)
         ok = __syncthreads_and(ok);
-        if (ok) load_plane(zz + 3);
-        if constexpr (dc) {   // node zz+1 enters; its centre P is the next step's centre point
-            C.m = m_next;
-            m_next = mask_at(zz + 2);
-            C.p = (ok && col) ? sP[slot(zz + 1) * SPLP + c0] : zero;
-            C.nxy = make_float2(0.0f, 0.0f);
-            C.nz = 0.0f;
+        if (!ok) return;
+        load_plane(zz + 3);
+        if constexpr (dc) {   // the nodes zz+1 enter; their centre P is the next step's centre point
+#pragma unroll
+            for (int q = 0; q < MPS_ROWS; ++q) {
+                C.q[q].m = m_next[q];
+                m_next[q] = mask_at(q, zz + 2);
+                C.q[q].p = sP[slot(zz + 1) * SPLP + c0 + q * SHX];   // also beyond the box: a column's neighbour
+                C.q[q].n0 = C.q[q].n1 = C.q[q].n2 = 0.0f;
+            }
         }
         // every lane runs the links (no branch: a warp runs them whenever one of its lanes has a
         // fluid node in flight); a lane without one adds onto a running sum it never stores
-        if (ok) {
-            const int s0 = slot(zz) * SPLP + c0;
-            static_for<0, 9>([&](auto K) {
-                constexpr int k = decltype(K)::value;
-                constexpr int dx = pt_dx(k), dy = pt_dy(k);
-                constexpr bool axis = dx * dx + dy * dy <= 1;   // links (dx, dy, -1) and (dx, dy, +1)
-                if constexpr ((dc && axis) || (db && (dx != 0 || dy != 0)) || (da && axis)) {
-                    const float4 vn = sV[s0 + dy * SHX + dx];
+        const int s0 = slot(zz) * SPLP + c0;
+        // the points (dx, j) of the columns' neighbourhood, read when first needed: point (dx, j)
+        // is (dx, dy = j - q) of column q
+        float4 V3[3][MPS_ROWS + 2], P3[3][MPS_ROWS + 2];
+        static_for<0, 9>([&](auto K) {
+            constexpr int k = decltype(K)::value;
+            constexpr int dx = pt_dx(k), dy = pt_dy(k);
+            constexpr bool axis = dx * dx + dy * dy <= 1;   // links (dx, dy, -1) and (dx, dy, +1)
+            if constexpr ((dc && axis) || (db && (dx != 0 || dy != 0)) || (da && axis)) {
+                static_for<0, MPS_ROWS>([&](auto QQ) {
+                    constexpr int q = decltype(QQ)::value;
+                    constexpr int j = dy + q;
+                    if constexpr (slab_first_use(k, q, da, db, dc)) {
+                        V3[dx + 1][j + 1] = sV[s0 + j * SHX + dx];
+                        if constexpr (!(dx == 0 && j >= 0 && j < MPS_ROWS)) P3[dx + 1][j + 1] = sP[s0 + j * SHX + dx];
+                    }
+                    const float4 vn = V3[dx + 1][j + 1];
                     float4 pn;
-                    if constexpr (dx == 0 && dy == 0) pn = B.p;
-                    else pn = sP[s0 + dy * SHX + dx];
+                    if constexpr (dx == 0 && j >= 0 && j < MPS_ROWS) pn = B.q[j].p;
+                    else pn = P3[dx + 1][j + 1];
                     // lambda w / 2 of the point's two weight classes times its fluid flag: axis
                     // links (dx, dy) = (0, 0) in z and the in-plane axis links, diagonal the rest
                     constexpr bool need_ax = (dx == 0 && dy == 0) || (db && dx * dx + dy * dy == 1);
@@ -293,47 +356,56 @@ __device__ __forceinline__ void mp_slab_planes(const Args &a, int par, int x0, i
                     if constexpr (dc && axis) {   // link (dx, dy, -1) of node zz+1
                         constexpr int l = link_of(dx, dy, -1);
                         constexpr int w = wclass(l);
+                        Node &c = C.q[q];
                         mp32_link(mp32_scatter_flag(a.a1[w], mp32_cdot<-dx, -dy, 1>(vn), w == 1 ? lw_ax : lw_dg),
-                                   pn, C.p, C.nxy.x, C.nxy.y, C.nz);
+                                  pn, c.p, c.n0, c.n1, c.n2);
                     }
                     if constexpr (db && (dx != 0 || dy != 0)) {   // link (dx, dy, 0) of node zz
                         constexpr int l = link_of(dx, dy, 0);
                         constexpr int w = wclass(l);
+                        Node &c = B.q[q];
                         mp32_link(mp32_scatter_flag(a.a1[w], mp32_cdot<-dx, -dy, 0>(vn), w == 1 ? lw_ax : lw_dg),
-                                   pn, B.p, B.nxy.x, B.nxy.y, B.nz);
+                                  pn, c.p, c.n0, c.n1, c.n2);
                     }
                     if constexpr (da && axis) {   // link (dx, dy, +1) of node zz-1
                         constexpr int l = link_of(dx, dy, 1);
                         constexpr int w = wclass(l);
+                        Node &c = A.q[q];
                         mp32_link(mp32_scatter_flag(a.a1[w], mp32_cdot<-dx, -dy, -1>(vn), w == 1 ? lw_ax : lw_dg),
-                                   pn, A.p, A.nxy.x, A.nxy.y, A.nz);
+                                  pn, c.p, c.n0, c.n1, c.n2);
                     }
-                }
-            });
-        }
+                });
+            }
+        });
         if constexpr (da) {
-            if (ok && (A.m & FLUID_BIT)) {   // node zz-1 has all its links
-                const unsigned r = plane * (unsigned)(zz - 1);
-                float n0 = A.nxy.x, n1 = A.nxy.y, n2 = A.nz;
-                const float4 p = A.p;
-                vt[0] += p.x * axA.x;
-                vt[1] += p.y * axA.y;
-                vt[2] += p.z * axA.z;
-                mp32_finish(p, axA.w, n0, n1, n2);
-                if (a.ads && (A.m & INTERFACIAL_BIT)) {
-                    cp_async_wait1();   // node zz-1's copy was committed a step ago
-                    a.A[par ^ 1][col0 + r] =
-                        mp32_adsorb(p, sA[((zz - 1) & 1) * MP_BLOCK], a.ka, a.kd, a.one_minus_kd, n0, n1, n2);
+#pragma unroll
+            for (int q = 0; q < MPS_ROWS; ++q) {
+                const Node &c = A.q[q];
+                if (c.m & FLUID_BIT) {   // node zz-1 has all its links
+                    const unsigned r = plane * (unsigned)(zz - 1) + (unsigned)(q * lx);
+                    float n0 = c.n0, n1 = c.n1, n2 = c.n2;
+                    vt[q][0] += c.p.x * axA[q].x;
+                    vt[q][1] += c.p.y * axA[q].y;
+                    vt[q][2] += c.p.z * axA[q].z;
+                    mp32_finish(c.p, axA[q].w, n0, n1, n2);
+                    if (a.ads && (c.m & INTERFACIAL_BIT)) {
+                        cp_async_wait1();   // node zz-1's copy was committed a step ago
+                        a.A[par ^ 1][col0 + r] = mp32_adsorb(c.p, sA[(2 * q + ((zz - 1) & 1)) * MPS_THREADS], a.ka, a.kd,
+                                                             a.one_minus_kd, n0, n1, n2);
+                    }
+                    __stcs(Pout + r, make_float4(n0, n1, n2, 0.0f));
                 }
-                __stcs(Pout + r, make_float4(n0, n1, n2, 0.0f));
             }
         }
-        // node zz+1's adsorbed part into the slot node zz-1 has just read: committed with the next
-        // plane's copies (or on its own where the planes are bulk-copied), it has landed by the
-        // time node zz+1 finishes, two steps on
+        // the adsorbed parts of the nodes zz+1 into the slots that the nodes zz-1 have just read:
+        // committed with the next plane's copies (or on their own where the planes are bulk-copied),
+        // they have landed by the time the nodes zz+1 finish, two steps on
         if constexpr (dc) {
-            if (ok && a.ads && (C.m & INTERFACIAL_BIT))
-                cp_async16(sA + ((zz + 1) & 1) * MP_BLOCK, a.A[par] + col0 + plane * (unsigned)(zz + 1));
+#pragma unroll
+            for (int q = 0; q < MPS_ROWS; ++q)
+                if (a.ads && (C.q[q].m & INTERFACIAL_BIT))
+                    cp_async16(sA + (2 * q + ((zz + 1) & 1)) * MPS_THREADS,
+                               a.A[par] + (col0 + plane * (unsigned)(zz + 1) + (unsigned)(q * lx)));
             if (tma) cp_async_commit();
         }
     };
@@ -345,16 +417,21 @@ __device__ __forceinline__ void mp_slab_planes(const Args &a, int par, int x0, i
     ok = __syncthreads_and(ok);
     if (ok) load_plane(z0 + 1);
     __syncthreads();
-    S0.p = (ok && col) ? sP[slot(z0 - 1) * SPLP + c0] : zero;   // centre P of plane z0-1
+    for (int q = 0; q < MPS_ROWS; ++q)   // centre P of plane z0-1
+        S0.q[q].p = ok ? sP[slot(z0 - 1) * SPLP + c0 + q * SHX] : zero;
     // S0, S1, S2 = nodes zz-1, zz, zz+1 at step zz (a loop unrolled by three to rotate the slots
     // instead costs more in instruction fetch than the register moves it saves)
     step(F{}, F{}, T{}, S2, S0, S1, z0 - 1);
-    for (int zz = z0; zz < z1; ++zz) {
+    for (int zz = z0; zz < z1 && ok; ++zz) {
         step(T{}, T{}, T{}, S0, S1, S2, zz);
         S0 = S1;
         S1 = S2;
     }
-    step(T{}, F{}, F{}, S0, S1, S2, z1);   // the last node's links from plane z1
+    if (ok) step(T{}, F{}, F{}, S0, S1, S2, z1);   // the last nodes' links from plane z1
+    for (int d = 0; d < 3; ++d) {
+        vacf[d] = (double)vt[0][d];
+        for (int q = 1; q < MPS_ROWS; ++q) vacf[d] += (double)vt[q][d];
+    }
     cp_async_wait0();   // no copy of this thread still lands when the block leaves
     if (!ok) {
         // a wait ran out: let the copies already issued into this block's shared memory land

@@ -33,7 +33,7 @@ __device__ __forceinline__ double block_sum_fixed(double v, double *sh)
     return v;
 }
 
-// Sum of 3 values over a block of MP_BLOCK threads in one pass (fixed order); valid in thread 0.
+// Sum of 3 values over a block of up to MP_BLOCK threads (a multiple of 32) in one pass (fixed order); valid in thread 0.
 __device__ __forceinline__ void block_sum3_fixed(double (&v)[3])
 {
     __shared__ double sh[3][MP_BLOCK / 32];
@@ -47,7 +47,7 @@ __device__ __forceinline__ void block_sum3_fixed(double (&v)[3])
     if (wid == 0) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            v[d] = lane < MP_BLOCK / 32 ? sh[d][lane] : 0.0;
+            v[d] = lane < (blockDim.x >> 5) ? sh[d][lane] : 0.0;
             v[d] = warp_sum_fixed(v[d]);
         }
     }
