@@ -88,6 +88,9 @@ LbConst64 make_const64(double tau)
         K.c2a2cs2[w] = K.c2a2[w] * csq;
         K.c3a1[w] = K.c3 * K.a1[w];
     }
+    int exp2 = 0;
+    const bool pow2 = std::fabs(std::frexp(K.c1, &exp2)) == 0.5;
+    K.form = K.c2 == 1.0 && K.c3 == 0.5 ? FORM_TAU1 : (pow2 ? FORM_POW2 : FORM_ANY);
     K.fix_c2 = std::llrint(std::ldexp(K.c2, 61));   // tau >= 1/2: at most 2^62
     K.fix_c1 = (1ll << 62) - 2 * K.fix_c2;
     K.fix_c3 = (1ll << 62) - K.fix_c2;

@@ -77,6 +77,8 @@ __host__ __device__ __forceinline__ void static_for(F &&f)
 
 // Reference constants in FP64, computed once on the host (module_lbmodel.f90:127-147,
 // module_collision.f90:28,99-103) and passed by value to the kernels.
+enum { FORM_ANY, FORM_POW2, FORM_TAU1 };   // flow64.cuh:collide_node
+
 struct LbConst64 {
     double a0[3], a1[3], a2[3], two_a2[3];  // per weight class
     double k1, k0;                          // (1 - cs^2) and (0 - cs^2)
@@ -89,6 +91,7 @@ struct LbConst64 {
     // fix_c2, c2/36 2^66, 2^63 (1 - c1 - sum of c2 a0)
     long long fix_c1, fix_c2, fix_c3, fix_c2_36;
     int fix_loss;
+    int form;   // of the strict collision: FORM_*
 };
 
 // Device-resident control block of the reference flow loop (equilibration.f90:143-491).

@@ -43,7 +43,9 @@ __host__ __device__ constexpr int role_of(int l)
 // module_collision.f90:77-108 for one fluid node, all 19 velocities.
 // FMASK: which components of the force are non-zero (bit 0 x, 1 y, 2 z); 0 = no force.
 // UCF: the force is the launch-uniform f_ext and c_l.F is taken from a.cf.
-// TAU1: the relaxation time is 1 (c1 = 0, c2 = 1, c3 = 1/2), the reference's default.
+// FORM, by the relaxation time: FORM_TAU1, tau = 1 (c1 = 0, c2 = 1, c3 = 1/2), the reference's
+// default; FORM_POW2, c1 = 1 - 1/tau a power of two in magnitude (tau = 0.8, 2/3, 4/3, 2, ..), so
+// that c1 n is exact; FORM_ANY.
 //
 // The step is bound by the FP64 pipe (one warp instruction per 19 cycles of an SM), so what counts
 // is the number of FP64 instructions.  Every rounding of the reference is kept, but a product that
@@ -53,13 +55,16 @@ __host__ __device__ constexpr int role_of(int l)
 //   x + a2 S              = fma(a2, S, x)
 //   (2 a2 cu) cF + x      = fma(2 a2, cu cF, x)      cu cF formed once per pair (both change sign)
 // and a1 and 2 a2 of a diagonal link are half of an axis link's, so T of a diagonal link is half
-// of the same expression with the axis constants (c3 T = (c3/2) (2 T)).  With TAU1 also
-//   c1 n + c2 neq         = fma(c1, n, neq),         x + c3 T = fma(c3, T, x).
-// (Exact unless a value falls below the smallest normal double.)  The step of the 192^3 porous
-// medium issues 334 FP64 instructions per node in the term-by-term form.
+// of the same expression with the axis constants (c3 T = (c3/2) (2 T)).  With FORM_POW2 also
+//   c1 n + c2 neq         = fma(c1, n, c2 neq)
+// and with FORM_TAU1 that without c2 and x + c3 T = fma(c3, T, x).
+// (Exact unless a value falls below the smallest normal double.)  The step of a porous medium
+// issues 334 FP64 instructions per node in the term-by-term form and 405 us for 0.52 M fluid nodes
+// (tau 0.8, loop); 287 and 319 us so far; with the sums and divisions in integers (moments19_units,
+// velocity) 231 and 261 us, with FORM_POW2 212 and 237 us, 88 % of the pipe.
 // ROLE: every velocity (-1), or a quarter of them: 0 the rest and axis velocities, 1 / 2 / 3 the
 // diagonals of the xy / xz / yz planes (role_of).
-template <int FMASK, bool UCF, bool TAU1, int ROLE = -1>
+template <int FMASK, bool UCF, int FORM, int ROLE = -1>
 __device__ __forceinline__ void collide_node(double (&n)[Q], const double rho, const double jx,
                                              const double jy, const double jz, const double ux,
                                              const double uy, const double uz, const double fx,
@@ -98,7 +103,9 @@ __device__ __forceinline__ void collide_node(double (&n)[Q], const double rho, c
         constexpr int l = decltype(L)::value;
         constexpr Vel c = vel(l);
         constexpr int w = wclass(l);
-        double r = TAU1 ? __fma_rn(K.c1, n[l], neq) : K.c1 * n[l] + K.c2 * neq;
+        double r = FORM == FORM_TAU1   ? __fma_rn(K.c1, n[l], neq)
+                   : FORM == FORM_POW2 ? __fma_rn(K.c1, n[l], K.c2 * neq)
+                                       : K.c1 * n[l] + K.c2 * neq;
         if constexpr (FMASK != 0) {
             double t1 = 0.0;
             if constexpr (FMASK & 1) t1 = c.x > 0 ? gxp : (c.x < 0 ? gxm : gx0);
@@ -118,7 +125,7 @@ __device__ __forceinline__ void collide_node(double (&n)[Q], const double rho, c
                                    ((FMASK & 4) && c.z != 0);
             if constexpr (hasT2) T = __fma_rn(K.two_a2[1], cucf, T);
             const double k3 = w == 2 ? K.c3h : K.c3;
-            r = TAU1 ? __fma_rn(k3, T, r) : r + k3 * T;
+            r = FORM == FORM_TAU1 ? __fma_rn(k3, T, r) : r + k3 * T;
         }
         n[l] = r;
     };
@@ -154,12 +161,92 @@ __device__ __forceinline__ void collide_strict_u(double (&n)[Q], const double rh
                                                  const double fx, const double fy, const double fz,
                                                  const FlowArgs64 &a, const bool force)
 {
-    if (a.K.c2 == 1.0 && a.K.c3 == 0.5) {
-        if (force) collide_node<FMASK, UCF, true, ROLE>(n, rho, jx, jy, jz, ux, uy, uz, fx, fy, fz, a);
-        else collide_node<0, true, true, ROLE>(n, rho, jx, jy, jz, ux, uy, uz, 0.0, 0.0, 0.0, a);
+    auto collide = [&](auto F) {
+        constexpr int form = decltype(F)::value;
+        if (force) collide_node<FMASK, UCF, form, ROLE>(n, rho, jx, jy, jz, ux, uy, uz, fx, fy, fz, a);
+        else collide_node<0, true, form, ROLE>(n, rho, jx, jy, jz, ux, uy, uz, 0.0, 0.0, 0.0, a);
+    };
+    if (a.K.form == FORM_TAU1) collide(std::integral_constant<int, FORM_TAU1>{});
+    else if (a.K.form == FORM_POW2) collide(std::integral_constant<int, FORM_POW2>{});
+    else collide(std::integral_constant<int, FORM_ANY>{});
+}
+
+// j / rho with the rounding of an IEEE division, on the integer pipes: a division is some ten
+// dependent FP64 instructions of 19 SM cycles a warp, this some 15 cycles, and the three of a node
+// share one reciprocal.  Long division of the mantissas: with r = 2^125 / R (R, J the mantissas at bit
+// 62) the quotient's first 54 bits M = floor are those of J r / 2^64 or one off, the remainder
+// J 2^k - M R (exact modulo 2^64) puts M right, and M's last bit with the remainder rounds to nearest
+// even.  Arguments outside 2^-767 .. 2^767 in magnitude (0 apart), or a rho <= 0, are divided in FP64.
+__device__ __forceinline__ bool div_range(double x)
+{
+    const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+    return e - 256u < 1534u;
+}
+
+__device__ __forceinline__ bool is_zero(double x)
+{
+    return ((unsigned)__double2hiint(x) << 1 | (unsigned)__double2loint(x)) == 0u;
+}
+
+__device__ __forceinline__ unsigned long long mantissa53(double x)
+{
+    return ((unsigned long long)(((unsigned)__double2hiint(x) & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(x);
+}
+
+// 2^125 / R: the reciprocal of R's leading 24 bits in FP32, then two Newton-Raphson steps
+// r <- r + r (1 - R r), each of which doubles the bits that are right (to 44, then to some 59)
+__device__ __forceinline__ unsigned long long recip125(unsigned long long R)
+{
+    const unsigned q = __float_as_uint(__frcp_rn((float)(unsigned)(R >> 39)));
+    unsigned long long r = (unsigned long long)((q & 0x7fffffu) | 0x800000u) << ((q >> 23) - 64u);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const long long e = (long long)((1ull << 61) - __umul64hi(R, r));
+        r += (unsigned long long)__mul64hi((long long)(r >> 1), e << 4);
+    }
+    return r;
+}
+
+__device__ __forceinline__ double div_recip(double j, double rho, unsigned long long r)
+{
+    const unsigned long long Rm = mantissa53(rho), Jm = mantissa53(j);
+    const unsigned hj = (unsigned)__double2hiint(j), hr = (unsigned)__double2hiint(rho);
+    const bool below = Jm < Rm;
+    unsigned long long M = __umul64hi(Jm << 10, r) >> (below ? 7 : 8);
+    long long rem = (long long)((Jm << (below ? 54 : 53)) - M * Rm);
+    if (rem < 0) {
+        --M;
+        rem += (long long)Rm;
+    } else if (rem >= (long long)Rm) {
+        ++M;
+        rem -= (long long)Rm;
+    }
+    const unsigned lo = (unsigned)M, up = lo & 1u & (unsigned)(rem != 0 || (lo & 2u));
+    const unsigned e = 1022u + ((hj >> 20) & 0x7ffu) - (hr >> 20) - (below ? 1u : 0u);
+    const unsigned long long bits = ((unsigned long long)(e << 20 | (hj & 0x80000000u)) << 32) + ((M >> 1) + up);
+    return is_zero(j) ? j : __longlong_as_double((long long)bits);
+}
+
+// one quotient, for the threads that share a node
+__device__ __forceinline__ double divide(double j, double rho)
+{
+    if (__double2hiint(rho) >= 0 && div_range(rho) && (div_range(j) || is_zero(j)))
+        return div_recip(j, rho, recip125(mantissa53(rho) << 10));
+    return j / rho;
+}
+
+__device__ __forceinline__ void velocity(double jx, double jy, double jz, double rho, double &ux, double &uy, double &uz)
+{
+    auto fits = [](double j) { return div_range(j) || is_zero(j); };
+    if (__double2hiint(rho) >= 0 && div_range(rho) && fits(jx) && fits(jy) && fits(jz)) {
+        const unsigned long long r = recip125(mantissa53(rho) << 10);
+        ux = div_recip(jx, rho, r);
+        uy = div_recip(jy, rho, r);
+        uz = div_recip(jz, rho, r);
     } else {
-        if (force) collide_node<FMASK, UCF, false, ROLE>(n, rho, jx, jy, jz, ux, uy, uz, fx, fy, fz, a);
-        else collide_node<0, true, false, ROLE>(n, rho, jx, jy, jz, ux, uy, uz, 0.0, 0.0, 0.0, a);
+        ux = jx / rho;
+        uy = jy / rho;
+        uz = jz / rho;
     }
 }
 
@@ -168,7 +255,9 @@ __device__ __forceinline__ void collide_strict(double (&n)[Q], const double rho,
                                                const double jz, const double fx, const double fy, const double fz,
                                                const FlowArgs64 &a, const bool force)
 {
-    collide_strict_u<FMASK, UCF>(n, rho, jx, jy, jz, jx / rho, jy / rho, jz / rho, fx, fy, fz, a, force);
+    double ux, uy, uz;
+    velocity(jx, jy, jz, rho, ux, uy, uz);
+    collide_strict_u<FMASK, UCF>(n, rho, jx, jy, jz, ux, uy, uz, fx, fy, fz, a, force);
 }
 
 // LBGPU_FP64_FUSED: density and flux from the pair sums and differences of opposite velocities
@@ -475,6 +564,82 @@ __device__ __forceinline__ void moments19(const double (&n)[Q], double fhx, doub
     jx = X;
     jy = Y;
     jz = Z;
+}
+
+// The same sums, each addition with its FP64 rounding, in 64-bit integers: a DADD takes 19 SM cycles
+// a warp, an integer addition rounded to 53 bits some 5.  The populations become integers 59 bits below
+// the largest one's binade, exact while they lie within 2^7 of it; false (and nothing written) for a
+// node with one outside, a negative or non-finite one, or a sum beyond 2^62 units.
+__device__ __forceinline__ long long round53(long long t)
+{
+    const int hi = (int)(t >> 32);
+    const int k = max(0, 11 - __clz(hi ^ (hi >> 31)));   // bits beyond 53 (a power of two may count one short: exact anyway)
+    const unsigned lo = (unsigned)t, cut = ~(0xffffffffu << k);
+    t += (long long)((cut >> 1) + ((lo >> k) & cut & 1u));
+    return t & ~(long long)cut;
+}
+
+// t units, of at most 53 significant bits, as a double
+__device__ __forceinline__ double from_units(long long t, int emax)
+{
+    const unsigned sign = (unsigned)(t >> 32) & 0x80000000u;
+    const unsigned long long mag = (unsigned long long)(t < 0 ? -t : t);
+    const int lz = __clzll((long long)mag);
+    const unsigned long long m = (mag << (lz & 63)) >> 11;
+    const unsigned long long bits = ((unsigned long long)((unsigned)(emax + 3 - lz) << 20 | sign) << 32) + m;
+    return t == 0 ? 0.0 : __longlong_as_double((long long)bits);
+}
+
+__device__ __forceinline__ bool to_units(double x, int emax, long long &t)
+{
+    const unsigned hi = (unsigned)__double2hiint(x);
+    const int down = emax - (int)((hi >> 20) & 0x7ffu);
+    const long long m = (long long)(mantissa53(x) << ((7 - down) & 63));
+    t = (int)hi < 0 ? -m : m;
+    return (unsigned)down <= 7u;
+}
+
+__device__ __forceinline__ bool moments19_units(const double (&n)[Q], bool fm, double fhx, double fhy, double fhz,
+                                                double &rho, double &jx, double &jy, double &jz)
+{
+    int emax = 0;
+#pragma unroll
+    for (int l = 0; l < Q; ++l) emax = max(emax, __double2hiint(n[l]) >> 20);   // a negative one counts as small
+    bool ok = (unsigned)(emax - 512) < 1024u;
+    long long v[Q];
+#pragma unroll
+    for (int l = 0; l < Q; ++l) ok &= to_units(n[l], emax, v[l]) && __double2hiint(n[l]) >= 0;
+    // the first addition of j is F/2's, which has finer bits: in FP64
+    long long X = v[1], Y = v[3], Z = v[5];
+    if (fm) {
+        if (__double2hiint(fhx) | __double2loint(fhx)) ok &= to_units(fhx + n[1], emax, X);
+        if (__double2hiint(fhy) | __double2loint(fhy)) ok &= to_units(fhy + n[3], emax, Y);
+        if (__double2hiint(fhz) | __double2loint(fhz)) ok &= to_units(fhz + n[5], emax, Z);
+    }
+    long long R = v[0];
+    static_for<1, Q>([&](auto L) {
+        constexpr int l = decltype(L)::value;
+        constexpr Vel c = vel(l);
+        R = round53(R + v[l]);
+        // no population reaches 2^60: at most 2^62 here keeps 6 more from wrapping unseen
+        if constexpr (l == 6 || l == 12 || l == 18) ok &= (unsigned long long)R <= (1ull << 62);
+        if constexpr (c.x != 0 && l != 1) X = round53(c.x > 0 ? X + v[l] : X - v[l]);
+        if constexpr (c.y != 0 && l != 3) Y = round53(c.y > 0 ? Y + v[l] : Y - v[l]);
+        if constexpr (c.z != 0 && l != 5) Z = round53(c.z > 0 ? Z + v[l] : Z - v[l]);
+    });
+    if (!ok) return false;
+    rho = from_units(R, emax);
+    jx = from_units(X, emax);
+    jy = from_units(Y, emax);
+    jz = from_units(Z, emax);
+    return true;
+}
+
+__device__ __forceinline__ void moments19_fast(const double (&n)[Q], bool fm, double fx, double fy, double fz,
+                                               double &rho, double &jx, double &jy, double &jz)
+{
+    const double hx = fm ? fx / 2.0 : 0.0, hy = fm ? fy / 2.0 : 0.0, hz = fm ? fz / 2.0 : 0.0;
+    if (!moments19_units(n, fm, hx, hy, hz, rho, jx, jy, jz)) moments19(n, hx, hy, hz, rho, jx, jy, jz);
 }
 
 // n < 0 and NaN / Inf tests on the bits, off the FP64 pipe (a comparison of doubles occupies it like

@@ -22,7 +22,7 @@
 namespace lbg {
 namespace {
 
-constexpr int BLOCK = 256;
+constexpr int BLOCK = 256, STEP_BLOCK = 128;
 
 struct Coords {
     int x, y, z;
@@ -106,8 +106,10 @@ __device__ void control_step(FlowCtl *c, double *hist)
     *c = d;
 }
 
+// Blocks per SM asked for, of 128 threads: measured on the same boxes, strict 237.5 us a step with 4,
+// 239.9 with 5, 239.3 with 6, 248 with 8; fused 149.4 with 4, 140.2 with 5, 160 with 6.
 template <int FMASK, bool FIELD, bool CHECK, bool REF, bool FUSED>
-__global__ void __launch_bounds__(BLOCK) k_flow_step(const FlowArgs64 a)
+__global__ void __launch_bounds__(STEP_BLOCK, FUSED ? 5 : 4) k_flow_step(const FlowArgs64 a)
 {
     int parity = a.parity, fm = a.force_moment, fc = a.force_collide;
     if constexpr (REF) {
@@ -151,8 +153,7 @@ __global__ void __launch_bounds__(BLOCK) k_flow_step(const FlowArgs64 a)
                 if (fm) moments19_pairs(n, fx / 2.0, fy / 2.0, fz / 2.0, rho, jx, jy, jz);
                 else moments19_pairs(n, 0.0, 0.0, 0.0, rho, jx, jy, jz);
             } else {
-                if (fm) moments19(n, fx / 2.0, fy / 2.0, fz / 2.0, rho, jx, jy, jz);
-                else moments19(n, 0.0, 0.0, 0.0, rho, jx, jy, jz);
+                moments19_fast(n, fm != 0, fx, fy, fz, rho, jx, jy, jz);
             }
             if constexpr (CHECK) {
                 const double ox = a.jx[node], oy = a.jy[node], oz = a.jz[node];
@@ -310,13 +311,14 @@ unsigned grid_of(long long N) { return (unsigned)((N + BLOCK - 1) / BLOCK); }
 
 // Threads per block of a step over n nodes.  A warp instruction of doubles occupies its quarter of
 // an SM for 64 cycles whatever its lanes, so a small box is spread over the SMs warp by warp: up to
-// 608 warps (152 SMs x 4 quarters) as one-warp blocks, then two-warp blocks until a block of eight
-// warps leaves no SM without its share (152 SMs x 8 blocks), where the fewer atomics of large
-// blocks win.
+// 608 warps (152 SMs x 4 quarters) as one-warp blocks, then two-warp blocks up to 64 warps an SM.
+// Above, four-warp blocks: a block's load, integer and FP64 phases overlap with those of the blocks
+// beside it, and smaller blocks leave at finer grain (0.52 M fluid nodes, strict loop: 248 us a step
+// with 256 threads, 241 with 128, 242 with 64; fused, 1.26 M: 154, 150, 151).
 unsigned step_block(long long n)
 {
     const long long warps = (n + 31) / 32;
-    return warps <= 608 ? 32u : (warps <= 152 * 8 * (BLOCK / 32) ? 64u : (unsigned)BLOCK);
+    return warps <= 608 ? 32u : (warps <= 152 * 64 ? 64u : (unsigned)STEP_BLOCK);
 }
 
 template <bool FIELD, bool CHECK, bool REF, bool FUSED>

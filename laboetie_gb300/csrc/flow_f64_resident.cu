@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(SPLIT ? 128 : RT, 1) k_flow64_resident(const R
             if (r.loop) bad = check19(n);
             double rho, jx = 0.0, jy = 0.0, jz = 0.0;
             if constexpr (FUSED) fused_step<FMASK, true, true>(n, fm, fc, fx, fy, fz, a, jx, jy, jz);
-            else moments19(n, fm ? fx / 2.0 : 0.0, fm ? fy / 2.0 : 0.0, fm ? fz / 2.0 : 0.0, rho, jx, jy, jz);
+            else moments19_fast(n, fm, fx, fy, fz, rho, jx, jy, jz);
             if (r.loop) {
                 const double e = max_nonneg(max_nonneg(fabs(jx - jold[0]), fabs(jy - jold[1])), fabs(jz - jold[2]));
                 err = (unsigned long long)__double_as_longlong(e);
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(SPLIT ? 128 : RT, 1) k_flow64_resident(const R
             smom[role][lane] = mom;
             __syncthreads();
             const double rho = smom[0][lane];
-            if (role > 0) su[role][lane] = mom / rho;
+            if (role > 0) su[role][lane] = divide(mom, rho);
             __syncthreads();
             const double jx = smom[1][lane], jy = smom[2][lane], jz = smom[3][lane];
             const double ux = su[1][lane], uy = su[2][lane], uz = su[3][lane];
