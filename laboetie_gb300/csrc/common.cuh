@@ -105,9 +105,6 @@ struct FlowCtl {
     int conv_without, conv_with;
     int max_steps;
     int exit_step;
-    unsigned status;               // lbgpu_status bits raised on the device
-    unsigned blocks_done;          // last-block-done counter
-    unsigned long long err_bits;   // running max of |j - j_old| as IEEE bits (non-negative)
     double target_error;
     double last_l2err;
     int hist_cap;
@@ -116,6 +113,10 @@ struct FlowCtl {
     // the next check reads, and the moment / collision forces of the next AA launch
     int check_fm, aa_fm, aa_fc;
     int exit_phase;         // AA phase of the state the loop exited on
+    // What every block of a launch updates, on a cache line of its own
+    alignas(128) unsigned long long err_bits;   // running max of |j - j_old| as IEEE bits (non-negative)
+    unsigned status;                            // lbgpu_status bits raised on the device
+    unsigned blocks_done;                       // last-block-done counter
 };
 
 // Maximum of two values that are each non-negative or a NaN with the sign bit clear (what fabs

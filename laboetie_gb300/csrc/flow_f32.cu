@@ -25,6 +25,7 @@ namespace lbg {
 namespace {
 
 constexpr int BLOCK = 256;
+constexpr unsigned CHECK_BLOCKS = 456;
 
 struct Coords32 {
     int X[3], Y[3], Z[3];
@@ -177,19 +178,24 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_aa32(const FlowArgs32 a)
 // n = d + w rho0 < 0 and non-finite tests, j stored for the next check; the last block runs the
 // control step.  A no-op once the loop has exited.  n < 0 is d < -w rho0, and for a float d that is
 // d < neg_below, the smallest float not below -w rho0 (formed exactly on the host).
-// 61^3 touching spheres (74 k fluid nodes), AA launch and check: 36.4 us per step with FP64
-// moments (bound by the FP64 pipe), 16.5 with these.
+// A block takes its share of the nodes in turn: CHECK_BLOCKS blocks fill the device three times per SM
+// (85 registers, so that a node's 19 loads are in flight together), and each ends with two atomics
+// and a fence on one cache line.  One block per 256 nodes queued thousands of them, beside a control
+// block in the same line that every block reads first.  AA launch and check, us per step, 1.26 M /
+// 4.25 M fluid nodes (porous 128^3 / 192^3): 453 / 1481 with FP64 moments; 260 / 931 with integer sums;
+// 144 / 483 with the counters on a line of their own; 85 / 270 so (30 / 107 of them the AA launch, 23 /
+// 78 the check's bytes at the HBM rate; 4 blocks of 64 registers: 126 / 439, 2 of 128: 92 / 296).
 template <bool SWAPPED, typename Off = unsigned>
-__global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
+__global__ void __launch_bounds__(BLOCK, 3) k_aa_check32(const FlowArgs32 a)
 {
     // the control block is written by the last block only, after every block has read it: plain
     // loads, which one request per SM serves
     if (a.ctl->done) return;
     const int fm = a.ctl->check_fm;
-    const unsigned i = blockIdx.x * BLOCK + threadIdx.x;
     unsigned long long err = 0;
     unsigned bad = 0;
-    if (i < a.Nf) {
+#pragma unroll 1
+    for (unsigned i = blockIdx.x * BLOCK + threadIdx.x; i < a.Nf; i += gridDim.x * BLOCK) {
         const unsigned c = a.cpos[i];
         const unsigned p = lattice_of(a, c);
         const double ox = a.jx[p], oy = a.jy[p], oz = a.jz[p];
@@ -201,7 +207,7 @@ __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
 #pragma unroll
             for (int l = 0; l < Q; ++l) f[l] = g[(size_t)l * a.Nf + i];
         }
-        bad = check_dev19(f, a);
+        bad |= check_dev19(f, a);
         double jx, jy, jz;
         exact_flux(f, jx, jy, jz);
         if (fm) {
@@ -209,7 +215,8 @@ __global__ void __launch_bounds__(BLOCK) k_aa_check32(const FlowArgs32 a)
             jy += a.half_force[1];
             jz += a.half_force[2];
         }
-        err = flux_change_bits(jx - ox, jy - oy, jz - oz);
+        const unsigned long long e = flux_change_bits(jx - ox, jy - oy, jz - oz);
+        err = e > err ? e : err;
         a.jx[p] = jx;
         a.jy[p] = jy;
         a.jz[p] = jz;
@@ -468,7 +475,7 @@ cudaError_t launch_aa_step_f32(const FlowArgs32 &a, bool odd, cudaStream_t s)
 
 cudaError_t launch_aa_check_f32(const FlowArgs32 &a, bool swapped, cudaStream_t s)
 {
-    const unsigned grid = (a.Nf + BLOCK - 1) / BLOCK;
+    const unsigned grid = std::min((a.Nf + BLOCK - 1) / BLOCK, CHECK_BLOCKS);
     if (swapped && a.wide) k_aa_check32<true, unsigned long long><<<grid, BLOCK, 0, s>>>(a);
     else if (swapped) k_aa_check32<true><<<grid, BLOCK, 0, s>>>(a);
     else k_aa_check32<false><<<grid, BLOCK, 0, s>>>(a);
