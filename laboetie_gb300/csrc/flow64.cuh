@@ -358,8 +358,9 @@ __device__ __forceinline__ void collide_node_fused(double (&n)[Q], const double 
 // depend on rho).  Nodes outside the fixed-point range -- a negative or non-finite
 // population, the largest one below 2^-895, rho from 8 times the largest one's binade up, |j| from
 // a quarter of it up, a force from a sixteenth of it up -- take the FP64 form.
-// Porous medium of 128^3 (1.26 M fluid nodes), tau 0.8: 400 -> 165 us a step (57 us of HBM traffic;
-// now bound by the integer pipes).  Error of j against binary128 after 120 steps of 24^3, tau 0.62 /
+// Porous medium of 128^3 (1.26 M fluid nodes), tau 0.8: 400 -> 135 us a step (57 us of HBM traffic;
+// now bound by the integer pipes): 165 as first built, 140 in blocks of 128 threads, 135 with the
+// short shifts of the common case.  Error of j against binary128 after 120 steps of 24^3, tau 0.62 /
 // 0.8 / 1.3: 1.4e-13 / 5e-13 / 3.5e-13 of its norm where the FP64 form has 6e-13 / 8e-13 / 9e-13.
 
 __device__ __forceinline__ long long mulhi(long long a, long long b) { return __mul64hi(a, b); }
@@ -375,7 +376,7 @@ __device__ __forceinline__ double fixed_to_double(long long v, int emax)
         return __hiloint2double(__double2hiint(r) + (emax - 1082) * (1 << 20), __double2loint(r));
     }
     const unsigned lo = (unsigned)v, half = 1u << (sh - 1);
-    const unsigned long long m = ((unsigned long long)v + (half - 1u) + ((lo >> sh) & 1u)) >> sh;
+    const unsigned long long m = ((unsigned long long)v + (half - 1u) + ((lo >> sh) & 1u)) >> (sh & 15);   // sh is 1 .. 10
     // the leading 1 of m adds one to the exponent field
     return __longlong_as_double((long long)(m + ((unsigned long long)(unsigned)(emax - 8 + sh) << 52)));
 }
@@ -412,22 +413,28 @@ __device__ __forceinline__ bool fused_fixed(double (&n)[Q], const bool fm, const
                                             double &oy, double &oz)
 {
     const LbConst64 &K = a.K;
-    int emax = 0;
+    int emax = 0, emin = 0x7ff;
     unsigned sign = 0;
 #pragma unroll
     for (int l = 0; l < Q; ++l) {
         const unsigned hi = (unsigned)__double2hiint(n[l]);
         sign |= hi;
         emax = max(emax, (int)(hi >> 20));
+        emin = min(emin, (int)(hi >> 20));
     }
     if ((int)sign < 0 || emax >= 0x7ff || emax < 128) return false;
     long long v[Q];
+    if (emin >= emax - 7) {   // as almost always: shifts of at most 7 to the left
 #pragma unroll
-    for (int l = 0; l < Q; ++l) {
-        const unsigned hi = (unsigned)__double2hiint(n[l]), lo = (unsigned)__double2loint(n[l]);
-        const int e = (int)(hi >> 20), sh = 7 - (emax - e);
-        const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
-        v[l] = e == 0 ? 0ll : (long long)(sh >= 0 ? m << sh : m >> min(-sh, 63));
+        for (int l = 0; l < Q; ++l)
+            v[l] = (long long)(mantissa53(n[l]) << ((7 - (emax - (__double2hiint(n[l]) >> 20))) & 7));
+    } else {
+#pragma unroll
+        for (int l = 0; l < Q; ++l) {
+            const int e = __double2hiint(n[l]) >> 20, sh = 7 - (emax - e);
+            const unsigned long long m = mantissa53(n[l]);
+            v[l] = e == 0 ? 0ll : (long long)(sh >= 0 ? m << sh : m >> min(-sh, 63));
+        }
     }
     // rho in three parts that cannot overflow (each v < 2^60)
     const long long r0 = v[0] + v[1] + v[2] + v[3] + v[4] + v[5] + v[6];
@@ -594,7 +601,7 @@ __device__ __forceinline__ bool to_units(double x, int emax, long long &t)
 {
     const unsigned hi = (unsigned)__double2hiint(x);
     const int down = emax - (int)((hi >> 20) & 0x7ffu);
-    const long long m = (long long)(mantissa53(x) << ((7 - down) & 63));
+    const long long m = (long long)(mantissa53(x) << ((7 - down) & 7));   // of use for down <= 7 only
     t = (int)hi < 0 ? -m : m;
     return (unsigned)down <= 7u;
 }
