@@ -176,11 +176,12 @@ __device__ __forceinline__ void collide_strict_u(double (&n)[Q], const double rh
 // share one reciprocal.  Long division of the mantissas: with r = 2^125 / R (R, J the mantissas at bit
 // 62) the quotient's first 54 bits M = floor are those of J r / 2^64 or one off, the remainder
 // J 2^k - M R (exact modulo 2^64) puts M right, and M's last bit with the remainder rounds to nearest
-// even.  Arguments outside 2^-767 .. 2^767 in magnitude (0 apart), or a rho <= 0, are divided in FP64.
+// even.  Arguments outside 2^-500 .. 2^500 in magnitude (0 apart), or a rho <= 0, are divided in FP64:
+// within, the quotient is a normal number, as its exponent put together here must be.
 __device__ __forceinline__ bool div_range(double x)
 {
     const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-    return e - 256u < 1534u;
+    return e - 523u < 1000u;
 }
 
 __device__ __forceinline__ bool is_zero(double x)
