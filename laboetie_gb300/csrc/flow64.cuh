@@ -356,13 +356,19 @@ __device__ __forceinline__ void collide_node_fused(double (&n)[Q], const double 
 // constants of the FP64 form do not quite sum to 1 (at tau = 1 as the weights in the reference's
 // code: 1/3 + 6/18 + 12/36 = 1 - 2^-54), so a step changes a node's mass by a fixed share of it: the
 // rest population takes that too (fix_loss; 4e-13 of rho after 7000 steps, and the tracer sums
-// depend on rho).  Nodes outside the fixed-point range -- a negative or non-finite
+// depend on rho).  The axis pairs take what the diagonals leave of the flux, which a collision keeps
+// apart from the force: rounded pair by pair instead, each a sixteenth of a unit too high on average,
+// j's error against binary128 in a porous medium of 96^3 after 120 steps at tau 0.8 was 4.5e-13 of its
+// norm across the force, where the FP64 form has 1.5e-13.  Nodes outside the fixed-point range -- a
+// negative or non-finite
 // population, the largest one below 2^-895, rho from 8 times the largest one's binade up, |j| from
 // a quarter of it up, a force from a sixteenth of it up -- take the FP64 form.
 // Porous medium of 128^3 (1.26 M fluid nodes), tau 0.8: 400 -> 135 us a step (57 us of HBM traffic;
-// now bound by the integer pipes): 165 as first built, 140 in blocks of 128 threads, 135 with the
-// short shifts of the common case.  Error of j against binary128 after 120 steps of 24^3, tau 0.62 /
-// 0.8 / 1.3: 1.4e-13 / 5e-13 / 3.5e-13 of its norm where the FP64 form has 6e-13 / 8e-13 / 9e-13.
+// now bound by the integer pipes): 165 as first built, 140 in blocks of 128 threads, 134 with the
+// short shifts of the common case, 135 since the axis pairs take the rest of the flux (the loop's step 195
+// and 188).  Error of jx / jy / jz against binary128, force along x, each of its norm: porous medium of
+// 96^3, tau 0.8, 120 steps 1.2e-14 / 2.9e-14 / 3.5e-14 where the FP64 form has 5.9e-14 / 1.4e-13 /
+// 1.5e-13; 64^3, tau 0.62, 400 steps 0.6e-14 / 1.4e-14 / 1.6e-14 and 3.2e-14 / 7.8e-14 / 8.7e-14.
 
 __device__ __forceinline__ long long mulhi(long long a, long long b) { return __mul64hi(a, b); }
 
@@ -509,32 +515,52 @@ __device__ __forceinline__ bool fused_fixed(double (&n)[Q], const bool fm, const
     const long long base_axis = 2 * base;
     long long rest = R - __mulhi((int)(R >> 31), K.fix_loss);
     const bool relax = K.fix_c1 != 0;
-    // (s, d) of a pair in v[l], v[inv l] -> its collided populations; A, B to nearest, and half a
-    // unit more for the rounding down of the c1 products
-    const long long half = relax ? 8 : 4;
-    auto pair = [&](auto P, long long A, long long B) {
-        constexpr int l = pair_l(decltype(P)::value);
-        constexpr int li = inv(l);
-        long long e = (A + half) >> 3, o = (B + half) >> 3;
-        if (relax) {
-            e += mulhi(v[l] * 2, K.fix_c1);
-            o += mulhi(v[li] * 2, K.fix_c1);
-        }
-        rest -= 2 * e;
-        n[l] = fixed_to_double(e + o, emax);
-        n[li] = fixed_to_double(e - o, emax);
+    // the flux after the collision, j - (c2/2) F + c3 F with j = sum c n + F/2: what streams in and F,
+    // or the part of F that a step has whose moments or collision alone take it
+    auto flux = [&](long long sum, long long g) {
+        if constexpr (FMASK == 0) return sum;
+        if (!(fm || fc)) return sum;
+        const long long h = mulhi(4 * g, K.fix_c2);   // c2 F / 2
+        const long long G = fm ? (fc ? g : h) : g - h;
+        return sum + ((G + (((int)sum >> 3) & 7)) >> 3);
     };
-    pair(std::integral_constant<int, 0>{}, base_axis + 2 * qx, 2 * bx);
-    pair(std::integral_constant<int, 1>{}, base_axis + 2 * qy, 2 * by);
-    pair(std::integral_constant<int, 2>{}, base_axis + 2 * qz, 2 * bz);
+    // (s, d) of a pair in v[l], v[inv l] -> its collided populations e + o (+ odd) and e - o; A, B to
+    // nearest, and half a unit more for the rounding down of the c1 products
+    const long long half = relax ? 8 : 4;
+    auto even = [&](auto P, long long A) {
+        long long e = (A + half) >> 3;
+        if (relax) e += mulhi(v[pair_l(decltype(P)::value)] * 2, K.fix_c1);
+        return e;
+    };
+    auto put = [&](auto P, long long e, long long o, long long odd) {
+        constexpr int l = pair_l(decltype(P)::value);
+        rest -= 2 * e + odd;
+        n[l] = fixed_to_double(e + o + odd, emax);
+        n[inv(l)] = fixed_to_double(e - o, emax);
+    };
+    long long tx = flux(sx, gx), ty = flux(sy, gy), tz = flux(sz, gz);
+    auto diagonal = [&](auto P, long long A, long long B) {
+        constexpr int l = pair_l(decltype(P)::value);
+        constexpr Vel c = vel(l);
+        long long o = (B + half) >> 3;
+        if (relax) o += mulhi(v[inv(l)] * 2, K.fix_c1);
+        if constexpr (c.x != 0) tx -= c.x > 0 ? 2 * o : -2 * o;
+        if constexpr (c.y != 0) ty -= c.y > 0 ? 2 * o : -2 * o;
+        if constexpr (c.z != 0) tz -= c.z > 0 ? 2 * o : -2 * o;
+        put(P, even(P, A), o, 0);
+    };
+    // an axis pair takes what the diagonals leave of its flux (n_l - n_inv l = t), as soon as it is known
     const long long mxy = mulhi(ux + uy, (hx + hy) * 4), mxz = mulhi(ux + uz, (hx + hz) * 4),
                     myz = mulhi(uy + uz, (hy + hz) * 4);
-    pair(std::integral_constant<int, 3>{}, base + mxy, bx + by);                        // (1, 1, 0)
-    pair(std::integral_constant<int, 4>{}, base + 2 * (qx + qy) - mxy, by - bx);        // (-1, 1, 0)
-    pair(std::integral_constant<int, 5>{}, base + mxz, bx + bz);                        // (1, 0, 1)
-    pair(std::integral_constant<int, 6>{}, base + 2 * (qx + qz) - mxz, bz - bx);        // (-1, 0, 1)
-    pair(std::integral_constant<int, 7>{}, base + myz, by + bz);                        // (0, 1, 1)
-    pair(std::integral_constant<int, 8>{}, base + 2 * (qy + qz) - myz, bz - by);        // (0, -1, 1)
+    diagonal(std::integral_constant<int, 3>{}, base + mxy, bx + by);                        // (1, 1, 0)
+    diagonal(std::integral_constant<int, 4>{}, base + 2 * (qx + qy) - mxy, by - bx);        // (-1, 1, 0)
+    diagonal(std::integral_constant<int, 5>{}, base + mxz, bx + bz);                        // (1, 0, 1)
+    diagonal(std::integral_constant<int, 6>{}, base + 2 * (qx + qz) - mxz, bz - bx);        // (-1, 0, 1)
+    put(std::integral_constant<int, 0>{}, even(std::integral_constant<int, 0>{}, base_axis + 2 * qx), tx >> 1, tx & 1);
+    diagonal(std::integral_constant<int, 7>{}, base + myz, by + bz);                        // (0, 1, 1)
+    diagonal(std::integral_constant<int, 8>{}, base + 2 * (qy + qz) - myz, bz - by);        // (0, -1, 1)
+    put(std::integral_constant<int, 1>{}, even(std::integral_constant<int, 1>{}, base_axis + 2 * qy), ty >> 1, ty & 1);
+    put(std::integral_constant<int, 2>{}, even(std::integral_constant<int, 2>{}, base_axis + 2 * qz), tz >> 1, tz & 1);
     n[0] = fixed_to_double(rest, emax);
     return true;
 }

@@ -1,0 +1,42 @@
+"""LBGPU_FP64_FUSED keeps the momentum of a box without walls or force: what a step adds to it is the
+rounding of the populations to doubles and no drift of the fixed-point arithmetic.
+
+Bound: a step rounds the 12 diagonal populations (near 1/36, last bit 2^-58) and 6 axis ones (near 1/18,
+2^-57) of a node, each with a standard deviation of 0.29 of its last bit; a component of the flux takes 8
+and 2 of them: 0.29 2^-58 (8 + 2 4)^1/2 = 1.2 2^-58 a node and step, the populations at rest included.  Six
+standard deviations of the sum."""
+import math
+
+import numpy as np
+import pytest
+
+from laboetie_gb300 import FP64_FUSED, Box
+
+pytestmark = pytest.mark.gpu
+
+C = np.array([(0, 0, 0), (1, 0, 0), (-1, 0, 0), (0, 1, 0), (0, -1, 0), (0, 0, 1), (0, 0, -1),
+              (1, 1, 0), (-1, 1, 0), (1, -1, 0), (-1, -1, 0), (1, 0, 1), (-1, 0, 1),
+              (1, 0, -1), (-1, 0, -1), (0, 1, 1), (0, -1, 1), (0, 1, -1), (0, -1, -1)])
+W = np.array([1 / 3] + [1 / 18] * 6 + [1 / 36] * 12).reshape(19, 1, 1, 1)
+
+
+def _flux(n):
+    return [math.fsum(x for l in range(19) if C[l, d] for x in (C[l, d] * n[l]).ravel()) for d in range(3)]
+
+
+@pytest.mark.parametrize("resident", ["0", None])
+@pytest.mark.parametrize("tau", [0.8, 1.0, 0.62, 1.37])
+def test_no_drift(monkeypatch, tau, resident):
+    if resident is not None:
+        monkeypatch.setenv("LBGPU_F64_RESIDENT", resident)
+    shape, steps = (20, 22, 24), 240
+    rng = np.random.default_rng(3)
+    n0 = W * (1 + 1e-3 * rng.standard_normal((19,) + shape))
+    with Box(np.zeros(shape, dtype=np.int8), relaxation_time=tau, precision=FP64_FUSED) as box:
+        box.flow_set(n0, n0.sum(0), [np.zeros(shape)] * 3)
+        box.flow_steps(1)
+        a = _flux(box.flow_get()[0])
+        box.flow_steps(steps)
+        b = _flux(box.flow_get()[0])
+    bound = 6 * 1.2 * 2.0 ** -58 * math.sqrt(np.prod(shape) * steps)
+    assert all(abs(x - y) <= bound for x, y in zip(a, b)), [(x - y) / bound for x, y in zip(a, b)]
