@@ -343,8 +343,8 @@ __device__ __forceinline__ void collide_node_fused(double (&n)[Q], const double 
 // The FP64 pipe issues one warp instruction per 19 cycles of an SM, a 64-bit integer addition takes
 // 0.3 and the high half of a 64 x 64-bit product 4.4, and the integer pipes are otherwise idle here.
 // So the fused step of an ordinary node runs in fixed point: its populations become integers on a
-// grid 60 bits below the largest one's binade (exact while they are within 2^7 of it, and finer
-// than its rounding below), moments are exact integer sums, and each result is rounded once to a
+// grid 60 bits below the largest one's binade (exact while they are within 2^7 of it, to nearest
+// below), moments are exact integer sums, and each result is rounded once to a
 // double.  j and what is made of it carry 3 more bits, so that the rounding down of a product's high
 // half leaves no bias worth a tenth of a unit (a bias in j, unlike a random error, adds up like a
 // force).  With c at the scale of a diagonal link (a0 = 1/36, a1 = 1/12, a2 = 1/8;
@@ -440,7 +440,8 @@ __device__ __forceinline__ bool fused_fixed(double (&n)[Q], const bool fm, const
         for (int l = 0; l < Q; ++l) {
             const int e = __double2hiint(n[l]) >> 20, sh = 7 - (emax - e);
             const unsigned long long m = mantissa53(n[l]);
-            v[l] = e == 0 ? 0ll : (long long)(sh >= 0 ? m << sh : m >> min(-sh, 63));
+            const int down = min(max(-sh, 1), 62);   // to nearest: cut off, small populations would lose mass
+            v[l] = e == 0 ? 0ll : (long long)(sh >= 0 ? m << sh : (m + (1ull << (down - 1))) >> down);
         }
     }
     // rho in three parts that cannot overflow (each v < 2^60)
