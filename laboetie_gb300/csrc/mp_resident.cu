@@ -113,17 +113,18 @@ __global__ void __launch_bounds__(Real<F64>::threads, 1) k_mp_resident(const MpR
 {
     using R = typename Real<F64>::T;
     constexpr int W = Real<F64>::words;
-    // neighbour addresses [18][T]; CLUSTER: P records [2][T][W]; F64: VACF terms [warps][3][32]
+    // CLUSTER: P records [2][T + 1][W], the last one zero; neighbour addresses [18][T]; F64: VACF terms
+    // [warps][3][32]
     extern __shared__ __align__(16) unsigned char smraw[];
     const unsigned T = blockDim.x, tid = threadIdx.x, lane = tid & 31;
     const unsigned rank = blockIdx.x;   // CLUSTER: one cluster, block = rank
     const unsigned i = rank * T + tid, nwarps = gridDim.x * (T / 32), warp = i / 32;
     const bool mine = i < r.Nf;
     R *const rec = reinterpret_cast<R *>(smraw);                                  // CLUSTER
-    unsigned *const nbr = reinterpret_cast<unsigned *>(smraw + (CLUSTER ? 2 * (size_t)T * W * sizeof(R) : 0)) + tid;
+    unsigned *const nbr = reinterpret_cast<unsigned *>(smraw + (CLUSTER ? 2 * (size_t)(T + 1) * W * sizeof(R) : 0)) + tid;
     double *const terms = reinterpret_cast<double *>(nbr - tid + (size_t)18 * T) + (tid / 32) * 96;   // F64
     const unsigned rec0 = CLUSTER ? smem_addr(smraw) : 0u;
-    const unsigned flip = CLUSTER ? (unsigned)(T * W * sizeof(R)) : 0u;   // bytes between the two P buffers
+    const unsigned flip = CLUSTER ? (unsigned)((T + 1) * W * sizeof(R)) : 0u;   // bytes between the two P buffers
 
     const int lx = F64 ? r.a64.lx : r.a32.lx, ly = F64 ? r.a64.ly : r.a32.ly, lz = F64 ? r.a64.lz : r.a32.lz;
     const bool ads = F64 ? r.a64.ads != 0 : r.a32.ads != 0;
@@ -155,12 +156,22 @@ __global__ void __launch_bounds__(Real<F64>::threads, 1) k_mp_resident(const MpR
                 const float4 vn = r.a32.V[rp];
                 s[l] = mp32_scatter(blocked, r.a32.a1[wclass(l)], mp32_cdot<-c.x, -c.y, -c.z>(vn), r.a32.lwh[wclass(l)]);
             }
-            // a blocked link's probability is 0: any record will do (its own)
+            // A blocked link's probability is 0.  FP64 adds 0 times the solid node's P, as mp_f64.cu does: the
+            // zero record in a cluster, a zero in memory else (times an infinite P of its own it would add
+            // NaN).  FP32 adds 0 times a difference from its own P: its own record will do.
             if constexpr (CLUSTER) {
-                const unsigned q = blocked ? i : r.place[rp], owner = q / T;
-                nbr[(l - 1) * T] = map_rank(rec0 + (unsigned)((q - owner * T) * W * sizeof(R)), owner);
+                unsigned owner, slot;
+                if (blocked && F64) {
+                    owner = rank;
+                    slot = T;
+                } else {
+                    const unsigned q = blocked ? i : r.place[rp];
+                    owner = q / T;
+                    slot = q - owner * T;
+                }
+                nbr[(l - 1) * T] = map_rank(rec0 + (unsigned)(slot * W * sizeof(R)), owner);
             } else {
-                nbr[(l - 1) * T] = blocked ? node : rp;
+                nbr[(l - 1) * T] = blocked && !F64 ? node : rp;
             }
         });
         if constexpr (F64) {
@@ -183,10 +194,11 @@ __global__ void __launch_bounds__(Real<F64>::threads, 1) k_mp_resident(const MpR
     }
     auto put = [&](unsigned buf) {   // own P into the cluster's buffer
 #pragma unroll
-        for (int d = 0; d < 3; ++d) rec[(buf * T + tid) * W + d] = p[d];
+        for (int d = 0; d < 3; ++d) rec[(buf * (T + 1) + tid) * W + d] = p[d];
     };
     if constexpr (CLUSTER) {
         if (mine) put(0);
+        if (F64 && tid < 2 * W) rec[(tid / W * (T + 1) + T) * W + tid % W] = 0;
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     } else {
         __syncthreads();
@@ -341,7 +353,7 @@ template <bool F64, bool CLUSTER>
 size_t smem_of(unsigned T)
 {
     using R = typename Real<F64>::T;
-    return (size_t)18 * T * sizeof(unsigned) + (CLUSTER ? 2 * (size_t)T * Real<F64>::words * sizeof(R) : 0) +
+    return (size_t)18 * T * sizeof(unsigned) + (CLUSTER ? 2 * (size_t)(T + 1) * Real<F64>::words * sizeof(R) : 0) +
            (F64 ? (size_t)T / 32 * 96 * sizeof(double) : 0);
 }
 

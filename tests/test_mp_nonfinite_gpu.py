@@ -1,0 +1,34 @@
+"""A tracer whose P has left the finite numbers: the steps of many per launch give the P that one launch
+per step gives."""
+import numpy as np
+import pytest
+
+from laboetie_gb300 import FP32_DEV, FP64, Box
+
+from test_flow_resident_gpu import box_with
+
+pytestmark = pytest.mark.gpu
+
+
+def run(monkeypatch, mode, precision, nat, values):
+    monkeypatch.setenv("LBGPU_MP_RESIDENT", mode)
+    fluid = np.argwhere(nat == 0)
+    rho = np.where(nat == 0, 1.0, 0.0)
+    j = [np.where(nat == 0, v, 0.0) for v in (1e-3, 2e-3, -3e-3)]
+    with Box(nat, precision=precision) as box:
+        box.mp_init(moments=(rho, j), Db=0.02)
+        P, A = box.mp_get()
+        for q, v in zip(fluid[::37], values):
+            P[tuple(q)] = v
+        box.mp_set(P, A, it_next=1)
+        vacf, _ = box.mp_propagate(1)
+        return vacf, box.mp_get()[0]
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_DEV])
+@pytest.mark.parametrize("nf", [900, 9000])
+@pytest.mark.parametrize("values", [(np.inf,), (-np.inf, -np.inf), (np.inf, -np.inf), (np.nan,)])
+def test_same_as_one_launch_per_step(monkeypatch, precision, nf, values):
+    nat = box_with(nf, 3)
+    want, got = (run(monkeypatch, m, precision, nat, values) for m in ("0", "1"))
+    assert np.array_equal(got[1], want[1], equal_nan=True)
