@@ -86,6 +86,7 @@ __device__ __forceinline__ double ld_cluster_f64(unsigned addr)
 // Sum of one FP32 value per lane, formed exactly in integers on a grid 33 bits below the largest
 // one and rounded once; valid in every lane as (unit exponent, integer), made a double by
 // warp_exact.  (Shuffled FP64 additions: five per value and warp, each 64 cycles of its quarter.)
+// Of no use with a non-finite term (exponent 255): see warp_nonfinite_sum.
 __device__ __forceinline__ long long warp_int_sum(float v, int &emax)
 {
     const unsigned b = __float_as_uint(v);
@@ -104,8 +105,16 @@ __device__ __forceinline__ long long warp_int_sum(float v, int &emax)
 __device__ __forceinline__ double warp_exact(long long k, int emax)
 {
     const double r = (double)k;   // one unit is 2^(emax - 183)
-    if (emax == 255) return __longlong_as_double(0x7ff8000000000000ll);   // a non-finite term
     return k == 0 ? 0.0 : __hiloint2double(__double2hiint(r) + (emax - 183) * (1 << 20), __double2loint(r));
+}
+
+// The sum of values with a non-finite one among them, as FP64 additions form it; valid in every lane.
+__device__ __noinline__ double warp_nonfinite_sum(float v)
+{
+    double s = (double)v;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
 }
 
 template <bool F64, bool CLUSTER>
@@ -229,7 +238,12 @@ __global__ void __launch_bounds__(Real<F64>::threads, 1) k_mp_resident(const MpR
             long long v[3];
 #pragma unroll
             for (int d = 0; d < 3; ++d) v[d] = warp_int_sum(p[d] * us[d], e[d]);
-            if (lane < 3)
+            if (max(max(e[0], e[1]), e[2]) == 255) {
+                double w[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) w[d] = e[d] == 255 ? warp_nonfinite_sum(p[d] * us[d]) : warp_exact(v[d], e[d]);
+                if (lane < 3) out[lane] = lane == 0 ? w[0] : (lane == 1 ? w[1] : w[2]);
+            } else if (lane < 3)
                 out[lane] = warp_exact(lane == 0 ? v[0] : (lane == 1 ? v[1] : v[2]), lane == 0 ? e[0] : (lane == 1 ? e[1] : e[2]));
         }
         // ---- the step

@@ -1,5 +1,5 @@
-"""A tracer whose P has left the finite numbers: the steps of many per launch give the P that one launch
-per step gives."""
+"""A tracer whose P has left the finite numbers: the steps of many per launch give the VACF and the P that
+one launch per step gives -- an infinite term makes the sum infinite, infinities of both signs NaN."""
 import numpy as np
 import pytest
 
@@ -31,4 +31,6 @@ def run(monkeypatch, mode, precision, nat, values):
 def test_same_as_one_launch_per_step(monkeypatch, precision, nf, values):
     nat = box_with(nf, 3)
     want, got = (run(monkeypatch, m, precision, nat, values) for m in ("0", "1"))
+    assert not np.isfinite(want[0]).any()
+    assert np.array_equal(got[0], want[0], equal_nan=True)
     assert np.array_equal(got[1], want[1], equal_nan=True)
