@@ -247,8 +247,9 @@ __device__ __forceinline__ void mp_node_table(const float *__restrict__ S, const
                 pn.y = __shfl_down_sync(0xffffffffu, pn.y, 1);
                 pn.z = __shfl_down_sync(0xffffffffu, pn.z, 1);
             }
-            // a blocked link (probability 0) may keep whatever finite P the shuffle gave
-            if (!near && !((m >> inv(l)) & 1u))
+            // also where the link is blocked (probability 0): the solid node's zero, not what the shuffle
+            // gave, which another pore may have driven to NaN
+            if (!near)
                 pn = __ldg(Pn + (unsigned)((c.x < 0 ? wrap_minus(x, lx) : wrap_plus(x, lx)) + Y[c.y + 1] + Z[c.z + 1]));
         }
         mp32_link(ld_once(S + (size_t)(l - 1) * Nf + k), pn, p, n0, n1, n2);

@@ -92,3 +92,27 @@ def test_slab_tiles_of_a_dense_box(monkeypatch):
     monkeypatch.setenv("LBGPU_BATCH_SLAB", "0")
     b, _ = run([nat], steps=(2, 6))
     same(a, b, False)
+
+
+def test_a_pore_gone_nan_leaves_the_others_alone(monkeypatch):
+    """Two pores without a connection, side by side in x, so that lanes of one warp hold nodes of both: the
+    force makes the wide one's flow unstable and its tracer NaN; the narrow one's stays what it is without a
+    table."""
+    monkeypatch.setenv("LBGPU_BATCH_SMEM", "0")
+    monkeypatch.setenv("LBGPU_BATCH_SLAB", "0")
+    nat = np.ones((32, 16, 36), dtype=np.int8)
+    nat[:, :, 1] = 0
+    nat[:, :, 3:34] = 0
+    nat[::8, ::6, 18] = 1   # obstacles: no laminar flow
+    out = []
+    for budget in (0, None):
+        with Batch(memory_budget=used if budget is None else budget) as b:   # None: no room for the table
+            i = b.add(nat, f_ext=(0.0, 0.0, 2e-2), tracer=TR)
+            used = b.info()["bytes"]
+            b.steps(4000)
+            b.mp_start(i)
+            b.steps(20)
+            out.append(b.mp_fields(i))
+    for table, plain in zip(*out):
+        assert np.isnan(plain[:, :, 3]).any() and np.isfinite(plain[:, :, 1]).all()
+        assert np.array_equal(table[:, :, 1], plain[:, :, 1])
