@@ -21,6 +21,7 @@
 #include "compact.cuh"
 #include "lbgpu.h"
 #include "mp_slab.cuh"
+#include "warpsum.cuh"
 
 namespace lbg {
 namespace {
@@ -329,25 +330,19 @@ __device__ __forceinline__ void block_sum3(double (&v)[3])
         }
 }
 
-// Sum of 3 values over a block of BATCH_BLOCK threads; valid in threads 0..2, thread d its value d in
-// v[0].  A warp's 32 terms are added by an FP32 tree (5 roundings; a thread of a slab tile adds up to
-// BATCH_SLAB_ZC terms in FP32 in sequence), the warps in FP64: 5 FP64 additions per value in every
-// warp would take a third of a node tile's time (19 SM cycles each).
+// Sum of 3 values over a block of BATCH_BLOCK threads; valid in threads 0..2, thread d its value d.
+// A warp's 32 terms are added exactly in integers (warpsum.cuh), the warps in FP64.
 __device__ __forceinline__ double tile_sum3(const float (&t)[3])
 {
-    __shared__ float sh[3][BATCH_BLOCK / 32];
-    float v[3] = {t[0], t[1], t[2]};
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[d] += __shfl_down_sync(0xffffffffu, v[d], o);
-    if ((threadIdx.x & 31) == 0)
-        for (int d = 0; d < 3; ++d) sh[d][threadIdx.x >> 5] = v[d];
+    __shared__ double sh[3][BATCH_BLOCK / 32];
+    const double v = warp_sum3_exact(t);
+    const int lane = threadIdx.x & 31;
+    if (lane < 3) sh[lane][threadIdx.x >> 5] = v;
     __syncthreads();
     double s = 0.0;
     if (threadIdx.x < 3)
 #pragma unroll
-        for (int k = 0; k < BATCH_BLOCK / 32; ++k) s += (double)sh[threadIdx.x][k];
+        for (int k = 0; k < BATCH_BLOCK / 32; ++k) s += sh[threadIdx.x][k];
     return s;
 }
 
