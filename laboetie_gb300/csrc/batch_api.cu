@@ -826,19 +826,22 @@ int lbgpu_batch_add(lbgpu_batch *b, const lbgpu_cell *c, const int8_t *nature, i
     const long long units = compact ? (long long)pos.size() : N;
     // Slab tiles (mp_slab.cuh) or node tiles in the tracer phase: the same P, so a matter of speed, and
     // decided by the box alone (its VACF sums are grouped by its tiles, and a box gives the same bits
-    // in any batch).  A slab tile sweeps 16 planes in about 27 us however few tiles there are, and
-    // visits solid nodes; a node tile costs 0.04 ns per fluid node at any porosity.  us per step of
-    // 1 / 4 / 40 boxes, slab against node tiles: touching spheres 64^3 (0.32 fluid) 27 / 34 / 212
-    // against 6.3 / 14 / 144, porous 64^3 (0.60) 28 / 37 / 223 against 7.2 / 24 / 255, cylinder
-    // 96^2 x 32 (0.72) 27 / 35 / 229 against 8.6 / 29 / 329, all fluid 64^3 23 / 29 / 188 against
-    // 11 / 34 / 368.  LBGPU_BATCH_SLAB=0 / 1: node / slab tiles for every box.
+    // in any batch).  A full device costs slab tiles 0.019 ns per node of their tiles, fluid or not, and
+    // node tiles 0.041 ns per fluid node: the line at half the tiles' nodes.  A slab tile sweeps its 16
+    // planes in 17 to 20 us however few there are, so boxes of fewer than 64, which come many to a
+    // batch or are few nodes, keep node tiles.  us per step of 1 / 4 / 16 / 40 boxes, slab against node tiles:
+    // touching spheres 64^3 (0.32 of the tiles' nodes fluid) 20 / 27 / 83 / 187 against 6.6 / 15 / 61 / 144,
+    // porous 48^3 (0.45) 20 / 21 / 43 / 116 against 6.0 / 13 / 46 / 112, porous 64^3 (0.60) 22 / 29 / 90 / 202
+    // against 7.9 / 24 / 107 / 258, cylinder 64^3 (0.69) 21 / 28 / 87 / 195 against 8.0 / 28 / 114 / 274; below 64
+    // tiles, slit 32^2 x 64 (0.97) 17 / 17 / 24 / 60 against 5.0 / 11 / 35 / 92.
+    // LBGPU_BATCH_SLAB=0 / 1: node / slab tiles for every box.
     const char *slab_env = std::getenv("LBGPU_BATCH_SLAB");
     const std::string slab_mode = slab_env ? slab_env : "";
     int nslab = compact && tracer && slab_mode != "0" ? batch_slab_tiles(c->lx, c->ly, c->lz) : 0;
     sl.slab_live.clear();
     if (nslab) {   // slab tile k: column tile k % nxy (MPS_TX x MPS_TY), planes [zc (k / nxy), + zc)
         const int tx = (c->lx + MPS_TX - 1) / MPS_TX, nxy = tx * ((c->ly + MPS_TY - 1) / MPS_TY);
-        long long nodes = 0;   // lattice nodes of the live tiles
+        long long nodes = 0;   // nodes of the live tiles, those beyond the box's sides in x and y among them
         for (int k = 0; k < nslab; ++k) {
             const int t = k % nxy, x0 = (t % tx) * MPS_TX, y0 = (t / tx) * MPS_TY, z0 = (k / nxy) * BATCH_SLAB_ZC;
             const int x1 = std::min(x0 + MPS_TX, c->lx), y1 = std::min(y0 + MPS_TY, c->ly),
@@ -853,11 +856,9 @@ int lbgpu_batch_add(lbgpu_batch *b, const lbgpu_cell *c, const int8_t *nature, i
                         }
             if (!fluid) continue;
             sl.slab_live.push_back(k);
-            nodes += (long long)(x1 - x0) * (y1 - y0) * (z1 - z0);
+            nodes += (long long)MPS_TX * MPS_TY * (z1 - z0);
         }
-        const double share = (double)units / (double)nodes;
-        const size_t live = sl.slab_live.size();
-        if (slab_mode != "1" && !((share >= 0.65 && live >= 64) || (share >= 0.5 && live >= 256))) {
+        if (slab_mode != "1" && (sl.slab_live.size() < 64 || 2 * units < nodes)) {
             nslab = 0;
             sl.slab_live.clear();
         }

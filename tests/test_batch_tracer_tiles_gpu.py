@@ -116,3 +116,20 @@ def test_a_pore_gone_nan_leaves_the_others_alone(monkeypatch):
     for table, plain in zip(*out):
         assert np.isnan(plain[:, :, 3]).any() and np.isfinite(plain[:, :, 1]).all()
         assert np.array_equal(table[:, :, 1], plain[:, :, 1])
+
+
+@pytest.mark.parametrize("nat,slab", [(geo.porous_spheres(64, 8.0, 0.60, 1), True), (geo.porous_spheres(48, 8.0, 0.60, 1), False),
+                                      (geo.cc(64, 64, 64), False), (geo.slit(32, 32, 64), False)],
+                         ids=["porous64", "porous48", "spheres64", "slit32"])
+def test_tiles_by_default(monkeypatch, nat, slab):
+    """The form a box takes shows in the grouping of its VACF sums: half the nodes of its slab tiles fluid,
+    and 64 of them at least, for slab tiles."""
+    out = {}
+    for mode in ("0", "1", None):
+        if mode is None:
+            monkeypatch.delenv("LBGPU_BATCH_SLAB")
+        else:
+            monkeypatch.setenv("LBGPU_BATCH_SLAB", mode)
+        out[mode] = run([nat], steps=(2, 40))[0]
+    assert not np.array_equal(out["0"][0][0][1], out["1"][0][0][1])
+    same(out[None], out["1" if slab else "0"], True)
