@@ -499,6 +499,8 @@ int lbgpu_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int h
     if (ctx->prev_kind == PREV_NONE)
         return ctx_fail(ctx, LBGPU_ERR_INVALID, "lbgpu_equilibration: call lbgpu_flow_init first");
     if (hist_cap < 0 || (hist_cap > 0 && !l2err_hist)) return LBGPU_ERR_INVALID;
+    // the loop's control block takes the place of the one in which a wait that ran out is kept
+    if (int rc = resident_status(ctx)) return rc;
     if (ctx->p.precision == LBGPU_FP32_DEV) {
         if (ctx->d_F[0])
             return ctx_fail(ctx, LBGPU_ERR_UNSUPPORTED,
