@@ -324,6 +324,7 @@ int lbgpu_flow_init(lbgpu_ctx *ctx)
     ctx->prev_force_moment = 0;
     ctx->force_last_collide = 0;
     ctx->moments_valid = true;
+    if (int rc = resident_discard(ctx)) return rc;
     return lbgpu_sync(ctx);
 }
 
@@ -347,6 +348,7 @@ int lbgpu_flow_set(lbgpu_ctx *ctx, const double *n, const double *density, const
     ctx->prev_kind = PREV_RAW;
     ctx->prev_force_moment = ctx->force_last_collide;
     ctx->moments_valid = true;
+    if (int rc = resident_discard(ctx)) return rc;
     return lbgpu_sync(ctx);
 }
 

@@ -90,6 +90,7 @@ int f32_flow_init(lbgpu_ctx *ctx)
     ctx->prev_kind = PREV_RAW;
     ctx->prev_force_moment = 0;
     ctx->force_last_collide = 0;
+    if (int rc = resident_discard(ctx)) return rc;
     LBG_CK(ctx, cudaStreamSynchronize(ctx->stream));
     return LBGPU_OK;
 }
@@ -119,6 +120,7 @@ int f32_flow_set(lbgpu_ctx *ctx, const double *n, const double *density, const d
         ctx->aa_phase = 0;
         ctx->prev_kind = PREV_RAW;
         ctx->prev_force_moment = ctx->force_last_collide;
+        if (int rc = resident_discard(ctx)) return rc;
         LBG_CK(ctx, cudaStreamSynchronize(s));
         return LBGPU_OK;
     }
@@ -133,6 +135,14 @@ int f32_flow_set(lbgpu_ctx *ctx, const double *n, const double *density, const d
     ctx->prev_kind = PREV_RAW;
     ctx->prev_force_moment = ctx->force_last_collide;
     LBG_CK(ctx, cudaStreamSynchronize(s));
+    return LBGPU_OK;
+}
+
+int resident_discard(lbgpu_ctx *ctx)
+{
+    if (!ctx->resident_unchecked) return LBGPU_OK;
+    ctx->resident_unchecked = false;
+    LBG_CK(ctx, cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(unsigned), ctx->stream));
     return LBGPU_OK;
 }
 

@@ -28,3 +28,17 @@ def box(request, monkeypatch):
 def test_equilibration_reports_the_steps_before_it(box):
     _, _, rc = box.equilibration(max_steps=20, check=False)
     assert rc == ERR_TIMEOUT
+
+
+@pytest.mark.parametrize("how", ["init", "set"])
+def test_a_new_state_is_not_charged_with_it(box, how):
+    if how == "init":
+        box.flow_init()
+    else:
+        w = np.array([1 / 3] + [1 / 18] * 6 + [1 / 36] * 12).reshape(19, 1, 1, 1)
+        n = np.ascontiguousarray(w * (NAT == 0))
+        box.flow_set(n, n.sum(0), [np.zeros(NAT.shape)] * 3)
+    box.sync()
+    box.flow_steps(20)
+    box.sync()
+    assert np.isfinite(box.flow_get()[0]).all()
