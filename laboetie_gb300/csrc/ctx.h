@@ -120,6 +120,8 @@ void pnp_release(lbgpu_ctx *ctx);
 const double *pnp_potential(const lbgpu_ctx *ctx);
 // LBGPU_ERR_TIMEOUT if a wait of a resident launch since the last call ran out (waits for the stream)
 int resident_status(lbgpu_ctx *ctx);
+// The error of a wait that ran out: reported once, and the flow state is gone (until init or set)
+int flow_timed_out(lbgpu_ctx *ctx, const char *what);
 // Forgets them: the state that those launches left has been replaced
 int resident_discard(lbgpu_ctx *ctx);
 // A zeroed device array of n doubles for the per-step results of a call, and its return.  The

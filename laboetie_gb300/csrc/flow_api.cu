@@ -571,9 +571,8 @@ int lbgpu_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int h
     if (exec) cudaGraphExecDestroy(exec);
     if (rc) return rc;
     if (h.status & LBGPU_ERR_TIMEOUT) {
-        LBG_CK(ctx, cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(h.status), s));
         hist_return(ctx, d_hist);
-        return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, "equilibration: a block did not reach the grid's barrier within its wait limit");
+        return flow_timed_out(ctx, "equilibration");
     }
     ctx->cur = h.parity;
     ctx->prev_kind = PREV_POST;

@@ -146,6 +146,13 @@ int resident_discard(lbgpu_ctx *ctx)
     return LBGPU_OK;
 }
 
+int flow_timed_out(lbgpu_ctx *ctx, const char *what)
+{
+    ctx->prev_kind = PREV_NONE;   // some nodes are steps ahead of others
+    LBG_CK(ctx, cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(unsigned), ctx->stream));
+    return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, std::string(what) + ": a block did not reach the grid's barrier within its wait limit");
+}
+
 int resident_status(lbgpu_ctx *ctx)
 {
     if (!ctx->resident_unchecked) return LBGPU_OK;
@@ -154,8 +161,7 @@ int resident_status(lbgpu_ctx *ctx)
     LBG_CK(ctx, cudaMemcpyAsync(&st, &ctx->d_ctl->status, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
     LBG_CK(ctx, cudaStreamSynchronize(ctx->stream));
     if (!(st & LBGPU_ERR_TIMEOUT)) return LBGPU_OK;
-    LBG_CK(ctx, cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(st), ctx->stream));   // reported once
-    return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, "flow steps: a block did not reach the grid's barrier within its wait limit");
+    return flow_timed_out(ctx, "flow steps");
 }
 
 int f32_flow_get(lbgpu_ctx *ctx, double *n, double *density, double *jx, double *jy, double *jz)
@@ -408,9 +414,8 @@ int f32_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int his
     if (exec) cudaGraphExecDestroy(exec);
     if (rc) return rc;
     if (h.status & LBGPU_ERR_TIMEOUT) {
-        LBG_CK(ctx, cudaMemsetAsync(&ctx->d_ctl->status, 0, sizeof(h.status), s));
         hist_return(ctx, d_hist);
-        return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, "equilibration: a block did not reach the grid's barrier within its wait limit");
+        return flow_timed_out(ctx, "equilibration");
     }
     ctx->aa_phase = h.exit_phase;
     ctx->prev_force_moment = h.exit_force_moment;

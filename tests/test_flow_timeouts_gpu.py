@@ -42,3 +42,29 @@ def test_a_new_state_is_not_charged_with_it(box, how):
     box.flow_steps(20)
     box.sync()
     assert np.isfinite(box.flow_get()[0]).all()
+
+
+def gone(box):
+    """No call hands out or goes on from the state."""
+    for call in (box.flow_get, lambda: box.flow_steps(4), lambda: box.equilibration(max_steps=4), lambda: box.mp_init(Db=0.01)):
+        with pytest.raises(LbgpuError):
+            call()
+
+
+def test_the_state_is_gone_once_reported(box):
+    with pytest.raises(LbgpuError) as e:
+        box.flow_get()
+    assert e.value.status == ERR_TIMEOUT
+    gone(box)
+    box.flow_init()
+    box.flow_steps(20)
+    box.flow_get()
+
+
+def test_the_state_is_gone_after_a_loop(box, monkeypatch):
+    box.flow_init()
+    monkeypatch.setenv("LBGPU_TEST_GRID_WAIT", "1")
+    _, _, rc = box.equilibration(max_steps=20, check=False)
+    monkeypatch.delenv("LBGPU_TEST_GRID_WAIT")
+    assert rc == ERR_TIMEOUT
+    gone(box)
