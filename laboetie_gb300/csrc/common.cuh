@@ -5,6 +5,7 @@
 // module_lbmodel.f90:68-86,143-147.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <type_traits>
 #include <utility>
@@ -118,6 +119,16 @@ struct FlowCtl {
     unsigned status;                            // lbgpu_status bits raised on the device
     unsigned blocks_done;                       // last-block-done counter
 };
+
+// The control block as a launch leaves it, with its status bits added to those that other blocks may be
+// setting at that moment.
+__device__ __forceinline__ void store_ctl(FlowCtl *to, const FlowCtl &c)
+{
+    static_assert(offsetof(FlowCtl, err_bits) == 128 && sizeof(FlowCtl) == 256, "the shared counters' line");
+    const unsigned long long *src = reinterpret_cast<const unsigned long long *>(&c);
+    for (int k = 0; k < 16; ++k) reinterpret_cast<unsigned long long *>(to)[k] = src[k];
+    if (c.status) atomicOr(&to->status, c.status);
+}
 
 // Maximum of two values that are each non-negative or a NaN with the sign bit clear (what fabs
 // returns), taken on their IEEE bit patterns: the order of non-negative doubles is the order of

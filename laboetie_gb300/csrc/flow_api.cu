@@ -566,7 +566,7 @@ int lbgpu_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int h
             rc = ctx_cuda(ctx, e, "lbgpu_equilibration");
             break;
         }
-        if (h.done) break;
+        if (h.done || (h.status & LBGPU_ERR_TIMEOUT)) break;
     }
     if (exec) cudaGraphExecDestroy(exec);
     if (rc) return rc;

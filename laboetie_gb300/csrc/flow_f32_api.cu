@@ -409,7 +409,7 @@ int f32_equilibration(lbgpu_ctx *ctx, int max_steps, double *l2err_hist, int his
             break;
         }
         phase = h.exit_phase;
-        if (h.done) break;
+        if (h.done || (h.status & LBGPU_ERR_TIMEOUT)) break;
     }
     if (exec) cudaGraphExecDestroy(exec);
     if (rc) return rc;

@@ -299,13 +299,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_aa_resident(const ResidentAr
             a.jy[p] = jy;
             a.jz[p] = jz;
         }
-        if (rank == 0 && tid == 0) {
-            if (!ok) {
-                ctl.status |= (unsigned)LBGPU_ERR_TIMEOUT;
-                ctl.done = 1;
-            }
-            *a.ctl = ctl;
-        }
+        if (rank == 0 && tid == 0) store_ctl(a.ctl, ctl);
     }
     if constexpr (CLUSTER) {
         cluster_barrier();   // a block's shared memory holds its nodes' populations
@@ -313,7 +307,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1) k_aa_resident(const ResidentAr
 #pragma unroll
             for (int l = 0; l < Q; ++l) a.g0[(size_t)l * a.Nf + i] = s.own[l * T];
         }
-    } else if (!LOOP && !ok && tid == 0) {
+    } else if (!ok && tid == 0) {
         atomicOr(&a.ctl->status, (unsigned)LBGPU_ERR_TIMEOUT);
     }
 }
@@ -417,12 +411,7 @@ size_t grid_sync_bytes() { return sizeof(GridSync); }
 
 static cudaError_t run(const ResidentPlan &plan, ResidentArgs &r, void *sync, bool loop, cudaStream_t s)
 {
-    // LBGPU_TEST_GRID_WAIT=1 (tests only): the grid waits for one block more than it has, so its
-    // bounded waits (50 ms then) run out without any fault
-    const char *env = std::getenv("LBGPU_TEST_GRID_WAIT");
-    const bool test = env && std::string(env) == "1";
-    r.wait.limit_ns = test ? 50000000ull : 2000000000ull;
-    r.wait.extra = test ? 1u : 0u;
+    r.wait = grid_wait();
     r.sync = static_cast<GridSync *>(sync);
     if (plan.cluster) return loop ? launch<true, true>(plan, r, s) : launch<true, false>(plan, r, s);
     const cudaError_t e = cudaMemsetAsync(sync, 0, sizeof(GridSync), s);

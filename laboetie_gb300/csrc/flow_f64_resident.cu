@@ -201,16 +201,9 @@ __global__ void __launch_bounds__(SPLIT ? 128 : RT, 1) k_flow64_resident(const R
                 for (int d = 0; d < 3; ++d) J[d][node] = jold[d];
             }
         }
-        if (blockIdx.x == 0 && tid == 0) {
-            if (!ok) {
-                ctl.status |= (unsigned)LBGPU_ERR_TIMEOUT;
-                ctl.done = 1;
-            }
-            *a.ctl = ctl;
-        }
-    } else if (!ok && tid == 0) {
-        atomicOr(&a.ctl->status, (unsigned)LBGPU_ERR_TIMEOUT);
+        if (blockIdx.x == 0 && tid == 0) store_ctl(a.ctl, ctl);
     }
+    if (!ok && tid == 0) atomicOr(&a.ctl->status, (unsigned)LBGPU_ERR_TIMEOUT);
 }
 
 using Kernel = void (*)(ResidentArgs64);
@@ -268,10 +261,7 @@ cudaError_t launch_resident64(const ResidentPlan &plan, const FlowArgs64 &a, int
     std::memset(&r, 0, sizeof(r));
     r.a = a;
     r.sync = static_cast<GridSync *>(sync);
-    const char *env = std::getenv("LBGPU_TEST_GRID_WAIT");   // tests: see flow_f32_resident.cu
-    const bool test = env && std::strcmp(env, "1") == 0;
-    r.wait.limit_ns = test ? 50000000ull : 2000000000ull;
-    r.wait.extra = test ? 1u : 0u;
+    r.wait = grid_wait();
     r.nsteps = nsteps;
     r.loop = loop ? 1 : 0;
     r.fon = fon;

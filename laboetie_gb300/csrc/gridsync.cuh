@@ -4,12 +4,15 @@
 // Thread 0 of a block adds the block's values to the round's slot, arrives on a counter (release)
 // and polls it (acquire) until every block has arrived.  The three slots rotate: after a round has
 // passed, the slot of the round before it is read by nobody any more and is cleared for the round
-// after next.  The poll is bounded; a block whose wait runs out reports it and the kernel ends.
+// after next.  The poll is bounded.  A block whose wait runs out says so in `failed`, which the waits of
+// the others read, so that they end too; each such block reports it to the host itself, as the others
+// may all have passed the launch's last rendezvous.
 // 152 blocks: 1.2 us without values, 1.6 us with them (a launch in a CUDA graph costs 1.04 us, and
 // a step that decides on a reduction needs its tail besides).
 #pragma once
 
 #include <cstdint>
+#include <cstdlib>
 
 #include "tma.cuh"
 
@@ -21,14 +24,30 @@ struct alignas(128) GridSync {
         unsigned bits;
     } slot[3];
     alignas(128) unsigned arrived;
+    alignas(128) unsigned failed;
 };
 
-// How a launch waits: the limit of each wait, and arrivals to wait for beyond the grid's own (0; a
-// test sets 1, so that the wait runs out without any fault).
+// How a launch waits: the limit of each wait, and for tests, so that waits run out without any fault,
+// arrivals to wait for beyond the grid's own (0) and the rendezvous, counted from 1, at which the last
+// block takes its wait as run out although all have arrived (0: none).
 struct GridWait {
     unsigned long long limit_ns;
     unsigned extra;
+    unsigned give_up;
 };
+
+// LBGPU_TEST_GRID_WAIT (tests only): 1: every wait runs out, after 50 ms; k > 1: the last block gives up at
+// the rendezvous k - 1.
+inline GridWait grid_wait()
+{
+    const char *env = std::getenv("LBGPU_TEST_GRID_WAIT");
+    const int test = env ? std::atoi(env) : 0;
+    GridWait w;
+    w.limit_ns = test > 0 ? 50000000ull : 2000000000ull;
+    w.extra = test == 1 ? 1u : 0u;
+    w.give_up = test > 1 ? (unsigned)(test - 1) : 0u;
+    return w;
+}
 
 __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p)
 {
@@ -84,9 +103,11 @@ __device__ __forceinline__ bool grid_barrier(GridSync *g, unsigned round, const 
             if ((it & 255u) == 255u) {
                 const unsigned long long t = global_ns();
                 if (t0 == 0) t0 = t;
-                else if (t - t0 > wait.limit_ns) break;
+                else if (t - t0 > wait.limit_ns || ld_acquire_gpu(&g->failed)) break;
             }
         }
+        if (wait.give_up == round + 1u && blockIdx.x == gridDim.x - 1u) done = false;
+        if (!done) atomicExch(&g->failed, 1u);
         if constexpr (VALUES) {
             rval = __ldcg(&s->value);
             rbit = __ldcg(&s->bits);

@@ -437,10 +437,7 @@ cudaError_t launch_mp_resident(const MpResident &m, const MpArgs64 *a64, const M
     std::memset(&r, 0, sizeof(r));
     if (a64) r.a64 = *a64;
     else r.a32 = *a32;
-    const char *env = std::getenv("LBGPU_TEST_GRID_WAIT");   // tests: see flow_f32_resident.cu
-    const bool test = env && std::strcmp(env, "1") == 0;
-    r.wait.limit_ns = test ? 50000000ull : 2000000000ull;
-    r.wait.extra = test ? 1u : 0u;
+    r.wait = grid_wait();
     r.sync = static_cast<GridSync *>(m.sync);
     r.fidx = m.fidx;
     r.place = m.place;

@@ -66,8 +66,8 @@ struct PnpLoop {
     int total;               // sum of the solves' sweep counts (iter - 1 each)
     int outer, equilibrium;  // outer iterations; the convergence test was met
     int converged, done;     // last solve converged; nothing left to do
-    unsigned status;
     double limit, anormf0;   // stopping value of the solve under way, SUM(ABS(phi)) of the last one
+    unsigned status;         // last: bits are added to it, the rest is stored by block 0
 };
 
 struct PnpResidentArgs {

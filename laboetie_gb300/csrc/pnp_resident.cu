@@ -176,10 +176,7 @@ __global__ void __launch_bounds__(RT, 1) k_pnp_resident(const PnpResidentArgs r)
     }
     if (tid == 0) L = *r.loop;
     if (!grid.barrier()) {
-        if (tid == 0 && blockIdx.x == 0) {
-            r.loop->status = LBGPU_ERR_TIMEOUT;
-            r.loop->done = 1;
-        }
+        if (tid == 0) atomicOr(&r.loop->status, (unsigned)LBGPU_ERR_TIMEOUT);
         return;
     }
     // values at the start of the outer iteration (kept across launches in r.bak)
@@ -388,12 +385,13 @@ __global__ void __launch_bounds__(RT, 1) k_pnp_resident(const PnpResidentArgs r)
         __syncthreads();
         if (sh.ok) break;
     }
-    if (tid == 0 && blockIdx.x == 0) {
-        if (!ok) {
-            L.status |= LBGPU_ERR_TIMEOUT;
-            L.done = 1;
+    if (tid == 0) {
+        if (!ok) atomicOr(&r.loop->status, (unsigned)LBGPU_ERR_TIMEOUT);
+        if (blockIdx.x == 0) {
+            constexpr int WORDS = (int)(offsetof(PnpLoop, status) / sizeof(unsigned));
+            for (int k = 0; k < WORDS; ++k) reinterpret_cast<unsigned *>(r.loop)[k] = reinterpret_cast<unsigned *>(&L)[k];
+            if (L.status) atomicOr(&r.loop->status, L.status);
         }
-        *r.loop = L;
     }
 }
 
@@ -426,10 +424,7 @@ PnpResidentPlan plan_pnp_resident(long long N)
 
 cudaError_t launch_pnp_resident(const PnpResidentPlan &plan, PnpResidentArgs &r, cudaStream_t s)
 {
-    const char *env = std::getenv("LBGPU_TEST_GRID_WAIT");   // tests: see flow_f32_resident.cu
-    const bool test = env && std::strcmp(env, "1") == 0;
-    r.wait.limit_ns = test ? 50000000ull : 2000000000ull;
-    r.wait.extra = test ? 1u : 0u;
+    r.wait = grid_wait();
     cudaError_t e = cudaMemsetAsync(r.sync, 0, sizeof(GridSync), s);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t c = {};

@@ -1,0 +1,68 @@
+"""One block of a many-step launch gives up at a rendezvous that all the others pass
+(LBGPU_TEST_GRID_WAIT=k: the last block, at the rendezvous k - 1), the launch's last one or an earlier one:
+the call reports it, although the first block, which writes the control block, has seen nothing."""
+import math
+
+import numpy as np
+import pytest
+
+from laboetie_gb300 import FP32_DEV, FP64, FP64_FUSED, Box, LbgpuError
+from laboetie_gb300 import geometry as geo
+
+pytestmark = pytest.mark.gpu
+
+ERR_TIMEOUT = 1 << 10
+NAT = geo.slit(4, 4, 64)
+KW = dict(f_ext=(1e-5, 0.0, 0.0))
+# rendezvous of a loop of two steps: FP64 one a step; FP32 one more before the first
+LAST = {FP64: 2, FP64_FUSED: 2, FP32_DEV: 3}
+
+
+@pytest.mark.parametrize("precision", [FP64, FP64_FUSED, FP32_DEV])
+@pytest.mark.parametrize("back", [0, 1])
+def test_loop(monkeypatch, precision, back):
+    monkeypatch.setenv("LBGPU_AA_RESIDENT", "grid")
+    with Box(NAT, precision=precision, **KW) as box:
+        box.flow_init()
+        monkeypatch.setenv("LBGPU_TEST_GRID_WAIT", str(LAST[precision] - back + 1))
+        _, _, rc = box.equilibration(max_steps=2, check=False)
+        assert rc == ERR_TIMEOUT
+        monkeypatch.setenv("LBGPU_TEST_GRID_WAIT", str(LAST[precision] + 2))   # beyond the last: nothing
+        box.flow_init()
+        steps, _, rc = box.equilibration(max_steps=2, check=False)
+        assert rc != ERR_TIMEOUT and steps == 2
+
+
+@pytest.mark.parametrize("precision", [FP64, FP64_FUSED, FP32_DEV])
+def test_fixed_steps(monkeypatch, precision):
+    monkeypatch.setenv("LBGPU_AA_RESIDENT", "grid")
+    with Box(NAT, precision=precision, **KW) as box:
+        box.flow_init()
+        monkeypatch.setenv("LBGPU_TEST_GRID_WAIT", "20")   # 20 steps have 19 rendezvous
+        box.flow_steps(20)
+        with pytest.raises(LbgpuError) as e:
+            box.sync()
+        assert e.value.status == ERR_TIMEOUT
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_DEV])
+def test_tracer(monkeypatch, precision):
+    monkeypatch.setenv("LBGPU_MP_RESIDENT", "grid")
+    rho = np.where(NAT == 0, 1.0, 0.0)
+    with Box(NAT, precision=precision) as box:
+        box.mp_init(moments=(rho, [0.0 * rho] * 3), Db=0.01, ka=0.01 * math.e, kd=0.01)
+        monkeypatch.setenv("LBGPU_TEST_GRID_WAIT", "20")
+        with pytest.raises(LbgpuError) as e:
+            box.mp_propagate(20)
+        assert e.value.status == ERR_TIMEOUT
+
+
+@pytest.mark.parametrize("at", [1, 2, 5, 30])
+def test_charges(monkeypatch, at):
+    nat = geo.cc(16, 16, 16)
+    with Box(nat) as box:
+        box.pnp_init(bjl=0.4, sigma=-1.0, lambda_D=4.0, D_plus=0.05, D_minus=0.05)
+        monkeypatch.setenv("LBGPU_TEST_GRID_WAIT", str(at + 1))
+        with pytest.raises(LbgpuError) as e:
+            box.sor()
+        assert e.value.status == ERR_TIMEOUT
