@@ -38,6 +38,7 @@ struct MpState {
     int it_next = 1;
     int converged = 0;
     unsigned pending = 0;  // error raised at init, reported by the first propagate
+    bool lost = false;     // a wait of a many-step launch ran out: P is not that of any step
     double vacf0[3] = {0, 0, 0};
 };
 
@@ -361,6 +362,13 @@ int mp_init_impl(lbgpu_ctx *ctx, const lbgpu_tracer *tr, const double *density, 
 
 extern "C" {
 
+static int mp_lost(lbgpu_ctx *ctx)
+{
+    return ctx_fail(ctx, LBGPU_ERR_TIMEOUT,
+                    "moment propagation: a block did not reach the grid's barrier within its wait limit (its state is lost: "
+                    "call lbgpu_mp_init or lbgpu_mp_set)");
+}
+
 // The steps of mp_run as resident launches: `c` is the control block as the call starts (its
 // thresholds set).  A launch that meets the convergence test before its last step is repeated up to
 // that step from the P it started from.
@@ -371,19 +379,21 @@ static int mp_run_resident(lbgpu_ctx *ctx, MpCtl &c, int nsteps, double *vacf_ou
     const MpArgs64 *a64 = s->prec == LBGPU_FP64 ? &s->a64 : nullptr;
     const MpArgs32 *a32 = a64 ? nullptr : &s->a32;
     std::vector<double> rows((size_t)3 * std::min(nsteps, s->res.max_steps));
-    unsigned failed = 0;
     int done = 0;
+    // n steps; VACF of each in rows, if asked for
+    auto launch = [&](int n, bool want) -> int {
+        unsigned failed = 0;
+        LBG_CK(ctx, launch_mp_resident(s->res, a64, a32, c.parity, n, s->res_vacf, st));
+        if (want) LBG_CK(ctx, cudaMemcpyAsync(rows.data(), s->res_vacf, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st));
+        LBG_CK(ctx, cudaMemcpyAsync(&failed, s->res.failed, sizeof(failed), cudaMemcpyDeviceToHost, st));
+        LBG_CK(ctx, cudaStreamSynchronize(st));
+        s->lost = failed != 0;
+        return failed ? mp_lost(ctx) : LBGPU_OK;
+    };
     if (timing) LBG_CK(ctx, cudaEventRecord(ctx->ev0, st));
     while (done < nsteps && !c.converged) {
         int n = std::min(nsteps - done, s->res.max_steps);
-        LBG_CK(ctx, launch_mp_resident(s->res, a64, a32, c.parity, n, s->res_vacf, st));
-        LBG_CK(ctx, cudaMemcpyAsync(rows.data(), s->res_vacf, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st));
-        LBG_CK(ctx, cudaMemcpyAsync(&failed, s->res.failed, sizeof(failed), cudaMemcpyDeviceToHost, st));
-        LBG_CK(ctx, cudaStreamSynchronize(st));
-        if (failed) {
-            c.status |= LBGPU_ERR_TIMEOUT;
-            return LBGPU_OK;
-        }
+        if (int rc = launch(n, true)) return rc;
         for (int k = 0; k < n && !c.converged; ++k) {
             bool conv = c.it + k > 2;
             for (int d = 0; d < 3; ++d) {
@@ -394,7 +404,7 @@ static int mp_run_resident(lbgpu_ctx *ctx, MpCtl &c, int nsteps, double *vacf_ou
             c.converged = 1;
             if (k + 1 < n) {
                 n = k + 1;
-                LBG_CK(ctx, launch_mp_resident(s->res, a64, a32, c.parity, n, s->res_vacf, st));
+                if (int rc = launch(n, false)) return rc;
             }
         }
         if (vacf_out) std::memcpy(vacf_out + 3 * (size_t)done, rows.data(), sizeof(double) * 3 * n);
@@ -423,6 +433,7 @@ static int mp_run(lbgpu_ctx *ctx, int nsteps, double *vacf_out, int *steps_done,
     if (!s) return ctx_fail(ctx, LBGPU_ERR_INVALID, "moment propagation: call lbgpu_mp_init first");
     if (s->pending)
         return ctx_fail(ctx, LBGPU_ERR_FRACTION, "somewhere restpart is negative");
+    if (s->lost) return mp_lost(ctx);
     if (steps_done) *steps_done = 0;
     if (is_converged) *is_converged = s->converged;
     if (nsteps <= 0) return LBGPU_OK;
@@ -446,9 +457,6 @@ static int mp_run(lbgpu_ctx *ctx, int nsteps, double *vacf_out, int *steps_done,
     }
     if (s->res.plan.blocks) {
         if (int rc = mp_run_resident(ctx, c, nsteps, vacf_out, timing, ms)) return rc;
-        if (c.status & LBGPU_ERR_TIMEOUT)
-            return ctx_fail(ctx, LBGPU_ERR_TIMEOUT,
-                            "moment propagation: a block did not reach the grid's barrier within its wait limit");
         s->it_next = c.last_it + 1;
         s->converged = c.converged;
         if (steps_done) *steps_done = c.last_it - c.it_base + 1;
@@ -538,6 +546,7 @@ int lbgpu_mp_get(lbgpu_ctx *ctx, double *P, double *P_ads)
     if (!ctx) return LBGPU_ERR_INVALID;
     MpState *s = ctx->mp;
     if (!s) return ctx_fail(ctx, LBGPU_ERR_INVALID, "lbgpu_mp_get: no moment propagation state");
+    if (s->lost) return mp_lost(ctx);
     const long long N = ctx->N;
     cudaStream_t st = ctx->stream;
     MpCtl c;
@@ -578,6 +587,7 @@ int lbgpu_mp_set(lbgpu_ctx *ctx, const double *P, const double *P_ads, int it_ne
     }
     s->it_next = it_next;
     s->converged = 0;
+    s->lost = false;
     return LBGPU_OK;
 }
 

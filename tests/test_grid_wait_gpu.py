@@ -66,3 +66,30 @@ def test_charges(monkeypatch, at):
         with pytest.raises(LbgpuError) as e:
             box.sor()
         assert e.value.status == ERR_TIMEOUT
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_DEV])
+@pytest.mark.parametrize("wait", ["1", "20"])
+def test_a_lost_tracer_state_stays_lost(monkeypatch, precision, wait):
+    """Neither steps nor results of it until the state is set or formed anew."""
+    monkeypatch.setenv("LBGPU_MP_RESIDENT", "grid")
+    rho = np.where(NAT == 0, 1.0, 0.0)
+    tr = dict(moments=(rho, [0.0 * rho] * 3), Db=0.01, ka=0.01 * math.e, kd=0.01)
+    with Box(NAT, precision=precision) as box:
+        box.mp_init(**tr)
+        box.mp_propagate(5)
+        state = box.mp_get()
+        box.mp_propagate(20)
+        want = box.mp_get()
+        for again in (lambda: box.mp_set(*state, it_next=6), lambda: (box.mp_init(**tr), box.mp_propagate(5))):
+            monkeypatch.setenv("LBGPU_TEST_GRID_WAIT", wait)
+            with pytest.raises(LbgpuError):
+                box.mp_propagate(20)
+            monkeypatch.delenv("LBGPU_TEST_GRID_WAIT")
+            for call in (lambda: box.mp_propagate(3), box.mp_get, lambda: box.time_mp_steps(3)):
+                with pytest.raises(LbgpuError) as e:
+                    call()
+                assert e.value.status == ERR_TIMEOUT
+            again()
+            box.mp_propagate(20)
+            assert all(np.array_equal(x, y) for x, y in zip(box.mp_get(), want))
