@@ -322,7 +322,7 @@ int need_charges(lbgpu_ctx *ctx, const char *fn)
 {
     if (!ctx->pnp)
         return ctx_fail(ctx, LBGPU_ERR_INVALID, std::string(fn) + ": call lbgpu_pnp_init (or lbgpu_pnp_set) first");
-    return LBGPU_OK;
+    return ctx->pnp->lost ? pnp_lost(ctx) : LBGPU_OK;
 }
 
 int alloc_zero(lbgpu_ctx *ctx, double **p, size_t n)

@@ -37,7 +37,14 @@ constexpr double PI_D = 3.141592653589793;   // acos(-1.0_dp), module_constants.
 
 const double *pnp_potential(const lbgpu_ctx *ctx)
 {
-    return ctx->pnp ? ctx->pnp->phi[ctx->pnp->par] : nullptr;
+    return ctx->pnp && !ctx->pnp->lost ? ctx->pnp->phi[ctx->pnp->par] : nullptr;
+}
+
+int pnp_lost(lbgpu_ctx *ctx)
+{
+    return ctx_fail(ctx, LBGPU_ERR_TIMEOUT,
+                    "Poisson-Nernst-Planck: a block did not reach the grid's barrier within its wait limit (the state is lost: "
+                    "call lbgpu_pnp_init or lbgpu_pnp_set)");
 }
 
 void pnp_release(lbgpu_ctx *ctx)
@@ -563,7 +570,7 @@ int need_pnp(lbgpu_ctx *ctx, const char *fn)
 {
     if (!ctx->pnp)
         return ctx_fail(ctx, LBGPU_ERR_INVALID, std::string(fn) + ": call lbgpu_pnp_init first");
-    return LBGPU_OK;
+    return ctx->pnp->lost ? pnp_lost(ctx) : LBGPU_OK;
 }
 
 }  // namespace
@@ -673,8 +680,7 @@ int lbgpu_pnp_set(lbgpu_ctx *ctx, const double *c_plus, const double *c_minus, c
                   double anormf0)
 {
     if (!ctx || !c_plus || !c_minus || !phi) return LBGPU_ERR_INVALID;
-    int rc = need_pnp(ctx, "lbgpu_pnp_set");
-    if (rc) return rc;
+    if (!ctx->pnp) return need_pnp(ctx, "lbgpu_pnp_set");
     PnpState *s = ctx->pnp;
     const size_t b = sizeof(double) * ctx->N;
     LBG_CK(ctx, cudaMemcpyAsync(s->cp, c_plus, b, cudaMemcpyHostToDevice, ctx->stream));
@@ -682,6 +688,7 @@ int lbgpu_pnp_set(lbgpu_ctx *ctx, const double *c_plus, const double *c_minus, c
     LBG_CK(ctx, cudaMemcpyAsync(s->phi[s->par], phi, b, cudaMemcpyHostToDevice, ctx->stream));
     s->anormf0 = anormf0;
     s->charged = true;
+    s->lost = false;
     return lbgpu_sync(ctx);
 }
 
@@ -755,9 +762,8 @@ static int run_resident(lbgpu_ctx *ctx, const PnpArgs &a, const PnpCtl &c, int m
         LBG_CK(ctx, cudaMemcpyAsync(&h, s->loop, sizeof(h), cudaMemcpyDeviceToHost, st));
         LBG_CK(ctx, cudaStreamSynchronize(st));
     } while (!h.done && !(h.status & LBGPU_ERR_TIMEOUT));
-    if (h.status & LBGPU_ERR_TIMEOUT)
-        return ctx_fail(ctx, LBGPU_ERR_TIMEOUT, "Poisson-Nernst-Planck: a block did not reach the grid's barrier within its wait limit");
-    return LBGPU_OK;
+    s->lost = (h.status & LBGPU_ERR_TIMEOUT) != 0;
+    return s->lost ? pnp_lost(ctx) : LBGPU_OK;
 }
 
 int lbgpu_sor(lbgpu_ctx *ctx, int *iters)

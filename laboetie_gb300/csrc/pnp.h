@@ -31,6 +31,7 @@ struct PnpResidentArgs;
 struct PnpLoop;
 struct GridSync;
 PnpResidentPlan plan_pnp_resident(long long N);
+int pnp_lost(lbgpu_ctx *ctx);   // the error of such a state
 size_t pnp_resident_partials(unsigned blocks);   // doubles of PnpResidentArgs::partial
 cudaError_t launch_pnp_resident(const PnpResidentPlan &plan, PnpResidentArgs &r, cudaStream_t s);
 
@@ -48,6 +49,7 @@ struct PnpState {
     int par = 0;                            // buffer holding phi
     double anormf0 = 0.0, rho_ch = 0.0;
     bool charged = false;
+    bool lost = false;                      // a wait of the resident loop ran out: phi, c+- are of no sweep
     KeptAllocs allocs;
     PnpResidentPlan resident{};             // with its own buffers:
     GridSync *gsync = nullptr;

@@ -93,3 +93,32 @@ def test_a_lost_tracer_state_stays_lost(monkeypatch, precision, wait):
             again()
             box.mp_propagate(20)
             assert all(np.array_equal(x, y) for x, y in zip(box.mp_get(), want))
+
+
+@pytest.mark.parametrize("wait", ["1", "12"])
+@pytest.mark.parametrize("loop", [True, False])
+def test_a_lost_charge_state_stays_lost(monkeypatch, wait, loop):
+    nat = geo.cc(16, 16, 16)
+    charges = dict(bjl=0.4, sigma=-1.0, lambda_D=4.0, D_plus=0.05, D_minus=0.05)
+    with Box(nat) as box:
+        box.pnp_init(**charges)
+        state = box.pnp_get()
+        box.sor()
+        want = box.pnp_get()
+        for again in (lambda: box.pnp_set(*state), lambda: box.pnp_init(**charges)):
+            box.pnp_set(*state)
+            monkeypatch.setenv("LBGPU_TEST_GRID_WAIT", wait)
+            with pytest.raises(LbgpuError):
+                box.poisson_nernst_planck(max_outer=3) if loop else box.sor()
+            monkeypatch.delenv("LBGPU_TEST_GRID_WAIT")
+            for call in (box.pnp_get, box.sor, box.just_eq_smolu, box.poisson_residual, box.electrostatic_pot,
+                         lambda: box.poisson_nernst_planck(max_outer=2)):
+                with pytest.raises(LbgpuError) as e:
+                    call()
+                assert e.value.status == ERR_TIMEOUT
+            with pytest.raises(LbgpuError):
+                box.mp_init(moments=(np.where(nat == 0, 1.0, 0.0), [np.zeros(nat.shape)] * 3), Db=0.01, z=1.0, charged=True)
+            again()
+            box.sor()
+            got = box.pnp_get()
+            assert all(np.array_equal(x, y) for x, y in zip(got[:3], want[:3])) and got[3] == want[3]
