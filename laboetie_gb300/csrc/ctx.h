@@ -118,6 +118,8 @@ void mp_release(lbgpu_ctx *ctx);
 void pnp_release(lbgpu_ctx *ctx);
 // device potential phi of the Poisson-Nernst-Planck state (N doubles), or null without one
 const double *pnp_potential(const lbgpu_ctx *ctx);
+// waits for the stream, for calls that have nothing to do with the flow state (lbgpu_sync reports its timeouts)
+int stream_wait(lbgpu_ctx *ctx, const char *what);
 // LBGPU_ERR_TIMEOUT if a wait of a resident launch since the last call ran out (waits for the stream)
 int resident_status(lbgpu_ctx *ctx);
 // The error of a wait that ran out: reported once, and the flow state is gone (until init or set)

@@ -359,7 +359,7 @@ int lbgpu_electrostatic_pot(lbgpu_ctx *ctx, const double elec_slope[3])
     k_ek_pot<<<blocks(ctx->N), EB, 0, ctx->stream>>>(s->phi[s->par], s->phi_tot, ctx->N, ctx->p.lx, ctx->p.ly,
                                                      elec_slope[0], elec_slope[1], elec_slope[2], zero);
     LBG_CK(ctx, cudaGetLastError());
-    return lbgpu_sync(ctx);
+    return stream_wait(ctx, "lbgpu_electrostatic_pot");
 }
 
 int lbgpu_comp_j(lbgpu_ctx *ctx, const double *n, double *jx, double *jy, double *jz)
@@ -555,7 +555,7 @@ int lbgpu_ek_get(lbgpu_ctx *ctx, double *phi_tot, double *solute_force)
         else
             std::memset(solute_force, 0, sizeof(double) * 3 * N);
     }
-    return lbgpu_sync(ctx);
+    return stream_wait(ctx, "lbgpu_ek_get");
 }
 
 }  // extern "C"

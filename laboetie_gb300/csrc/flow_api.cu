@@ -210,6 +210,8 @@ int hist_take(lbgpu_ctx *ctx, size_t n, double **p)
     return LBGPU_OK;
 }
 
+int stream_wait(lbgpu_ctx *ctx, const char *what) { return ctx_cuda(ctx, cudaStreamSynchronize(ctx->stream), what); }
+
 void hist_return(lbgpu_ctx *ctx, double *p)
 {
     if (p && p != ctx->d_hist) cudaFreeAsync(p, ctx->stream);
@@ -428,7 +430,7 @@ int lbgpu_collide(lbgpu_ctx *ctx, double *n, const double *density, const double
     a.force_collide = 1;
     LBG_CK(ctx, launch_collide_f64(a, 7, true, s));
     LBG_CK(ctx, cudaMemcpyAsync(n, ob->n[1], sizeof(double) * Q * N, cudaMemcpyDeviceToHost, s));
-    return lbgpu_sync(ctx);
+    return stream_wait(ctx, "lbgpu_collide");
 }
 
 int lbgpu_bounce_back_stream(lbgpu_ctx *ctx, double *n)
@@ -449,7 +451,7 @@ int lbgpu_bounce_back_stream(lbgpu_ctx *ctx, double *n)
     a.nout = ob->n[1];
     LBG_CK(ctx, launch_stream_f64(a, s));
     LBG_CK(ctx, cudaMemcpyAsync(n, ob->n[1], sizeof(double) * Q * N, cudaMemcpyDeviceToHost, s));
-    return lbgpu_sync(ctx);
+    return stream_wait(ctx, "lbgpu_bounce_back_stream");
 }
 
 int lbgpu_moments(lbgpu_ctx *ctx, const double *n, const double *f_ext_x, const double *f_ext_y,

@@ -138,7 +138,7 @@ int lbgpu_set_force_field(lbgpu_ctx *ctx, const double *fx, const double *fy, co
         if (!ctx->d_F[d]) LBG_CK(ctx, cudaMalloc((void **)&ctx->d_F[d], sizeof(double) * ctx->N));
         LBG_CK(ctx, cudaMemcpyAsync(ctx->d_F[d], h[d], sizeof(double) * ctx->N, cudaMemcpyHostToDevice, ctx->stream));
     }
-    return lbgpu_sync(ctx);
+    return stream_wait(ctx, "lbgpu_set_force_field");
 }
 
 }  // extern "C"

@@ -632,14 +632,14 @@ int lbgpu_pnp_init(lbgpu_ctx *ctx, const lbgpu_pnp_params *p, double *anormf0)
     // charges_init.f90:23-135 on the host, node by node in the reference's order
     if (p->bjl <= eps) {                       // :25 no charge at all
         if (anormf0) *anormf0 = 0.0;
-        return lbgpu_sync(ctx);
+        return stream_wait(ctx, "lbgpu_pnp_init");
     }
     const double pi = PI_D, kBT = 1.0 / 3.0;
     double rho_0 = std::fabs(p->lambda_D) <= eps ? 0.0 : 1.0 / (4.0 * pi * p->bjl * (p->lambda_D * p->lambda_D));
     s->rho_ch = 1.0 / (4.0 * pi * p->bjl * (p->lambda_D * p->lambda_D));
     if (!(std::fabs(p->sigma) > eps)) {
         if (anormf0) *anormf0 = 0.0;
-        return lbgpu_sync(ctx);
+        return stream_wait(ctx, "lbgpu_pnp_init");
     }
     if (p->charge_distrib != 0)                // 'sol' stops the reference (charges_init.f90:96-100)
         return ctx_fail(ctx, LBGPU_ERR_UNSUPPORTED, "only surface charge is implemented for now in charge_init.f90");
@@ -689,7 +689,7 @@ int lbgpu_pnp_set(lbgpu_ctx *ctx, const double *c_plus, const double *c_minus, c
     s->anormf0 = anormf0;
     s->charged = true;
     s->lost = false;
-    return lbgpu_sync(ctx);
+    return stream_wait(ctx, "lbgpu_pnp_set");
 }
 
 int lbgpu_pnp_get(lbgpu_ctx *ctx, double *c_plus, double *c_minus, double *phi, double *anormf0)
@@ -704,7 +704,7 @@ int lbgpu_pnp_get(lbgpu_ctx *ctx, double *c_plus, double *c_minus, double *phi, 
     if (c_minus) LBG_CK(ctx, cudaMemcpyAsync(c_minus, s->cm, b, cudaMemcpyDeviceToHost, ctx->stream));
     if (phi) LBG_CK(ctx, cudaMemcpyAsync(phi, s->phi[s->par], b, cudaMemcpyDeviceToHost, ctx->stream));
     if (anormf0) *anormf0 = s->anormf0;
-    return lbgpu_sync(ctx);
+    return stream_wait(ctx, "lbgpu_pnp_get");
 }
 
 static int sor_solve(lbgpu_ctx *ctx, int *iters, bool defer_anorm);
@@ -786,7 +786,7 @@ static int sor_solve(lbgpu_ctx *ctx, int *iters, bool defer_anorm)
     if (iters) *iters = 0;
     if (s->p.sigma == 0.0) {   // sor.f90:29-33
         LBG_CK(ctx, cudaMemsetAsync(s->phi[s->par], 0, sizeof(double) * ctx->N, st));
-        return lbgpu_sync(ctx);
+        return stream_wait(ctx, "lbgpu_sor");
     }
     PnpArgs a;
     fill_pnp_args(ctx, a);
@@ -903,7 +903,7 @@ int lbgpu_just_eq_smolu(lbgpu_ctx *ctx, int *iters)
         iter = iter + 1;
     }
     if (iters) *iters = iter;
-    return lbgpu_sync(ctx);
+    return stream_wait(ctx, "lbgpu_just_eq_smolu");
 }
 
 int lbgpu_poisson_residual(lbgpu_ctx *ctx, double *residual, double *anormf0)

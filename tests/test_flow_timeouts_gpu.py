@@ -18,6 +18,7 @@ def box(request, monkeypatch):
     """A box whose last 20 steps did not reach their end."""
     monkeypatch.setenv("LBGPU_AA_RESIDENT", "grid")
     with Box(NAT, precision=request.param, **KW) as b:
+        b.kind = request.param
         b.flow_init()
         monkeypatch.setenv("LBGPU_TEST_GRID_WAIT", "1")
         b.flow_steps(20)
@@ -68,3 +69,16 @@ def test_the_state_is_gone_after_a_loop(box, monkeypatch):
     monkeypatch.delenv("LBGPU_TEST_GRID_WAIT")
     assert rc == ERR_TIMEOUT
     gone(box)
+
+
+def test_calls_without_the_flow_state_do_not_report_it(box):
+    if box.kind != FP32_DEV:
+        w = np.array([1 / 3] + [1 / 18] * 6 + [1 / 36] * 12).reshape(19, 1, 1, 1)
+        n = np.ascontiguousarray(w * (NAT == 0))
+        z = [np.zeros(NAT.shape)] * 3
+        box.bounce_back_stream(box.collide(n, n.sum(0), z, z))
+    box.pnp_init(bjl=0.4, sigma=0.0)
+    box.pnp_set(*box.pnp_get())
+    with pytest.raises(LbgpuError) as e:
+        box.flow_get()
+    assert e.value.status == ERR_TIMEOUT
