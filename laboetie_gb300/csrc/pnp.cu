@@ -534,13 +534,13 @@ void anorm_worker(PnpState *s, long long N, int device)
     }
 }
 
-int anorm_begin(lbgpu_ctx *ctx)
+int anorm_begin(lbgpu_ctx *ctx, const double *phi = nullptr)   // null: the current phi
 {
     PnpState *s = ctx->pnp;
     if (!s->phi_host) LBG_CK(ctx, cudaMallocHost((void **)&s->phi_host, sizeof(double) * ctx->N));
     if (!s->anorm_ev) LBG_CK(ctx, cudaEventCreateWithFlags(&s->anorm_ev, cudaEventDisableTiming));
     if (!s->anorm_thread.joinable()) s->anorm_thread = std::thread(anorm_worker, s, ctx->N, ctx->p.device);
-    LBG_CK(ctx, cudaMemcpyAsync(s->phi_host, s->phi[s->par], sizeof(double) * ctx->N, cudaMemcpyDeviceToHost,
+    LBG_CK(ctx, cudaMemcpyAsync(s->phi_host, phi ? phi : s->phi[s->par], sizeof(double) * ctx->N, cudaMemcpyDeviceToHost,
                                 ctx->stream));
     LBG_CK(ctx, cudaEventRecord(s->anorm_ev, ctx->stream));
     {
@@ -734,6 +734,7 @@ static int run_resident(lbgpu_ctx *ctx, const PnpArgs &a, const PnpCtl &c, int m
     cudaStream_t st = ctx->stream;
     std::memset(&h, 0, sizeof(h));
     h.limit = c.limit;
+    h.limit_exact = 1;
     LBG_CK(ctx, cudaMemcpyAsync(s->loop, &h, sizeof(h), cudaMemcpyHostToDevice, st));
     PnpResidentArgs r;
     std::memset(&r, 0, sizeof(r));
@@ -761,6 +762,17 @@ static int run_resident(lbgpu_ctx *ctx, const PnpArgs &a, const PnpCtl &c, int m
         LBG_CK(ctx, launch_pnp_resident(s->resident, r, st));
         LBG_CK(ctx, cudaMemcpyAsync(&h, s->loop, sizeof(h), cudaMemcpyDeviceToHost, st));
         LBG_CK(ctx, cudaStreamSynchronize(st));
+        if (h.undecided && !(h.status & LBGPU_ERR_TIMEOUT)) {   // phi before the solve is in bak[0]
+            if (int rc = anorm_begin(ctx, s->bak[0])) return rc;
+            double before = s->anormf0;
+            if (int rc = anorm_end(ctx)) return rc;
+            std::swap(before, s->anormf0);   // anormf0 stays that of the call's start until its end
+            h.limit = r.limit_factor * before;
+            h.limit_exact = 1;
+            h.undecided = 0;
+            h.resume_conv = h.residual <= h.limit;
+            LBG_CK(ctx, cudaMemcpyAsync(s->loop, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+        }
     } while (!h.done && !(h.status & LBGPU_ERR_TIMEOUT));
     s->lost = (h.status & LBGPU_ERR_TIMEOUT) != 0;
     return s->lost ? pnp_lost(ctx) : LBGPU_OK;

@@ -66,7 +66,14 @@ struct PnpLoop {
     int total;               // sum of the solves' sweep counts (iter - 1 each)
     int outer, equilibrium;  // outer iterations; the convergence test was met
     int converged, done;     // last solve converged; nothing left to do
+    // The stopping value of a solve is a multiple of SUM(ABS(phi)) before it, which the reference adds up
+    // in storage order.  Within a call the device's sum stands in for it, and where that could matter --
+    // the residual as near the stopping value as the two sums may be -- the launch ends undecided and the
+    // host, with the sum in storage order, decides for it.
+    int limit_exact;         // the stopping value is of the sum in storage order
+    int undecided, resume_conv;
     double limit, anormf0;   // stopping value of the solve under way, SUM(ABS(phi)) of the last one
+    double residual, anorm;  // undecided: of the last sweep
     unsigned status;         // last: bits are added to it, the rest is stored by block 0
 };
 

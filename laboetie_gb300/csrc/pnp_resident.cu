@@ -15,9 +15,9 @@
 // The right-hand side (c+ - c-) is formed once per solve.  48^3 touching spheres, per sweep:
 // 21.3 us as launches of the term-by-term sweep.
 //
-// Sums that decide (residual, flux sums, relative changes, anormf0 between the solves of one call)
-// are formed in a fixed order: 128 strided lanes of a block, then the blocks in order, by every
-// block alike, so all take the same decision.
+// Sums that decide (residual, flux sums, relative changes) are formed in a fixed order: 128 strided
+// lanes of a block, then the blocks in order, by every block alike, so all take the same decision.
+// So is the sum of |phi| between the solves of one call, whose order the reference fixes (PnpLoop).
 #include <algorithm>
 #include <cstring>
 
@@ -198,10 +198,15 @@ __global__ void __launch_bounds__(RT, 1) k_pnp_resident(const PnpResidentArgs r)
         }
         const double rhs = a.factor * (cp - cm);
         int iter = L.in_solve ? L.iter : 0;
-        bool conv = false, capped = false;
-        const double limit = L.limit;
-        double anorm = 0.0;
-        while (ok && !conv && !capped && sweeps < r.max_sweeps) {
+        bool conv = L.in_solve && L.resume_conv, capped = !conv && iter >= r.max_iter, undecided = false;
+        // N < 2^17 additions in storage order and fewer on the device: the two sums of |phi| lie within
+        // 2^-35 of each other.  Compared as bits, in the order of the non-negative doubles they are (a
+        // comparison of doubles by every thread costs a sweep what an addition does); -1: never.
+        const double limit = L.limit, margin = L.limit_exact ? 0.0 : 0x1p-35 * limit;
+        const long long below = limit >= 0.0 ? __double_as_longlong(limit - margin) : -1,
+                        above = limit >= 0.0 ? __double_as_longlong(limit + margin) : -1;
+        double anorm = L.anorm, residual = 0.0;
+        while (ok && !conv && !capped && !undecided && sweeps < r.max_sweeps) {
             double v[2] = {0.0, 0.0};
             if (mine) {
                 double s = a.a0[0] * phi;   // 0 + w_0 phi
@@ -226,9 +231,12 @@ __global__ void __launch_bounds__(RT, 1) k_pnp_resident(const PnpResidentArgs r)
             if (!ok) break;
             ++iter;
             ++sweeps;
+            residual = sh.tot[0];
             anorm = sh.tot[1];
-            conv = sh.tot[0] <= limit;
-            capped = !conv && iter >= r.max_iter;
+            const long long bits = __double_as_longlong(residual);
+            conv = bits <= below;
+            undecided = !conv && bits <= above;
+            capped = !conv && !undecided && iter >= r.max_iter;
         }
         if (!ok) break;
         const bool solved = conv || capped;
@@ -236,11 +244,16 @@ __global__ void __launch_bounds__(RT, 1) k_pnp_resident(const PnpResidentArgs r)
         if (tid == 0) {
             L.in_solve = solved ? 0 : 1;
             L.iter = iter;
+            L.undecided = undecided;
+            L.resume_conv = 0;
+            L.residual = residual;
+            L.anorm = anorm;
             if (solved) {
                 L.total += iter - 1;   // the count the reference prints (sor.f90:87)
                 L.converged = conv;
                 L.anormf0 = anorm;
                 L.limit = r.limit_factor * anorm;
+                L.limit_exact = 0;
                 if (!conv) {
                     L.status |= LBGPU_ERR_STEP_CAP;
                     L.done = 1;
