@@ -152,7 +152,8 @@ struct lbgpu_batch {
     BatchTicket *d_ticket = nullptr;
     bool aa_tuned = false;
     bool smem_tuned = false;
-    // workspace of the calls that hand fields back, grown to the largest box asked for
+    // workspace of the calls that hand fields back, grown to the largest box asked for up to WS_KEPT and
+    // taken, like the tables, from what the budget leaves; a larger one lasts for its call
     double *d_ws = nullptr;
     size_t ws_bytes = 0;
     std::vector<int> desc_slot;   // descriptor index -> slot
@@ -181,18 +182,6 @@ int grow(T **p, int &cap, int need, cudaStream_t s)
 }
 
 size_t table_bytes(const BatchInst &d) { return sizeof(float) * (Q - 1) * (size_t)d.Nf; }
-
-int workspace(lbgpu_batch *b, size_t bytes)
-{
-    if (bytes <= b->ws_bytes) return LBGPU_OK;
-    LBB_CK(cudaStreamSynchronize(b->stream));
-    cudaFree(b->d_ws);
-    b->d_ws = nullptr;
-    b->ws_bytes = 0;
-    LBB_CK(cudaMalloc((void **)&b->d_ws, bytes));
-    b->ws_bytes = bytes;
-    return LBGPU_OK;
-}
 
 void drop_graphs(lbgpu_batch *b)
 {
@@ -297,12 +286,19 @@ int rebuild(lbgpu_batch *b)
     return LBGPU_OK;
 }
 
-// Frees the tables of boxes (their steps form the probabilities from V again, with the same bits)
-// until `need` more bytes fit the budget.
+bool leaves_room(const lbgpu_batch *b, size_t need) { return b->used + b->tables + b->ws_bytes + need <= b->budget; }
+
+// Frees the kept workspace and the tables of boxes (their steps form the probabilities from V again, with
+// the same bits) until `need` more bytes fit the budget.
 int make_room(lbgpu_batch *b, size_t need)
 {
+    if (b->d_ws && !leaves_room(b, need)) {
+        LBB_CK(cudaFreeAsync(b->d_ws, b->stream));
+        b->d_ws = nullptr;
+        b->ws_bytes = 0;
+    }
     for (auto &sl : b->slots) {
-        if (b->used + b->tables + need <= b->budget) break;
+        if (leaves_room(b, need)) break;
         if (!sl.active || !sl.d.S) continue;
         LBB_CK(cudaFreeAsync(sl.d.S, b->stream));
         sl.d.S = nullptr;
@@ -311,6 +307,53 @@ int make_room(lbgpu_batch *b, size_t need)
     }
     return LBGPU_OK;
 }
+
+// cudaMallocAsync, without tables where the device itself has no room (others use it too)
+cudaError_t alloc_or_drop_tables(lbgpu_batch *b, void **p, size_t bytes, int &rc)
+{
+    rc = LBGPU_OK;
+    cudaError_t e = cudaMallocAsync(p, bytes, b->stream);
+    if (e == cudaErrorMemoryAllocation && (b->tables || b->d_ws)) {
+        cudaGetLastError();
+        if ((rc = make_room(b, b->budget))) return cudaSuccess;
+        e = cudaMallocAsync(p, bytes, b->stream);
+    }
+    return e;
+}
+
+// Device memory of one call on the batch's stream.
+struct CallMemory {
+    lbgpu_batch *b;
+    double *p = nullptr;
+    bool kept = true;
+    explicit CallMemory(lbgpu_batch *batch) : b(batch) {}
+    ~CallMemory()
+    {
+        if (kept) return;
+        cudaFreeAsync(p, b->stream);
+        cudaStreamSynchronize(b->stream);   // the pool gives it back here
+    }
+    int get(size_t bytes)
+    {
+        constexpr size_t WS_KEPT = 16u << 20;   // moments of 0.5 M nodes
+        int rc;
+        if (bytes > b->ws_bytes && bytes <= WS_KEPT && leaves_room(b, bytes - b->ws_bytes)) {
+            if (b->d_ws) LBB_CK(cudaFreeAsync(b->d_ws, b->stream));
+            b->d_ws = nullptr;
+            b->ws_bytes = 0;
+            LBB_CK(alloc_or_drop_tables(b, (void **)&b->d_ws, bytes, rc));
+            if (rc) return rc;
+            b->ws_bytes = bytes;
+        }
+        if (bytes <= b->ws_bytes) {
+            p = b->d_ws;
+            return LBGPU_OK;
+        }
+        LBB_CK(alloc_or_drop_tables(b, (void **)&p, bytes, rc));
+        kept = rc != LBGPU_OK;
+        return rc;
+    }
+};
 
 // One AA launch of the flow-phase tiles in the variant the tuner chose (descriptors insts: the
 // batch's, or the tuner's scratch copies).
@@ -768,7 +811,7 @@ void lbgpu_batch_destroy(lbgpu_batch *b)
     cudaFree(b->d_du);
     cudaFree(b->d_counts);
     cudaFree(b->d_ticket);
-    cudaFree(b->d_ws);
+    if (b->d_ws) cudaFree(b->d_ws);
     for (cudaEvent_t ev : {b->ev0, b->ev1, b->fork, b->join, b->join2, b->fork_mp, b->join_mp})
         if (ev) cudaEventDestroy(ev);
     if (b->side) cudaStreamDestroy(b->side);
@@ -872,13 +915,9 @@ int lbgpu_batch_add(lbgpu_batch *b, const lbgpu_cell *c, const int8_t *nature, i
     sl.bytes = L.total;
     sl.ntile = ntacc;
     if (int rc = make_room(b, L.total)) return rc;
-    cudaError_t me = cudaMallocAsync(&sl.mem, L.total, s);
-    if (me == cudaErrorMemoryAllocation && b->tables) {   // others use the device too: without tables
-        cudaGetLastError();
-        if (int rc = make_room(b, b->budget)) return rc;
-        me = cudaMallocAsync(&sl.mem, L.total, s);
-    }
-    LBB_CK(me);
+    int room = LBGPU_OK;
+    LBB_CK(alloc_or_drop_tables(b, &sl.mem, L.total, room));
+    if (room) return room;
     char *base = static_cast<char *>(sl.mem);
     BatchInst &d = sl.d;
     std::memset(&d, 0, sizeof(d));
@@ -1039,8 +1078,9 @@ int lbgpu_batch_moments(lbgpu_batch *b, int id, double *rho, double *jx, double 
     const BatchInst &d = b->slots[id].d;
     const int N = d.N;
     cudaStream_t s = b->stream;
-    if ((rc = workspace(b, sizeof(double) * 4 * (size_t)N))) return rc;
-    double *tmp = b->d_ws;
+    CallMemory mem(b);
+    if ((rc = mem.get(sizeof(double) * 4 * (size_t)N))) return rc;
+    double *tmp = mem.p;
     if (d.compact) LBB_CK(cudaMemsetAsync(tmp, 0, sizeof(double) * 4 * (size_t)N, s));   // solid nodes: zeros
     LBB_CK(launch_batch_moments(b->d_insts, desc, batch_units(d), tmp, tmp + N, tmp + 2 * (size_t)N,
                                 tmp + 3 * (size_t)N, s));
@@ -1067,7 +1107,7 @@ int lbgpu_batch_mp_start(lbgpu_batch *b, int id)
     if (sl.d.phase != BATCH_FLOW) return bfail(LBGPU_ERR_INVALID, "lbgpu_batch_mp_start: tracer phase already started");
     cudaStream_t s = b->stream;
     const size_t tb = table_bytes(sl.d);
-    if (sl.d.compact && sl.d.zc == 0 && !sl.d.S && b->used + b->tables + tb <= b->budget) {
+    if (sl.d.compact && sl.d.zc == 0 && !sl.d.S && leaves_room(b, tb)) {
         if (cudaMallocAsync((void **)&sl.d.S, tb, s) == cudaSuccess) {
             b->tables += tb;
             b->dirty = true;
@@ -1119,12 +1159,13 @@ int lbgpu_batch_mp_fields(lbgpu_batch *b, int id, double *P, double *P_ads)
     if (sl.d.phase != BATCH_MP) return bfail(LBGPU_ERR_INVALID, "lbgpu_batch_mp_fields: no tracer phase");
     const size_t N = (size_t)sl.d.N;
     double *outs[2] = {P, P_ads};
-    if (P && P_ads && sl.d.A[0] && N <= field_chunk_nodes((long long)N)) {
-        if (int rc = workspace(b, sizeof(double) * 6 * N)) return rc;
+    CallMemory mem(b);
+    if (P && P_ads && sl.d.A[0] && 2 * N <= FIELD_CHUNK) {
+        if (int rc = mem.get(sizeof(double) * 6 * N)) return rc;
         Field3 f[2] = {};
         f[0].rec = sl.d.P[0];
         f[1].rec = sl.d.A[0];
-        LBB_CK(fields_to_host(f[0], f[1], (long long)N, b->d_ws, P, P_ads, b->stream));
+        LBB_CK(fields_to_host(f[0], f[1], (long long)N, mem.p, P, P_ads, b->stream));
         return LBGPU_OK;
     }
     for (int q = 0; q < 2; ++q) {
@@ -1135,8 +1176,9 @@ int lbgpu_batch_mp_fields(lbgpu_batch *b, int id, double *P, double *P_ads)
             std::memset(outs[q], 0, sizeof(double) * 3 * N);
             continue;
         }
-        if (int rc = workspace(b, sizeof(double) * 3 * field_chunk_nodes((long long)N))) return rc;
-        LBB_CK(field_to_host(f, (long long)N, b->d_ws, outs[q], b->stream));
+        if (!mem.p)
+            if (int rc = mem.get(sizeof(double) * 3 * field_chunk_nodes((long long)N))) return rc;
+        LBB_CK(field_to_host(f, (long long)N, mem.p, outs[q], b->stream));
     }
     return LBGPU_OK;
 }

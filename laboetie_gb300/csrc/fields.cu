@@ -49,8 +49,6 @@ unsigned blocks(size_t n) { return (unsigned)((n + BLOCK - 1) / BLOCK); }
 
 }  // namespace
 
-size_t field_chunk_nodes(long long N) { return (size_t)(N < (1ll << 22) ? N : (1ll << 22)); }
-
 namespace {
 cudaError_t pack(const Field3 &f, size_t at, unsigned n, double *stage, cudaStream_t s)
 {
@@ -84,7 +82,7 @@ cudaError_t field_to_host(const Field3 &f, long long N, double *stage, double *h
     for (size_t at = 0; at < (size_t)N; at += chunk) {
         const unsigned n = (unsigned)((size_t)N - at < chunk ? (size_t)N - at : chunk);
         cudaError_t e = pack(f, at, n, stage, s);
-        ready_pages({{host + 3 * at, sizeof(double) * 3 * n}});
+        if (at == 0) ready_pages({{host, sizeof(double) * 3 * (size_t)N}});
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(host + 3 * at, stage, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, s);
         if (e != cudaSuccess) return e;

@@ -13,11 +13,13 @@ struct Field3 {
     double *comp[3];
 };
 
-// nodes converted at a time; `stage` below holds 3 doubles of each
-size_t field_chunk_nodes(long long N);
-// host[3 i + d] = component d of node i (and back), waiting for the stream
+// nodes converted at a time; `stage` below holds 3 doubles of each (12 MiB at most)
+constexpr size_t FIELD_CHUNK = 1u << 19;
+inline size_t field_chunk_nodes(long long N) { return (size_t)N < FIELD_CHUNK ? (size_t)N : FIELD_CHUNK; }
+// host[3 i + d] = component d of node i (and back), waiting for the stream; stage: field_chunk_nodes(N)
+// nodes
 cudaError_t field_to_host(const Field3 &f, long long N, double *stage, double *host, cudaStream_t s);
-// both fields of a box of one chunk at once (a: host_a, b: host_b), with 6 doubles of stage per node
+// both fields of a box of half a chunk at most at once (a: host_a, b: host_b), with 6 doubles of stage per node
 cudaError_t fields_to_host(const Field3 &a, const Field3 &b, long long N, double *stage, double *host_a, double *host_b,
                            cudaStream_t s);
 cudaError_t field_from_host(const Field3 &f, long long N, double *stage, const double *host, cudaStream_t s);

@@ -33,7 +33,7 @@ struct MpState {
     KeptAllocs allocs;
     MpResident res{};             // many steps per launch (mp_resident.cu) where the box is small
     double *res_vacf = nullptr;   // VACF of one launch's steps
-    double *stage = nullptr;      // staging of lbgpu_mp_get / _set, at most 96 MiB
+    double *stage = nullptr;      // staging of lbgpu_mp_get / _set, at most 12 MiB
     unsigned nblocks = 0;
     int it_next = 1;
     int converged = 0;
