@@ -30,15 +30,21 @@ struct HostRange {
 
 namespace host_pages_detail {
 
-// Whether 8 pages spread over the range are all present: making present pages ready costs as much
-// as a fifth of the copy, so a buffer in use is left alone.
+// Whether the range's pages are all present, or, of more than 64, 8 spread over it: making present pages
+// ready costs as much as a fifth of the copy, so a buffer in use is left alone.
 inline bool present(char *a, size_t len, size_t page)
 {
-    const size_t pages = len / page, step = pages / 8 ? pages / 8 : 1;
-    for (size_t k = 0; k < pages; k += step) {
-        unsigned char v = 0;
-        if (mincore(a + k * page, page, &v) != 0 || !(v & 1)) return false;
+    constexpr size_t ALL = 64, SAMPLES = 8;
+    unsigned char v[ALL];
+    const size_t pages = len / page;
+    if (pages <= ALL) {   // one call
+        if (mincore(a, len, v) != 0) return false;
+        for (size_t k = 0; k < pages; ++k)
+            if (!(v[k] & 1)) return false;
+        return true;
     }
+    for (size_t k = 0; k < pages; k += pages / SAMPLES)
+        if (mincore(a + k * page, page, v) != 0 || !(v[0] & 1)) return false;
     return true;
 }
 
@@ -59,15 +65,17 @@ inline void ready_pages(std::initializer_list<HostRange> ranges)
     size_t total = 0;
     for (const HostRange &r : ranges) {
         if (!r.p || !r.bytes || n == MAX_RANGES) continue;
+        char *a = (char *)((size_t)r.p / page * page);
+        const size_t len = ((size_t)((char *)r.p + r.bytes - a) + page - 1) / page * page;
+        // first, as a buffer in use is the common case and this the cheaper question (lbgpu_moments of 41^3:
+        // 312 us without any, 328 with CUDA's for each of its four arrays)
+        if (host_pages_detail::present(a, len, page)) continue;
         cudaPointerAttributes at;
         if (cudaPointerGetAttributes(&at, r.p) != cudaSuccess) {
             cudaGetLastError();
             continue;
         }
         if (at.type != cudaMemoryTypeUnregistered) continue;
-        char *a = (char *)((size_t)r.p / page * page);
-        const size_t len = ((size_t)((char *)r.p + r.bytes - a) + page - 1) / page * page;
-        if (host_pages_detail::present(a, len, page)) continue;
         todo[n++] = {a, len};
         total += len;
     }
