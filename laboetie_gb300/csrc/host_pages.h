@@ -14,7 +14,7 @@
 
 #include <atomic>
 #include <initializer_list>
-#include <system_error>
+#include <exception>
 #include <thread>
 
 #ifndef MADV_POPULATE_WRITE
@@ -98,7 +98,7 @@ inline void ready_pages(std::initializer_list<HostRange> ranges)
         for (std::thread &t : helper) {
             try {
                 t = std::thread(work);
-            } catch (const std::system_error &) {   // no more threads: this one does it
+            } catch (const std::exception &) {   // no more threads, or no memory for one: this one does it
                 break;
             }
         }

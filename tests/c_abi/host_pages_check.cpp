@@ -3,7 +3,20 @@
 #include "host_pages.h"
 
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
+#include <new>
+
+static int news_left = -1;   // allocations until one fails (-1: none does)
+void *operator new(size_t n)
+{
+    if (news_left == 0) throw std::bad_alloc();
+    if (news_left > 0) --news_left;
+    if (void *p = std::malloc(n)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 static int asked;
 extern "C" cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *)
@@ -29,5 +42,16 @@ int main()
             std::printf("%zu %d asked %d kept %d\n", bytes, used, asked, (int)same);
             munmap(p, bytes + 8192);
         }
+    // no memory for the first, second or third helper thread
+    for (int n = 0; n < 3; ++n) {
+        const size_t bytes = 64 << 20;
+        char *p = (char *)mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+        news_left = n;
+        lbg::ready_pages({{p, bytes}});
+        news_left = -1;
+        std::printf("helpers %d\n", n);
+        std::fflush(stdout);
+        munmap(p, bytes);
+    }
     return 0;
 }
