@@ -221,7 +221,13 @@ int mp_init_impl(lbgpu_ctx *ctx, const lbgpu_tracer *tr, const double *density, 
     double *rho = ctx->d_rho, *J[3] = {ctx->d_j[0], ctx->d_j[1], ctx->d_j[2]};
     double *tmp = nullptr;
     if (density) {
-        LBG_CK(ctx, cudaMallocAsync(&tmp, sizeof(double) * 4 * N, st));
+        cudaError_t e = cudaMallocAsync(&tmp, sizeof(double) * 4 * N, st);
+        if (e == cudaErrorMemoryAllocation) {   // give the older state's buffers back first
+            cudaGetLastError();
+            s->allocs.drop_spare();
+            e = cudaMallocAsync(&tmp, sizeof(double) * 4 * N, st);
+        }
+        LBG_CK(ctx, e);
         const double *h[4] = {density, jx, jy, jz};
         for (int q = 0; q < 4; ++q)
             LBG_CK(ctx, cudaMemcpyAsync(tmp + q * N, h[q], sizeof(double) * N, cudaMemcpyHostToDevice, st));

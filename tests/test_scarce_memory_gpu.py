@@ -1,0 +1,61 @@
+"""Calls on a device with little memory left: what they did before states kept their buffers for the next
+one, and results were converted on the device, they still do."""
+import gc
+
+import numpy as np
+import pytest
+
+from laboetie_gb300 import FP32_DEV, FP64, Box
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+TR = dict(Db=0.01, f_ext=(0.0, 0.0, 1e-5))
+ADS = dict(ka=0.027, kd=0.01, **TR)
+NAT = np.zeros((96, 96, 96), dtype=np.int8)
+MOMENTS = (np.ones(NAT.shape), [np.full(NAT.shape, v) for v in (1e-3, 0.0, -2e-3)])
+
+
+@pytest.fixture
+def leave():
+    """leave(bytes): takes device memory until about that much is free; leave(None): gives it back."""
+    held = []
+
+    def take(free):
+        if free is None:
+            held.clear()
+            gc.collect()
+            torch.cuda.empty_cache()
+            return
+        torch.cuda.synchronize()
+        for _ in range(64):   # in pieces of whole 2 MiB pages
+            more = (torch.cuda.mem_get_info()[0] - free) >> 21 << 21
+            if more <= 0:
+                break
+            try:
+                held.append(torch.empty(more, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                try:
+                    held.append(torch.empty(more // 2 >> 21 << 21 or 1 << 21, dtype=torch.uint8, device="cuda"))
+                except torch.OutOfMemoryError:
+                    break
+    yield take
+    take(None)
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_DEV])
+def test_a_smaller_state_over_a_larger_one(leave, precision):
+    """28 MB of moments to upload, 10 MB free, and an older state with 28 MB (FP32) or 42 MB (FP64) that the
+    new one does not need."""
+    with Box(NAT, precision=precision) as box:
+        box.mp_init(moments=MOMENTS, **TR)
+        box.mp_propagate(2)
+        want = box.mp_get()
+    with Box(NAT, precision=precision) as box:
+        box.mp_init(moments=MOMENTS, **ADS)
+        leave(10 << 20)
+        box.mp_init(moments=MOMENTS, **TR)
+        leave(None)
+        box.mp_propagate(2)
+        got = box.mp_get()
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
