@@ -353,6 +353,16 @@ struct CallMemory {
         kept = rc != LBGPU_OK;
         return rc;
     }
+    // the staging of a field of N nodes: as many of field_chunk_nodes(N) as the device has room for
+    int get_stage(long long N, size_t &nodes)
+    {
+        const size_t least = std::min(FIELD_CHUNK_LEAST, field_chunk_nodes(N));
+        for (nodes = field_chunk_nodes(N);; nodes = std::max(nodes / 2, least)) {
+            const int rc = get(sizeof(double) * 3 * nodes);
+            if (rc == LBGPU_OK || nodes == least) return rc;
+            if (cudaGetLastError() != cudaErrorMemoryAllocation) return rc;
+        }
+    }
 };
 
 // One AA launch of the flow-phase tiles in the variant the tuner chose (descriptors insts: the
@@ -1160,8 +1170,11 @@ int lbgpu_batch_mp_fields(lbgpu_batch *b, int id, double *P, double *P_ads)
     const size_t N = (size_t)sl.d.N;
     double *outs[2] = {P, P_ads};
     CallMemory mem(b);
+    size_t chunk = 0;
     if (P && P_ads && sl.d.A[0] && 2 * N <= FIELD_CHUNK) {
-        if (int rc = mem.get(sizeof(double) * 6 * N)) return rc;
+        if (int rc = mem.get_stage(2 * (long long)N, chunk)) return rc;
+    }
+    if (chunk == 2 * N) {
         Field3 f[2] = {};
         f[0].rec = sl.d.P[0];
         f[1].rec = sl.d.A[0];
@@ -1177,8 +1190,8 @@ int lbgpu_batch_mp_fields(lbgpu_batch *b, int id, double *P, double *P_ads)
             continue;
         }
         if (!mem.p)
-            if (int rc = mem.get(sizeof(double) * 3 * field_chunk_nodes((long long)N))) return rc;
-        LBB_CK(field_to_host(f, (long long)N, mem.p, outs[q], b->stream));
+            if (int rc = mem.get_stage((long long)N, chunk)) return rc;
+        LBB_CK(field_to_host(f, (long long)N, mem.p, chunk, outs[q], b->stream));
     }
     return LBGPU_OK;
 }

@@ -76,9 +76,8 @@ cudaError_t fields_to_host(const Field3 &a, const Field3 &b, long long N, double
     return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
 }
 
-cudaError_t field_to_host(const Field3 &f, long long N, double *stage, double *host, cudaStream_t s)
+cudaError_t field_to_host(const Field3 &f, long long N, double *stage, size_t chunk, double *host, cudaStream_t s)
 {
-    const size_t chunk = field_chunk_nodes(N);
     for (size_t at = 0; at < (size_t)N; at += chunk) {
         const unsigned n = (unsigned)((size_t)N - at < chunk ? (size_t)N - at : chunk);
         cudaError_t e = pack(f, at, n, stage, s);
@@ -90,9 +89,8 @@ cudaError_t field_to_host(const Field3 &f, long long N, double *stage, double *h
     return cudaStreamSynchronize(s);
 }
 
-cudaError_t field_from_host(const Field3 &f, long long N, double *stage, const double *host, cudaStream_t s)
+cudaError_t field_from_host(const Field3 &f, long long N, double *stage, size_t chunk, const double *host, cudaStream_t s)
 {
-    const size_t chunk = field_chunk_nodes(N);
     for (size_t at = 0; at < (size_t)N; at += chunk) {
         const unsigned n = (unsigned)((size_t)N - at < chunk ? (size_t)N - at : chunk);
         cudaError_t e = cudaMemcpyAsync(stage, host + 3 * at, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s);

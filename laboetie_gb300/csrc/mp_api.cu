@@ -34,6 +34,7 @@ struct MpState {
     MpResident res{};             // many steps per launch (mp_resident.cu) where the box is small
     double *res_vacf = nullptr;   // VACF of one launch's steps
     double *stage = nullptr;      // staging of lbgpu_mp_get / _set, at most 12 MiB
+    size_t stage_nodes = 0;       // of field_chunk_nodes, or fewer where the device had no room
     unsigned nblocks = 0;
     int it_next = 1;
     int converged = 0;
@@ -65,8 +66,19 @@ constexpr double EPS = 2.220446049250313e-16;  // epsilon(1._dp)
 
 int stage_init(lbgpu_ctx *ctx, MpState *s)
 {
-    if (s->stage) return LBGPU_OK;
-    LBG_CK(ctx, s->allocs.get((void **)&s->stage, sizeof(double) * 3 * field_chunk_nodes(ctx->N)));
+    const size_t least = std::min(FIELD_CHUNK_LEAST, field_chunk_nodes(ctx->N));
+    for (size_t n = field_chunk_nodes(ctx->N); n > s->stage_nodes; n = std::max(n / 2, least)) {
+        double *p = nullptr;
+        const cudaError_t e = s->allocs.get((void **)&p, sizeof(double) * 3 * n);
+        if (e == cudaSuccess) {
+            s->stage = p;
+            s->stage_nodes = n;
+            return LBGPU_OK;
+        }
+        if (e != cudaErrorMemoryAllocation || (n == least && !s->stage)) return ctx_cuda(ctx, e, "staging of tracer fields");
+        cudaGetLastError();
+        if (n == least) break;
+    }
     return LBGPU_OK;
 }
 
@@ -567,7 +579,7 @@ int lbgpu_mp_get(lbgpu_ctx *ctx, double *P, double *P_ads)
             continue;
         }
         if (int rc = stage_init(ctx, s)) return rc;
-        LBG_CK(ctx, field_to_host(field_of(s, par, q), N, s->stage, outs[q], st));
+        LBG_CK(ctx, field_to_host(field_of(s, par, q), N, s->stage, s->stage_nodes, outs[q], st));
     }
     return LBGPU_OK;
 }
@@ -589,7 +601,7 @@ int lbgpu_mp_set(lbgpu_ctx *ctx, const double *P, const double *P_ads, int it_ne
     for (int q = 0; q < 2; ++q) {
         if (!ins[q]) continue;
         if (int rc = stage_init(ctx, s)) return rc;
-        LBG_CK(ctx, field_from_host(field_of(s, par, q), N, s->stage, ins[q], st));
+        LBG_CK(ctx, field_from_host(field_of(s, par, q), N, s->stage, s->stage_nodes, ins[q], st));
     }
     s->it_next = it_next;
     s->converged = 0;

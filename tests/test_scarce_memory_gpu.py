@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from laboetie_gb300 import FP32_DEV, FP64, Box
+from laboetie_gb300.lbgpu import Batch
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -59,3 +60,32 @@ def test_a_smaller_state_over_a_larger_one(leave, precision):
         box.mp_propagate(2)
         got = box.mp_get()
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("precision", [FP64, FP32_DEV])
+def test_fields_with_little_room(leave, precision):
+    """6 MB free: less than the staging of the box's fields (12 MiB) takes."""
+    with Box(NAT, precision=precision) as box:
+        box.mp_init(moments=MOMENTS, **ADS)
+        box.mp_propagate(3)
+        leave(6 << 20)
+        got = box.mp_get()
+        box.mp_set(*got, it_next=4)
+        leave(None)
+        want = box.mp_get()
+        assert all(np.array_equal(a, b) for a, b in zip(got, want)) and np.abs(got[0]).max() > 0
+
+
+def test_batch_fields_with_little_room(leave):
+    with Batch() as b:
+        ids = [b.add(NAT[:64], f_ext=(0.0, 0.0, 1e-5), tracer=ADS), b.add(NAT, f_ext=(0.0, 0.0, 1e-5), tracer=ADS)]
+        b.steps(4)
+        for i in ids:
+            b.mp_start(i)
+        b.steps(4)
+        leave(6 << 20)
+        got = [b.mp_fields(i) for i in ids]
+        leave(None)
+        want = [b.mp_fields(i) for i in ids]
+    for g, w in zip(got, want):
+        assert all(np.array_equal(x, y) for x, y in zip(g, w)) and np.abs(g[0]).max() > 0
