@@ -113,8 +113,14 @@ int resident_init(lbgpu_ctx *ctx, MpState *s)
                  b_place = up(sizeof(uint32_t) * (m.plan.cluster ? N : 1)),
                  b_scratch = up(m.plan.cluster ? 1 : (f64 ? 3 * sizeof(double) : sizeof(float4)) * (size_t)N);
     char *mem = nullptr;
-    int rc = alloc_zero(ctx, s, &mem, b_part + b_vacf + b_sync + 256 + b_idx + b_place + b_scratch);
-    if (rc) return rc;
+    const size_t bytes = b_part + b_vacf + b_sync + 256 + b_idx + b_place + b_scratch;
+    const cudaError_t e = s->allocs.get((void **)&mem, bytes);
+    if (e == cudaErrorMemoryAllocation) {   // no room: one launch per step
+        cudaGetLastError();
+        return LBGPU_OK;
+    }
+    LBG_CK(ctx, e);
+    LBG_CK(ctx, cudaMemsetAsync(mem, 0, bytes, ctx->stream));
     m.part = reinterpret_cast<double *>(mem);
     s->res_vacf = reinterpret_cast<double *>(mem += b_part);
     m.sync = mem += b_vacf;

@@ -89,3 +89,32 @@ def test_batch_fields_with_little_room(leave):
         want = [b.mp_fields(i) for i in ids]
     for g, w in zip(got, want):
         assert all(np.array_equal(x, y) for x, y in zip(g, w)) and np.abs(g[0]).max() > 0
+
+
+@pytest.mark.parametrize("precision,side", [(FP64, 40), (FP32_DEV, 60)])
+def test_many_steps_per_launch_without_room(leave, monkeypatch, precision, side):
+    """Room for the state of a box, and not for the workspace (16 MiB and one more P) of its many-step
+    launches: one launch per step."""
+    nat = (np.random.default_rng(4).random((side, side, side)) < 0.65).astype(np.int8)
+
+    def run(box):
+        box.mp_init(**ADS)
+        leave(None)
+        box.mp_propagate(7)
+        return box.mp_get()
+    out = []
+    for free in (None, "less"):
+        with Box(nat, precision=precision, f_ext=(1e-5, 0.0, 0.0)) as box:
+            box.flow_init()
+            box.flow_steps(5)
+            box.sync()
+            if free:
+                leave(need - (10 << 20))
+            before = torch.cuda.mem_get_info()[0]
+            out.append(run(box))
+            if not free:
+                box.mp_release()
+                box.mp_init(**ADS)
+                need = before - torch.cuda.mem_get_info()[0]
+    want, got = out
+    assert all(np.array_equal(a, b) for a, b in zip(got, want)) and np.abs(got[0]).max() > 0
