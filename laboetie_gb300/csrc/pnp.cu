@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(PB) k_sor_jacobi(const PnpArgs a, double *phi0
         double q;
         if constexpr (FIRST) {
             q = a.factor * (a.cp[r] - a.cm[r]);
-            rhs[r] = q;
+            if (rhs) rhs[r] = q;
         } else {
             q = rhs[r];
         }
@@ -622,7 +622,13 @@ int lbgpu_pnp_init(lbgpu_ctx *ctx, const lbgpu_pnp_params *p, double *anormf0)
         if ((rc = alloc(&d, (sizeof(PnpLoop) + 7) / sizeof(double)))) return rc;
         s->loop = reinterpret_cast<PnpLoop *>(d);
     } else if (jacobi) {
-        if ((rc = alloc(&s->rhs, N))) return rc;
+        const cudaError_t e = s->allocs.get((void **)&s->rhs, sizeof(double) * N);
+        if (e == cudaErrorMemoryAllocation) {   // no room: every sweep forms it, and the products, by itself
+            cudaGetLastError();
+            s->rhs = nullptr;
+        } else {
+            LBG_CK(ctx, e);
+        }
     }
     // partials: 4 per block, twice (two reductions read back together); results: 4, twice
     if ((rc = alloc(&s->partial, 8 * (size_t)MP_MAX_BLOCKS)) || (rc = alloc(&s->result, 8))) return rc;
@@ -840,7 +846,7 @@ static int sor_solve(lbgpu_ctx *ctx, int *iters, bool defer_anorm)
                     else k_sor_color_gen<<<grid, PB, 0, st>>>(b, s->phi[s->par]);
                 }
             } else {
-                if (k == 0) k_sor_jacobi<true><<<grid, PB, 0, st>>>(a, s->phi[0], s->phi[1], s->fp, s->fm, s->rhs);
+                if (k == 0 || !s->rhs) k_sor_jacobi<true><<<grid, PB, 0, st>>>(a, s->phi[0], s->phi[1], s->fp, s->fm, s->rhs);
                 else k_sor_jacobi<false><<<grid, PB, 0, st>>>(a, s->phi[0], s->phi[1], s->fp, s->fm, s->rhs);
             }
         }

@@ -41,7 +41,7 @@ struct PnpState {
     double *cp = nullptr, *cm = nullptr;
     // flux_site_plus / flux_site_minus; during a Jacobi solve, w_axis phi by sweep parity
     double *fp = nullptr, *fm = nullptr;
-    double *rhs = nullptr;                  // Jacobi solve: 4 pi bjl kBT/2 (c+ - c-)
+    double *rhs = nullptr;                  // Jacobi solve: 4 pi bjl kBT/2 (c+ - c-); null without room
     double *bak[3] = {nullptr, nullptr, nullptr};  // phi_old, c_plus_old, c_minus_old
     double *partial = nullptr;              // 4 per block
     double *result = nullptr;               // 4 reduced sums

@@ -6,7 +6,8 @@ import numpy as np
 import pytest
 
 from laboetie_gb300 import FP32_DEV, FP64, Box
-from laboetie_gb300.lbgpu import Batch
+from laboetie_gb300 import geometry as geo
+from laboetie_gb300.lbgpu import POISSON_JACOBI, Batch
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -118,3 +119,22 @@ def test_many_steps_per_launch_without_room(leave, monkeypatch, precision, side)
                 need = before - torch.cuda.mem_get_info()[0]
     want, got = out
     assert all(np.array_equal(a, b) for a, b in zip(got, want)) and np.abs(got[0]).max() > 0
+
+
+def test_charges_without_room_for_the_right_hand_side(leave):
+    """17 MB of it at 128^3, with 10 MB less free than the state takes with it: the same sweeps."""
+    nat = geo.cc(128, 128, 128)
+    charges = dict(bjl=0.4, sigma=-20.0, lambda_D=4.0, D_plus=0.05, D_minus=0.05, solver=POISSON_JACOBI, omega=1.2, tol=1e-5)
+    out = []
+    for free in (None, "less"):
+        with Box(nat, precision=FP32_DEV) as box:
+            if free:
+                leave(need - (10 << 20))
+            before = torch.cuda.mem_get_info()[0]
+            box.pnp_init(**charges)
+            need = before - torch.cuda.mem_get_info()[0]
+            leave(None)
+            out.append((box.sor(), box.pnp_get()))
+    (n, want), (m, got) = out
+    assert n == m > 2 and want[3] == got[3]
+    assert all(np.array_equal(a, b) for a, b in zip(got[:3], want[:3])) and np.abs(got[2]).max() > 0
