@@ -39,12 +39,14 @@ struct Real<false> {
     using T = float;
     static constexpr int threads = RT32;
     static constexpr int words = 4;   // shared-memory record of a node's P: one 16-byte access
+    static constexpr int extra = 0;   // records beyond the nodes'
 };
 template <>
 struct Real<true> {
     using T = double;
     static constexpr int threads = RT64;
     static constexpr int words = 3;
+    static constexpr int extra = 1;   // zero
 };
 
 struct MpResidentArgs {
@@ -89,18 +91,18 @@ __global__ void __launch_bounds__(Real<F64>::threads, 1) k_mp_resident(const MpR
 {
     using R = typename Real<F64>::T;
     constexpr int W = Real<F64>::words;
-    // CLUSTER: P records [2][T + 1][W], the last one zero; neighbour addresses [18][T]; F64: VACF terms
+    // CLUSTER: P records [2][TR][W], in FP64 the last one zero; neighbour addresses [18][T]; F64: VACF terms
     // [warps][3][32]
     extern __shared__ __align__(16) unsigned char smraw[];
-    const unsigned T = blockDim.x, tid = threadIdx.x, lane = tid & 31;
+    const unsigned T = blockDim.x, TR = T + Real<F64>::extra, tid = threadIdx.x, lane = tid & 31;
     const unsigned rank = blockIdx.x;   // CLUSTER: one cluster, block = rank
     const unsigned i = rank * T + tid, nwarps = gridDim.x * (T / 32), warp = i / 32;
     const bool mine = i < r.Nf;
     R *const rec = reinterpret_cast<R *>(smraw);                                  // CLUSTER
-    unsigned *const nbr = reinterpret_cast<unsigned *>(smraw + (CLUSTER ? 2 * (size_t)(T + 1) * W * sizeof(R) : 0)) + tid;
+    unsigned *const nbr = reinterpret_cast<unsigned *>(smraw + (CLUSTER ? 2 * (size_t)TR * W * sizeof(R) : 0)) + tid;
     double *const terms = reinterpret_cast<double *>(nbr - tid + (size_t)18 * T) + (tid / 32) * 96;   // F64
     const unsigned rec0 = CLUSTER ? smem_addr(smraw) : 0u;
-    const unsigned flip = CLUSTER ? (unsigned)((T + 1) * W * sizeof(R)) : 0u;   // bytes between the two P buffers
+    const unsigned flip = CLUSTER ? (unsigned)(TR * W * sizeof(R)) : 0u;   // bytes between the two P buffers
 
     const int lx = F64 ? r.a64.lx : r.a32.lx, ly = F64 ? r.a64.ly : r.a32.ly, lz = F64 ? r.a64.lz : r.a32.lz;
     const bool ads = F64 ? r.a64.ads != 0 : r.a32.ads != 0;
@@ -170,11 +172,11 @@ __global__ void __launch_bounds__(Real<F64>::threads, 1) k_mp_resident(const MpR
     }
     auto put = [&](unsigned buf) {   // own P into the cluster's buffer
 #pragma unroll
-        for (int d = 0; d < 3; ++d) rec[(buf * (T + 1) + tid) * W + d] = p[d];
+        for (int d = 0; d < 3; ++d) rec[(buf * TR + tid) * W + d] = p[d];
     };
     if constexpr (CLUSTER) {
         if (mine) put(0);
-        if (F64 && tid < 2 * W) rec[(tid / W * (T + 1) + T) * W + tid % W] = 0;
+        if (F64 && tid < 2 * W) rec[(tid / W * TR + T) * W + tid % W] = 0;
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     } else {
         __syncthreads();
@@ -326,7 +328,7 @@ template <bool F64, bool CLUSTER>
 size_t smem_of(unsigned T)
 {
     using R = typename Real<F64>::T;
-    return (size_t)18 * T * sizeof(unsigned) + (CLUSTER ? 2 * (size_t)(T + 1) * Real<F64>::words * sizeof(R) : 0) +
+    return (size_t)18 * T * sizeof(unsigned) + (CLUSTER ? 2 * (size_t)(T + Real<F64>::extra) * Real<F64>::words * sizeof(R) : 0) +
            (F64 ? (size_t)T / 32 * 96 * sizeof(double) : 0);
 }
 
