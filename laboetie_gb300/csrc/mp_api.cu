@@ -40,6 +40,7 @@ struct MpState {
     int converged = 0;
     unsigned pending = 0;  // error raised at init, reported by the first propagate
     bool lost = false;     // a wait of a many-step launch ran out: P is not that of any step
+    bool diverged = false; // VACF has left the finite numbers: one launch per step
     double vacf0[3] = {0, 0, 0};
 };
 
@@ -395,7 +396,8 @@ static int mp_lost(lbgpu_ctx *ctx)
 
 // The steps of mp_run as resident launches: `c` is the control block as the call starts (its
 // thresholds set).  A launch that meets the convergence test before its last step is repeated up to
-// that step from the P it started from.
+// that step from the P it started from.  One with a VACF that is not finite counts for nothing: the run is
+// left as it stood before it, and diverged (mp_resident.cu is for finite P).
 static int mp_run_resident(lbgpu_ctx *ctx, MpCtl &c, int nsteps, double *vacf_out, bool timing, float *ms)
 {
     MpState *s = ctx->mp;
@@ -418,6 +420,8 @@ static int mp_run_resident(lbgpu_ctx *ctx, MpCtl &c, int nsteps, double *vacf_ou
     while (done < nsteps && !c.converged) {
         int n = std::min(nsteps - done, s->res.max_steps);
         if (int rc = launch(n, true)) return rc;
+        s->diverged = !std::all_of(rows.begin(), rows.begin() + 3 * n, [](double v) { return std::isfinite(v); });
+        if (s->diverged) break;
         for (int k = 0; k < n && !c.converged; ++k) {
             bool conv = c.it + k > 2;
             for (int d = 0; d < 3; ++d) {
@@ -439,6 +443,7 @@ static int mp_run_resident(lbgpu_ctx *ctx, MpCtl &c, int nsteps, double *vacf_ou
         done += n;
     }
     c.done = 1;
+    s->it_next = c.it;
     if (timing) {
         LBG_CK(ctx, cudaEventRecord(ctx->ev1, st));
         LBG_CK(ctx, cudaEventSynchronize(ctx->ev1));
@@ -465,12 +470,15 @@ static int mp_run(lbgpu_ctx *ctx, int nsteps, double *vacf_out, int *steps_done,
     MpCtl c;
     LBG_CK(ctx, cudaMemcpyAsync(&c, s->a64.ctl, sizeof(c), cudaMemcpyDeviceToHost, st));
     LBG_CK(ctx, cudaStreamSynchronize(st));
-    c.it = s->it_next;
-    c.it_base = s->it_next;
-    c.max_it = s->it_next + nsteps - 1;
-    c.done = 0;
-    c.converged = 0;
-    c.blocks_done = 0;
+    auto begin = [&](int steps) {
+        c.it = s->it_next;
+        c.it_base = s->it_next;
+        c.max_it = s->it_next + steps - 1;
+        c.done = 0;
+        c.converged = 0;
+        c.blocks_done = 0;
+    };
+    begin(nsteps);
     // module_moment_propagation.f90:284: |vacf| < 1/(2 lx ly lz / Db) and < 1.e-12 (a default real)
     if (timing) {
         c.thr1 = c.thr2 = -1.0;  // never converges: every step runs
@@ -479,13 +487,19 @@ static int mp_run(lbgpu_ctx *ctx, int nsteps, double *vacf_out, int *steps_done,
         c.thr1 = 1.0 / den;
         c.thr2 = (double)1.e-12f;
     }
-    if (s->res.plan.blocks) {
+    int before = 0;   // steps of this call made by many-step launches
+    if (s->res.plan.blocks && !s->diverged) {
         if (int rc = mp_run_resident(ctx, c, nsteps, vacf_out, timing, ms)) return rc;
-        s->it_next = c.last_it + 1;
-        s->converged = c.converged;
-        if (steps_done) *steps_done = c.last_it - c.it_base + 1;
-        if (is_converged) *is_converged = c.converged;
-        return LBGPU_OK;
+        before = c.it - c.it_base;
+        if (!s->diverged) {
+            s->converged = c.converged;
+            if (steps_done) *steps_done = before;
+            if (is_converged) *is_converged = c.converged;
+            return LBGPU_OK;
+        }
+        nsteps -= before;   // the rest, launch by launch
+        if (vacf_out) vacf_out += 3 * (size_t)before;
+        begin(nsteps);
     }
     LBG_CK(ctx, cudaMemcpyAsync(s->a64.ctl, &c, sizeof(c), cudaMemcpyHostToDevice, st));
     double *hist = nullptr;
@@ -548,7 +562,7 @@ static int mp_run(lbgpu_ctx *ctx, int nsteps, double *vacf_out, int *steps_done,
     s->a64.hist = s->a32.hist = nullptr;
     s->it_next = c.last_it + 1;
     s->converged = c.converged;
-    if (steps_done) *steps_done = done;
+    if (steps_done) *steps_done = before + done;
     if (is_converged) *is_converged = c.converged;
     return LBGPU_OK;
 }
@@ -612,6 +626,7 @@ int lbgpu_mp_set(lbgpu_ctx *ctx, const double *P, const double *P_ads, int it_ne
     s->it_next = it_next;
     s->converged = 0;
     s->lost = false;
+    s->diverged = false;
     return LBGPU_OK;
 }
 

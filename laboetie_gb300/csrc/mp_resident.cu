@@ -11,7 +11,8 @@
 // VACF leaves the step: each warp stores its three sums per step, and a second kernel adds the
 // warps in a fixed order after the launch.  The convergence test (it > 2 and |VACF| below both
 // thresholds) is made on the host then; the launch leaves the P it started from untouched, so a
-// run that turned out to converge inside it is repeated up to that step.  Per step, a reduction
+// run that turned out to converge inside it is repeated up to that step, and one whose VACF did not stay
+// finite is left to the launches per step: the kernels below are for finite P.  Per step, a reduction
 // with its last-block decision costs 6 us of FP64 shuffles, fences and dependent reads.  us per
 // step, as launches against here: 1 x 50 x 50 cell (2,323 fluid nodes) FP32 11.1 / 1.57, FP64
 // 20.0 / 9.2 (most of it its 126 FP64 instructions of 64 cycles each); 30^3 touching spheres
@@ -39,14 +40,12 @@ struct Real<false> {
     using T = float;
     static constexpr int threads = RT32;
     static constexpr int words = 4;   // shared-memory record of a node's P: one 16-byte access
-    static constexpr int extra = 0;   // records beyond the nodes'
 };
 template <>
 struct Real<true> {
     using T = double;
     static constexpr int threads = RT64;
     static constexpr int words = 3;
-    static constexpr int extra = 1;   // zero
 };
 
 struct MpResidentArgs {
@@ -91,18 +90,17 @@ __global__ void __launch_bounds__(Real<F64>::threads, 1) k_mp_resident(const MpR
 {
     using R = typename Real<F64>::T;
     constexpr int W = Real<F64>::words;
-    // CLUSTER: P records [2][TR][W], in FP64 the last one zero; neighbour addresses [18][T]; F64: VACF terms
-    // [warps][3][32]
+    // neighbour addresses [18][T]; CLUSTER: P records [2][T][W]; F64: VACF terms [warps][3][32]
     extern __shared__ __align__(16) unsigned char smraw[];
-    const unsigned T = blockDim.x, TR = T + Real<F64>::extra, tid = threadIdx.x, lane = tid & 31;
+    const unsigned T = blockDim.x, tid = threadIdx.x, lane = tid & 31;
     const unsigned rank = blockIdx.x;   // CLUSTER: one cluster, block = rank
     const unsigned i = rank * T + tid, nwarps = gridDim.x * (T / 32), warp = i / 32;
     const bool mine = i < r.Nf;
     R *const rec = reinterpret_cast<R *>(smraw);                                  // CLUSTER
-    unsigned *const nbr = reinterpret_cast<unsigned *>(smraw + (CLUSTER ? 2 * (size_t)TR * W * sizeof(R) : 0)) + tid;
+    unsigned *const nbr = reinterpret_cast<unsigned *>(smraw + (CLUSTER ? 2 * (size_t)T * W * sizeof(R) : 0)) + tid;
     double *const terms = reinterpret_cast<double *>(nbr - tid + (size_t)18 * T) + (tid / 32) * 96;   // F64
     const unsigned rec0 = CLUSTER ? smem_addr(smraw) : 0u;
-    const unsigned flip = CLUSTER ? (unsigned)(TR * W * sizeof(R)) : 0u;   // bytes between the two P buffers
+    const unsigned flip = CLUSTER ? (unsigned)(T * W * sizeof(R)) : 0u;   // bytes between the two P buffers
 
     const int lx = F64 ? r.a64.lx : r.a32.lx, ly = F64 ? r.a64.ly : r.a32.ly, lz = F64 ? r.a64.lz : r.a32.lz;
     const bool ads = F64 ? r.a64.ads != 0 : r.a32.ads != 0;
@@ -134,22 +132,12 @@ __global__ void __launch_bounds__(Real<F64>::threads, 1) k_mp_resident(const MpR
                 const float4 vn = r.a32.V[rp];
                 s[l] = mp32_scatter(blocked, r.a32.a1[wclass(l)], mp32_cdot<-c.x, -c.y, -c.z>(vn), r.a32.lwh[wclass(l)]);
             }
-            // A blocked link's probability is 0.  FP64 adds 0 times the solid node's P, as mp_f64.cu does: the
-            // zero record in a cluster, a zero in memory else (times an infinite P of its own it would add
-            // NaN).  FP32 adds 0 times a difference from its own P: its own record will do.
+            // a blocked link's probability is 0: any record of finite values will do (its own)
             if constexpr (CLUSTER) {
-                unsigned owner, slot;
-                if (blocked && F64) {
-                    owner = rank;
-                    slot = T;
-                } else {
-                    const unsigned q = blocked ? i : r.place[rp];
-                    owner = q / T;
-                    slot = q - owner * T;
-                }
-                nbr[(l - 1) * T] = map_rank(rec0 + (unsigned)(slot * W * sizeof(R)), owner);
+                const unsigned q = blocked ? i : r.place[rp], owner = q / T;
+                nbr[(l - 1) * T] = map_rank(rec0 + (unsigned)((q - owner * T) * W * sizeof(R)), owner);
             } else {
-                nbr[(l - 1) * T] = blocked && !F64 ? node : rp;
+                nbr[(l - 1) * T] = blocked ? node : rp;
             }
         });
         if constexpr (F64) {
@@ -172,11 +160,10 @@ __global__ void __launch_bounds__(Real<F64>::threads, 1) k_mp_resident(const MpR
     }
     auto put = [&](unsigned buf) {   // own P into the cluster's buffer
 #pragma unroll
-        for (int d = 0; d < 3; ++d) rec[(buf * TR + tid) * W + d] = p[d];
+        for (int d = 0; d < 3; ++d) rec[(buf * T + tid) * W + d] = p[d];
     };
     if constexpr (CLUSTER) {
         if (mine) put(0);
-        if (F64 && tid < 2 * W) rec[(tid / W * TR + T) * W + tid % W] = 0;
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     } else {
         __syncthreads();
@@ -204,7 +191,7 @@ __global__ void __launch_bounds__(Real<F64>::threads, 1) k_mp_resident(const MpR
             if (lane < 24 && (lane & 7) == 0) out[lane >> 3] = t;
         } else {
             const float t[3] = {p[0] * us[0], p[1] * us[1], p[2] * us[2]};
-            const double w = warp_sum3_exact(t);
+            const double w = warp_sum3_finite(t);
             if (lane < 3) out[lane] = w;
         }
         // ---- the step
@@ -328,7 +315,7 @@ template <bool F64, bool CLUSTER>
 size_t smem_of(unsigned T)
 {
     using R = typename Real<F64>::T;
-    return (size_t)18 * T * sizeof(unsigned) + (CLUSTER ? 2 * (size_t)(T + Real<F64>::extra) * Real<F64>::words * sizeof(R) : 0) +
+    return (size_t)18 * T * sizeof(unsigned) + (CLUSTER ? 2 * (size_t)T * Real<F64>::words * sizeof(R) : 0) +
            (F64 ? (size_t)T / 32 * 96 * sizeof(double) : 0);
 }
 

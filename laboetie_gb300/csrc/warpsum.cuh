@@ -40,7 +40,21 @@ static __device__ __noinline__ double warp_nonfinite_sum(float v)
     return s;
 }
 
-// Sums of three values per lane: lane d < 3 returns the sum of t[d].
+// Sums of three finite values per lane: lane d < 3 returns the sum of t[d], NaN with a non-finite term.
+__device__ __forceinline__ double warp_sum3_finite(const float (&t)[3])
+{
+    const int lane = threadIdx.x & 31;
+    int e[3];
+    long long v[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) v[d] = warp_int_sum(t[d], e[d]);
+    if (lane >= 3) return 0.0;
+    const int emax = lane == 0 ? e[0] : (lane == 1 ? e[1] : e[2]);
+    const double s = warp_exact(lane == 0 ? v[0] : (lane == 1 ? v[1] : v[2]), emax);
+    return emax == 255 ? __longlong_as_double(0x7ff8000000000000ll) : s;
+}
+
+// The same with whatever FP64 additions make of non-finite terms.
 __device__ __forceinline__ double warp_sum3_exact(const float (&t)[3])
 {
     const int lane = threadIdx.x & 31;
