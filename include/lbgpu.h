@@ -52,7 +52,7 @@ enum lbgpu_status {
     LBGPU_ERR_FLUX_SUM = 1 << 7,           /* just_eq_smolu.f90:108-112 "sum of all flux does not add up" */
     LBGPU_ERR_CHARGE = 1 << 8,             /* charge_test.f90:20-24 "charge is not conserved" */
     LBGPU_ERR_UNSUPPORTED = 1 << 9,        /* an input the reference has no defined result for */
-    LBGPU_ERR_TIMEOUT = 1 << 10            /* a device-side wait ran out of its iteration limit */
+    LBGPU_ERR_TIMEOUT = 1 << 10            /* a device-side wait ran out of its limit; the state of that call is lost */
 };
 
 /* Storage / arithmetic of the flow and tracer populations. */

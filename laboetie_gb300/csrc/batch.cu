@@ -123,8 +123,7 @@ __device__ __forceinline__ void aa_node_compact(const BatchInst &I, unsigned i, 
 // operations in the same order (mp_slab.cuh helpers, mp_link_order), so a batched box's P is
 // bit-identical to a single box's; with INIT, P(t=1), the node's fixed (u*, D) in aux and its
 // VACF(0) term (before the 1/Pstat factor) instead (module_moment_propagation.f90:112-136).
-// vt receives the node's VACF term in FP32 (a thread's few nodes; FP64 across threads, as the
-// single box sums them).
+// vt receives the node's VACF term in FP32 (added exactly over a warp, in FP64 beyond).
 template <bool INIT>
 __device__ __forceinline__ void mp_node(const float4 *V, const float4 *Pn, float4 *Pnext,
                                         const float4 *An, float4 *Anext, float4 *aux, unsigned r, int x,
@@ -481,8 +480,9 @@ __global__ void __launch_bounds__(BATCH_BLOCK, MINB) k_batch_aa_list(const Batch
 // sums.  Bound by L2 and memory traffic (the table's 72 B, P of the neighbouring rows, (u*, D)) at
 // large sizes.  16 tubes of 32^2 x L (846 k fluid nodes), per step: 54.9 us as slab tiles, 48.5 as
 // node tiles forming the probabilities from V, 41 with the table, 35.5 with each SM on a run of
-// consecutive tiles (42 registers: 51, 64 and 85 take 39.9, 42.5 and 46.6 us); 82 us before the FP64
-// shuffles of the VACF terms were taken out of the node tiles.
+// consecutive tiles (42 registers: 51, 64 and 85 take 39.9, 42.5 and 46.6 us); 82 us with FP64 shuffles
+// for the VACF terms.  Their exact sums take 1.0 us, the solid node's zero across a blocked link 0.8 (256
+// cells beside the tubes, 48.3 in all; selects or predicated moves in place of that load 50 to 53).
 template <bool INIT>
 __global__ void __launch_bounds__(BATCH_BLOCK, 6) k_batch_mp(const BatchInst *__restrict__ insts,
                                                           const BatchTile *__restrict__ tiles,
