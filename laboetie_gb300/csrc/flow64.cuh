@@ -365,8 +365,7 @@ __device__ __forceinline__ void collide_node_fused(double (&n)[Q], const double 
 // a quarter of it up, a force from a sixteenth of it up -- take the FP64 form.
 // Porous medium of 128^3 (1.26 M fluid nodes), tau 0.8: 400 -> 135 us a step (57 us of HBM traffic;
 // now bound by the integer pipes): 165 as first built, 140 in blocks of 128 threads, 134 with the
-// short shifts of the common case, 135 since the axis pairs take the rest of the flux (the loop's step 195
-// and 188).  Error of jx / jy / jz against binary128, force along x, each of its norm: porous medium of
+// short shifts of the common case and since the axis pairs take the rest of the flux (the loop's step 195).  Error of jx / jy / jz against binary128, force along x, each of its norm: porous medium of
 // 96^3, tau 0.8, 120 steps 1.2e-14 / 2.9e-14 / 3.5e-14 where the FP64 form has 5.9e-14 / 1.4e-13 /
 // 1.5e-13; 64^3, tau 0.62, 400 steps 0.6e-14 / 1.4e-14 / 1.6e-14 and 3.2e-14 / 7.8e-14 / 8.7e-14.
 
@@ -414,7 +413,7 @@ __device__ __forceinline__ long long force_to_fixed(double F, int emax)
 
 // One fused step of a node: n, after streaming, becomes the collided populations.  Returns false,
 // with n untouched, for a node outside the fixed-point range.  WANT_J: its j, as doubles.
-template <int FMASK, bool WANT_J>
+template <int FMASK, bool WANT_J, bool FORMS>
 __device__ __forceinline__ bool fused_fixed(double (&n)[Q], const bool fm, const bool fc, const double fx,
                                             const double fy, const double fz, const FlowArgs64 &a, double &ox,
                                             double &oy, double &oz)
@@ -515,64 +514,84 @@ __device__ __forceinline__ bool fused_fixed(double (&n)[Q], const bool fm, const
     const long long base = 2 * mulhi(R, K.fix_c2_36) - mulhi((qx + qy + qz) * 2, THIRD);
     const long long base_axis = 2 * base;
     long long rest = R - __mulhi((int)(R >> 31), K.fix_loss);
-    const bool relax = K.fix_c1 != 0;
     // the flux after the collision, j - (c2/2) F + c3 F with j = sum c n + F/2: what streams in and F,
     // or the part of F that a step has whose moments or collision alone take it
-    auto flux = [&](long long sum, long long g) {
-        if constexpr (FMASK == 0) return sum;
-        if (!(fm || fc)) return sum;
-        const long long h = mulhi(4 * g, K.fix_c2);   // c2 F / 2
-        const long long G = fm ? (fc ? g : h) : g - h;
-        return sum + ((G + (((int)sum >> 3) & 7)) >> 3);
+    auto flux = [&](auto D, long long sum, long long g) {
+        if constexpr (!(FMASK & decltype(D)::value)) {
+            return sum;
+        } else {
+            if (!(fm || fc)) return sum;
+            long long G = g;
+            if (!(fm && fc)) {
+                const long long h = mulhi(4 * g, K.fix_c2);   // c2 F / 2
+                G = fm ? h : g - h;
+            }
+            return sum + ((G + (((int)sum >> 3) & 7)) >> 3);
+        }
     };
-    // (s, d) of a pair in v[l], v[inv l] -> its collided populations e + o (+ odd) and e - o; A, B to
-    // nearest, and half a unit more for the rounding down of the c1 products
-    const long long half = relax ? 8 : 4;
-    auto even = [&](auto P, long long A) {
-        long long e = (A + half) >> 3;
-        if (relax) e += mulhi(v[pair_l(decltype(P)::value)] * 2, K.fix_c1);
-        return e;
-    };
-    auto put = [&](auto P, long long e, long long o, long long odd) {
-        constexpr int l = pair_l(decltype(P)::value);
-        rest -= 2 * e + odd;
-        n[l] = fixed_to_double(e + o + odd, emax);
-        n[inv(l)] = fixed_to_double(e - o, emax);
-    };
-    long long tx = flux(sx, gx), ty = flux(sy, gy), tz = flux(sz, gz);
-    auto diagonal = [&](auto P, long long A, long long B) {
-        constexpr int l = pair_l(decltype(P)::value);
-        constexpr Vel c = vel(l);
-        long long o = (B + half) >> 3;
-        if (relax) o += mulhi(v[inv(l)] * 2, K.fix_c1);
-        if constexpr (c.x != 0) tx -= c.x > 0 ? 2 * o : -2 * o;
-        if constexpr (c.y != 0) ty -= c.y > 0 ? 2 * o : -2 * o;
-        if constexpr (c.z != 0) tz -= c.z > 0 ? 2 * o : -2 * o;
-        put(P, even(P, A), o, 0);
-    };
-    // an axis pair takes what the diagonals leave of its flux (n_l - n_inv l = t), as soon as it is known
+    long long tx = flux(std::integral_constant<int, 1>{}, sx, gx), ty = flux(std::integral_constant<int, 2>{}, sy, gy),
+              tz = flux(std::integral_constant<int, 4>{}, sz, gz);
     const long long mxy = mulhi(ux + uy, (hx + hy) * 4), mxz = mulhi(ux + uz, (hx + hz) * 4),
                     myz = mulhi(uy + uz, (hy + hz) * 4);
-    diagonal(std::integral_constant<int, 3>{}, base + mxy, bx + by);                        // (1, 1, 0)
-    diagonal(std::integral_constant<int, 4>{}, base + 2 * (qx + qy) - mxy, by - bx);        // (-1, 1, 0)
-    diagonal(std::integral_constant<int, 5>{}, base + mxz, bx + bz);                        // (1, 0, 1)
-    diagonal(std::integral_constant<int, 6>{}, base + 2 * (qx + qz) - mxz, bz - bx);        // (-1, 0, 1)
-    put(std::integral_constant<int, 0>{}, even(std::integral_constant<int, 0>{}, base_axis + 2 * qx), tx >> 1, tx & 1);
-    diagonal(std::integral_constant<int, 7>{}, base + myz, by + bz);                        // (0, 1, 1)
-    diagonal(std::integral_constant<int, 8>{}, base + 2 * (qy + qz) - myz, bz - by);        // (0, -1, 1)
-    put(std::integral_constant<int, 1>{}, even(std::integral_constant<int, 1>{}, base_axis + 2 * qy), ty >> 1, ty & 1);
-    put(std::integral_constant<int, 2>{}, even(std::integral_constant<int, 2>{}, base_axis + 2 * qz), tz >> 1, tz & 1);
+    // (s, d) of a pair in v[l], v[inv l] -> its collided populations e + o (+ odd) and e - o; A, B to
+    // nearest, and half a unit more for the rounding down of the c1 products
+    auto pairs = [&](const auto relax) {
+        const long long half = relax ? 8 : 4;
+        auto put = [&](auto P, long long e, long long o, int odd) {
+            constexpr int l = pair_l(decltype(P)::value);
+            rest -= 2 * e + odd;
+            n[l] = fixed_to_double(e + o + odd, emax);
+            n[inv(l)] = fixed_to_double(e - o, emax);
+        };
+        auto diagonal = [&](auto P, long long A, long long B) {
+            constexpr int l = pair_l(decltype(P)::value);
+            constexpr Vel c = vel(l);
+            long long e = (A + half) >> 3, o = (B + half) >> 3;
+            if (relax) {
+                e += mulhi(v[l] * 2, K.fix_c1);
+                o += mulhi(v[inv(l)] * 2, K.fix_c1);
+            }
+            if constexpr (c.x != 0) tx -= c.x > 0 ? 2 * o : -2 * o;
+            if constexpr (c.y != 0) ty -= c.y > 0 ? 2 * o : -2 * o;
+            if constexpr (c.z != 0) tz -= c.z > 0 ? 2 * o : -2 * o;
+            put(P, e, o, 0);
+        };
+        // an axis pair takes what the diagonals leave of its flux t: n_l - n_inv l = 2 o + odd = t
+        auto axis = [&](auto P, long long A, long long o, int odd) {
+            long long e = (A + half) >> 3;
+            if (relax) e += mulhi(v[pair_l(decltype(P)::value)] * 2, K.fix_c1);
+            put(P, e, o, odd);
+        };
+        diagonal(std::integral_constant<int, 3>{}, base + mxy, bx + by);                        // (1, 1, 0)
+        diagonal(std::integral_constant<int, 4>{}, base + 2 * (qx + qy) - mxy, by - bx);        // (-1, 1, 0)
+        diagonal(std::integral_constant<int, 5>{}, base + mxz, bx + bz);                        // (1, 0, 1)
+        diagonal(std::integral_constant<int, 6>{}, base + 2 * (qx + qz) - mxz, bz - bx);        // (-1, 0, 1)
+        diagonal(std::integral_constant<int, 7>{}, base + myz, by + bz);                        // (0, 1, 1)
+        diagonal(std::integral_constant<int, 8>{}, base + 2 * (qy + qz) - myz, bz - by);        // (0, -1, 1)
+        axis(std::integral_constant<int, 0>{}, base_axis + 2 * qx, tx >> 1, (int)tx & 1);
+        axis(std::integral_constant<int, 1>{}, base_axis + 2 * qy, ty >> 1, (int)ty & 1);
+        axis(std::integral_constant<int, 2>{}, base_axis + 2 * qz, tz >> 1, (int)tz & 1);
+    };
+    // FORMS: no test of c1 at every pair, for the one warp of a quarter that a small box has (10 x 11 x 14
+    // porous, tau 1, 800 steps: 3.38 ms against 3.55); a full device loses more by the registers of both
+    // (three components of force 152 us a step against 150)
+    if constexpr (FORMS) {
+        if (K.fix_c1 != 0) pairs(std::true_type{});
+        else pairs(std::false_type{});
+    } else {
+        pairs(K.fix_c1 != 0);
+    }
     n[0] = fixed_to_double(rest, emax);
     return true;
 }
 
 // One fused step of a node, in fixed point or, outside its range, in FP64.
-template <int FMASK, bool UCF, bool WANT_J>
+template <int FMASK, bool UCF, bool WANT_J, bool FORMS>
 __device__ __forceinline__ void fused_step(double (&n)[Q], const bool fm, const bool fc, const double fx,
                                            const double fy, const double fz, const FlowArgs64 &a, double &jx,
                                            double &jy, double &jz)
 {
-    if (fused_fixed<FMASK, WANT_J>(n, fm, fc, fx, fy, fz, a, jx, jy, jz)) return;
+    if (fused_fixed<FMASK, WANT_J, FORMS>(n, fm, fc, fx, fy, fz, a, jx, jy, jz)) return;
     double rho;
     if (fm) moments19_pairs(n, fx / 2.0, fy / 2.0, fz / 2.0, rho, jx, jy, jz);
     else moments19_pairs(n, 0.0, 0.0, 0.0, rho, jx, jy, jz);

@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(STEP_BLOCK, FUSED ? 5 : 4) k_flow_step(const F
             }
             double rho, jx = 0.0, jy = 0.0, jz = 0.0;
             if constexpr (FUSED && !FIELD) {
-                fused_step<FMASK, true, CHECK>(n, fm != 0, fc != 0, fx, fy, fz, a, jx, jy, jz);
+                fused_step<FMASK, true, CHECK, false>(n, fm != 0, fc != 0, fx, fy, fz, a, jx, jy, jz);
             } else if constexpr (FUSED) {
                 if (fm) moments19_pairs(n, fx / 2.0, fy / 2.0, fz / 2.0, rho, jx, jy, jz);
                 else moments19_pairs(n, 0.0, 0.0, 0.0, rho, jx, jy, jz);

@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(SPLIT ? 128 : RT, 1) k_flow64_resident(const R
             for (int l = 0; l < Q; ++l) n[l] = __ldcg(src + off[l]);
             if (r.loop) bad = check19(n);
             double rho, jx = 0.0, jy = 0.0, jz = 0.0;
-            if constexpr (FUSED) fused_step<FMASK, true, true>(n, fm, fc, fx, fy, fz, a, jx, jy, jz);
+            if constexpr (FUSED) fused_step<FMASK, true, true, true>(n, fm, fc, fx, fy, fz, a, jx, jy, jz);
             else moments19_fast(n, fm, fx, fy, fz, rho, jx, jy, jz);
             if (r.loop) {
                 const double e = max_nonneg(max_nonneg(fabs(jx - jold[0]), fabs(jy - jold[1])), fabs(jz - jold[2]));
