@@ -335,7 +335,7 @@ struct CallMemory {
     }
     int get(size_t bytes)
     {
-        constexpr size_t WS_KEPT = 16u << 20;   // moments of 0.5 M nodes
+        constexpr size_t WS_KEPT = 32u << 20;   // moments of 1 M nodes
         int rc;
         if (bytes > b->ws_bytes && bytes <= WS_KEPT && leaves_room(b, bytes - b->ws_bytes)) {
             if (b->d_ws) LBB_CK(cudaFreeAsync(b->d_ws, b->stream));
